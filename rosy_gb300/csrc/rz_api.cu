@@ -839,6 +839,7 @@ ShadeParams shade_params(rz_ctx* c) {
     sh.views = c->d_views;
     sh.view_count = (uint32_t)c->views.size();
     sh.samples = c->samples;
+    sh.gbuffer = c->gbuffer ? 1u : 0u;
     sh.shade_blocks = c->shade_blocks;
     sh.draws = c->d_opaque_draws;
     sh.draw_count = c->opaque_draw_count;

@@ -211,6 +211,7 @@ struct ShadeParams {
     const float* srgb_table;      // 256 entries
     int blended;                  // 1: k_shade stores the RGBA16F draw image (color16) for k_blend
     uint32_t samples;             // camera-pass samples per pixel of the views (1 or 4)
+    uint32_t gbuffer;             // 1: the views have a G-buffer (ViewRec::gb_albedo)
     // the opaque camera setup's per-triangle (draw, varying record of each vertex),
     // indexed by pass-global triangle id; null for the blended list, whose
     // triangles are then looked up through the draw list and the index buffer

@@ -911,86 +911,6 @@ __device__ __forceinline__ float resolve4(float a, float b, float c, float d) {
     return half_round(((a + b) + (c + d)) * 0.25f);
 }
 
-// One pixel of a 4x multisampled view: each distinct triangle among its samples
-// is shaded once at the pixel centre (no sample shading, as the reference's
-// pipeline), its colour is rounded to RGBA16F and given to the samples it
-// covers; uncovered samples keep the clear colour. Without blended surfaces the
-// samples are resolved and encoded here; with them they go to the RGBA16F
-// sample planes for k_blend. The depth output is sample 0's.
-template <bool kLit>
-__device__ __forceinline__ void shade_msaa(const ShadeParams& P, const ViewRec& VR, const float* s_srgb,
-                                           const PixelNdc& pn, int px, int py, size_t p) {
-    const size_t plane = (size_t)VR.width * VR.height;
-    uint32_t ids[kMsaaSamples];
-    unsigned long long key0 = 0;
-#pragma unroll
-    for (int k = 0; k < kMsaaSamples; ++k) {
-        const unsigned long long key = VR.vis[p + k * plane];
-        if (k == 0) key0 = key;
-        ids[k] = (uint32_t)key;
-    }
-    float cs[kMsaaSamples][4];
-    const Sampler smp{&P, s_srgb};
-    const bool gbuffer = VR.gb_albedo != nullptr;
-    float gs[kMsaaSamples][6];  // G-buffer values per sample (albedo rgb, normal xyz)
-#pragma unroll
-    for (int k = 0; k < kMsaaSamples; ++k) {
-        float c[4] = {0.0f, 0.05f, 0.1f, 1.0f};  // clear colour, src/Engine/Graphics.cpp:5416-5419
-        float aux[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        int same = -1;
-#pragma unroll
-        for (int j = 0; j < k; ++j)
-            if (same < 0 && ids[j] == ids[k]) same = j;
-        if (same >= 0) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) cs[k][i] = cs[same][i];
-#pragma unroll
-            for (int i = 0; i < 6; ++i) gs[k][i] = gs[same][i];
-            continue;
-        }
-        if (ids[k] != 0) {
-            float o[4];
-            if (shade_pixel<kLit>(P, VR, *VR.scene, smp, ids[k] - 1u, px, py, o, gbuffer ? aux : nullptr, &pn)) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) c[i] = o[i];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) cs[k][i] = half_round(c[i]);
-#pragma unroll
-        for (int i = 0; i < 6; ++i) gs[k][i] = aux[i];
-    }
-    if (gbuffer) {
-        // G-buffer of a multisampled pixel: albedo and normal averaged over the samples,
-        // coverage = covered samples / 4 in the albedo's alpha
-        float g[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) g[i] = ((gs[0][i] + gs[1][i]) + (gs[2][i] + gs[3][i])) * 0.25f;
-        uint32_t covered = 0;
-#pragma unroll
-        for (int k = 0; k < kMsaaSamples; ++k) covered += ids[k] != 0 ? 1u : 0u;
-        VR.gb_albedo[p] = encode_srgb8(half_round(g[0])) | (encode_srgb8(half_round(g[1])) << 8) |
-                          (encode_srgb8(half_round(g[2])) << 16) | (encode_unorm8((float)covered * 0.25f) << 24);
-        const float len2 = g[3] * g[3] + g[4] * g[4] + g[5] * g[5];
-        const float inv = len2 > 0.0f ? rsqrtf(len2) : 0.0f;
-        VR.gb_normal[p] = encode_octahedral(g[3] * inv, g[4] * inv, g[5] * inv);
-    }
-    VR.depth[p] = __uint_as_float((uint32_t)(key0 >> 32));
-    if (P.blended) {
-#pragma unroll
-        for (int k = 0; k < kMsaaSamples; ++k) {
-            const __half2 rg = __floats2half2_rn(cs[k][0], cs[k][1]), ba = __floats2half2_rn(cs[k][2], cs[k][3]);
-            VR.color16[p + k * plane] =
-                make_uint2(*reinterpret_cast<const uint32_t*>(&rg), *reinterpret_cast<const uint32_t*>(&ba));
-        }
-        return;
-    }
-    float r[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r[i] = resolve4(cs[0][i], cs[1][i], cs[2][i], cs[3][i]);
-    VR.color[p] = encode_srgb8(r[0]) | (encode_srgb8(r[1]) << 8) | (encode_srgb8(r[2]) << 16) | (encode_unorm8(r[3]) << 24);
-}
-
 // The pixel (px, py) of this thread in the block's 16x16 tile, and its
 // pixel-centre coordinates. Each lane of a warp (16 columns, 2 rows) computes its
 // column's and its row's coordinate (the values ndc() gives) and takes its quad's
@@ -1060,30 +980,199 @@ __global__ void __launch_bounds__(256, 4) k_shade(ShadeParams P) {
     VR.color[p] = r | (g << 8) | (b << 16) | (a << 24);
 }
 
-// k_shade for 4x multisampled views.
+// k_shade for 4x multisampled views. Each distinct triangle among a pixel's
+// samples is shaded once at the pixel centre (no sample shading, as the
+// reference's pipeline), its colour is rounded to RGBA16F and given to the samples
+// it covers; uncovered samples keep the clear colour. Without blended surfaces the
+// samples are resolved and encoded here; with them they go to the RGBA16F sample
+// planes for k_blend. The depth output is sample 0's.
+//
+// Bound by the instruction issue of the fragment stage, like k_shade, times the
+// distinct triangles a warp meets: a pixel inside a triangle shows one, a pixel on
+// an edge two to four, and with triangles of a few pixels almost every warp holds
+// one with three or four. So the tile's (pixel, triangle) pairs are listed in
+// shared memory first - every pixel's first triangle in pixel order, then the
+// second ones, and so on, so that neighbours stay neighbours - and the block's
+// threads shade the list, all lanes busy, in one copy of the fragment stage.
+// 1920x1080, 262,144 triangles of a median 4 square pixels: the frame went from
+// 527 to 307 us against four conditional copies of the stage per pixel.
+constexpr int kMsaaItems = 256 * kMsaaSamples;  // (pixel, triangle) pairs of a tile, at most
+
+// A tile's pixel-centre coordinates (the values ndc() gives): its columns and rows.
+struct TileNdc {
+    float x[16], y[16];
+};
+
+// Shades the listed pairs of the tile at (tx0, ty0): item i is the triangle
+// item_id[i] (id + 1) at pixel item_px[i] (row * 16 + column). Writes its RGBA16F
+// colour to item_col[i] and, with a G-buffer, its six values to item_aux + 6 i.
+template <bool kLit, bool kAux>
+__device__ __forceinline__ void shade_items(const ShadeParams& P, const ViewRec& VR, const float* s_srgb, const TileNdc& tn,
+                                            int tx0, int ty0, int tid, int total, const uint32_t* item_id,
+                                            const uint8_t* item_px, uint2* item_col, float* item_aux) {
+    const Sampler smp{&P, s_srgb};
+#pragma unroll 1
+    for (int i = tid; i < total; i += 256) {
+        const int t = item_px[i], lx = t & 15, ly = t >> 4;
+        const PixelNdc pn{tn.x[lx], tn.y[ly], tn.x[lx & ~1], tn.y[ly & ~1], tn.x[lx | 1], tn.y[ly | 1]};
+        float c[4] = {0.0f, 0.05f, 0.1f, 1.0f};  // clear colour, src/Engine/Graphics.cpp:5416-5419
+        float aux[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        float o[4];
+        if (shade_pixel<kLit>(P, VR, *VR.scene, smp, item_id[i] - 1u, tx0 + lx, ty0 + ly, o, kAux ? aux : nullptr, &pn)) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) c[k] = o[k];
+        }
+        const __half2 rg = __floats2half2_rn(c[0], c[1]), ba = __floats2half2_rn(c[2], c[3]);
+        item_col[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&rg), *reinterpret_cast<const uint32_t*>(&ba));
+        if (kAux) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) item_aux[6 * i + k] = aux[k];
+        }
+    }
+}
+
+template <bool kAux>  // the views have a G-buffer
 __global__ void __launch_bounds__(256, 4) k_shade_msaa(ShadeParams P) {
     __shared__ float s_srgb[256];
     __shared__ uint32_t s_view;
-    {
-        const int t = threadIdx.y * blockDim.x + threadIdx.x;
-        s_srgb[t] = P.srgb_table[t];
-        if (t == 0) s_view = tile_view(P.views, P.view_count, blockIdx.x + P.block_offset);
-    }
+    __shared__ TileNdc s_ndc;
+    __shared__ uint32_t s_count[kMsaaSamples][8];  // per rank and warp: pixels with that many distinct triangles
+    __shared__ uint32_t s_id[kMsaaItems];
+    __shared__ uint8_t s_px[kMsaaItems];
+    __shared__ uint2 s_col[kMsaaItems];
+    extern __shared__ float s_aux[];  // kMsaaItems x 6, with a G-buffer
+    const int tid = threadIdx.y * 16 + threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    s_srgb[tid] = P.srgb_table[tid];
+    if (tid == 0) s_view = tile_view(P.views, P.view_count, blockIdx.x + P.block_offset);
     __syncthreads();
     const ViewRec& VR = P.views[s_view];
-    int px, py;
-    const PixelNdc pn = pixel_ndc(P, VR, px, py);
-    if (px >= VR.width || py >= VR.height) return;
-    const size_t p = (size_t)py * VR.width + px;
-    if (lit_view(*VR.scene)) shade_msaa<true>(P, VR, s_srgb, pn, px, py, p);
-    else shade_msaa<false>(P, VR, s_srgb, pn, px, py, p);
+    const uint32_t lt = blockIdx.x + P.block_offset - VR.shade_block_base;
+    const uint32_t tiles_x = ((uint32_t)VR.width + 15) / 16;
+    const int tx0 = (int)(lt % tiles_x) * 16, ty0 = (int)(lt / tiles_x) * 16;
+    const int px = tx0 + (int)threadIdx.x, py = ty0 + (int)threadIdx.y;
+    const bool inside = px < VR.width && py < VR.height;
+    const size_t plane = (size_t)VR.width * VR.height;
+    const size_t p = inside ? (size_t)py * VR.width + px : 0;
+    if (tid < 16) s_ndc.x[tid] = ndc(tx0 + tid, VR.width);
+    else if (tid < 32) s_ndc.y[tid - 16] = ndc(ty0 + tid - 16, VR.height);
+    // the pixel's distinct triangles: sample k shows the rank[k]-th one
+    uint32_t ids[kMsaaSamples], distinct[kMsaaSamples];
+#pragma unroll
+    for (int k = 0; k < kMsaaSamples; ++k) ids[k] = 0u;
+    if (inside) {
+#pragma unroll
+        for (int k = 0; k < kMsaaSamples; ++k) {
+            const unsigned long long key = VR.vis[p + k * plane];
+            if (k == 0) VR.depth[p] = __uint_as_float((uint32_t)(key >> 32));
+            ids[k] = (uint32_t)key;
+        }
+    }
+    uint32_t n = 0, ranks = 0;
+#pragma unroll
+    for (int k = 0; k < kMsaaSamples; ++k) {
+        distinct[k] = 0u;
+        uint32_t r = n;
+#pragma unroll
+        for (int j = k - 1; j >= 0; --j)
+            if (ids[j] == ids[k]) r = (ranks >> (4 * j)) & 7u;
+        if (ids[k] == 0u) {
+            r = 7u;  // not covered
+        } else if (r == n) {
+#pragma unroll
+            for (int j = 0; j < kMsaaSamples; ++j)
+                if ((uint32_t)j == n) distinct[j] = ids[k];
+            ++n;
+        }
+        ranks |= r << (4 * k);
+    }
+    uint32_t before[kMsaaSamples];  // lanes before this one in the warp with a triangle of that rank
+#pragma unroll
+    for (int r = 0; r < kMsaaSamples; ++r) {
+        const uint32_t m = __ballot_sync(0xffffffffu, n > (uint32_t)r);
+        before[r] = __popc(m & ((1u << lane) - 1u));
+        if (lane == 0) s_count[r][warp] = __popc(m);
+    }
+    __syncthreads();
+    uint64_t slots = 0;  // where the pixel's triangles sit in the list, 16 bits per rank
+    uint32_t total = 0;
+#pragma unroll
+    for (int r = 0; r < kMsaaSamples; ++r) {
+        uint32_t at = total + before[r];
+        for (int w = 0; w < 8; ++w) {
+            if (w < warp) at += s_count[r][w];
+            total += s_count[r][w];
+        }
+        slots |= (uint64_t)at << (16 * r);
+        if (n > (uint32_t)r) {
+            s_id[at] = distinct[r];
+            s_px[at] = (uint8_t)tid;
+        }
+    }
+    __syncthreads();
+    if (lit_view(*VR.scene)) shade_items<true, kAux>(P, VR, s_srgb, s_ndc, tx0, ty0, tid, (int)total, s_id, s_px, s_col, s_aux);
+    else shade_items<false, kAux>(P, VR, s_srgb, s_ndc, tx0, ty0, tid, (int)total, s_id, s_px, s_col, s_aux);
+    __syncthreads();
+    if (!inside) return;
+    float cs[kMsaaSamples][4];
+#pragma unroll
+    for (int k = 0; k < kMsaaSamples; ++k) {
+        const uint32_t r = (ranks >> (4 * k)) & 7u;
+        cs[k][0] = half_round(0.0f);  // clear colour, src/Engine/Graphics.cpp:5416-5419
+        cs[k][1] = half_round(0.05f);
+        cs[k][2] = half_round(0.1f);
+        cs[k][3] = half_round(1.0f);
+        if (r != 7u) {
+            const uint2 c = s_col[(slots >> (16 * r)) & 0xffffu];
+            const __half2 rg = *reinterpret_cast<const __half2*>(&c.x), ba = *reinterpret_cast<const __half2*>(&c.y);
+            cs[k][0] = __low2float(rg);
+            cs[k][1] = __high2float(rg);
+            cs[k][2] = __low2float(ba);
+            cs[k][3] = __high2float(ba);
+        }
+    }
+    if (kAux) {
+        // G-buffer of a multisampled pixel: albedo and normal averaged over the samples,
+        // coverage = covered samples / 4 in the albedo's alpha
+        float gs[kMsaaSamples][6], g[6];
+        uint32_t covered = 0;
+#pragma unroll
+        for (int k = 0; k < kMsaaSamples; ++k) {
+            const uint32_t r = (ranks >> (4 * k)) & 7u;
+            covered += r != 7u ? 1u : 0u;
+#pragma unroll
+            for (int i = 0; i < 6; ++i) gs[k][i] = r != 7u ? s_aux[6 * ((slots >> (16 * r)) & 0xffffu) + i] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) g[i] = ((gs[0][i] + gs[1][i]) + (gs[2][i] + gs[3][i])) * 0.25f;
+        VR.gb_albedo[p] = encode_srgb8(half_round(g[0])) | (encode_srgb8(half_round(g[1])) << 8) |
+                          (encode_srgb8(half_round(g[2])) << 16) | (encode_unorm8((float)covered * 0.25f) << 24);
+        const float len2 = g[3] * g[3] + g[4] * g[4] + g[5] * g[5];
+        const float inv = len2 > 0.0f ? rsqrtf(len2) : 0.0f;
+        VR.gb_normal[p] = encode_octahedral(g[3] * inv, g[4] * inv, g[5] * inv);
+    }
+    if (P.blended) {
+#pragma unroll
+        for (int k = 0; k < kMsaaSamples; ++k) {
+            const __half2 rg = __floats2half2_rn(cs[k][0], cs[k][1]), ba = __floats2half2_rn(cs[k][2], cs[k][3]);
+            VR.color16[p + k * plane] =
+                make_uint2(*reinterpret_cast<const uint32_t*>(&rg), *reinterpret_cast<const uint32_t*>(&ba));
+        }
+        return;
+    }
+    float c4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c4[i] = resolve4(cs[0][i], cs[1][i], cs[2][i], cs[3][i]);
+    VR.color[p] = encode_srgb8(c4[0]) | (encode_srgb8(c4[1]) << 8) | (encode_srgb8(c4[2]) << 16) | (encode_unorm8(c4[3]) << 24);
 }
 
 void launch_shade(const ShadeParams& p, cudaStream_t stream) {
     if (p.shade_blocks == 0) return;
     note_launch();
     if (p.samples > 1) {
-        k_shade_msaa<<<p.shade_blocks, dim3(16, 16), 0, stream>>>(p);
+        // the G-buffer values of the listed pairs: 24 KB, within the default limit with the static arrays
+        if (p.gbuffer) k_shade_msaa<true><<<p.shade_blocks, dim3(16, 16), kMsaaItems * 6 * sizeof(float), stream>>>(p);
+        else k_shade_msaa<false><<<p.shade_blocks, dim3(16, 16), 0, stream>>>(p);
         return;
     }
     k_shade<<<p.shade_blocks, dim3(16, 16), 0, stream>>>(p);

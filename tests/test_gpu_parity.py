@@ -222,6 +222,25 @@ def test_msaa_parity(gpu, oracle, name):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("width,height,triangles", [(16, 16, 20000), (17, 15, 20000), (33, 1, 3000), (1, 40, 3000),
+                                                    (47, 31, 1), (64, 48, 300)])
+def test_msaa_tiles_of_one_to_four_triangles(gpu, oracle, width, height, triangles):
+    """Tiles whose list of (pixel, triangle) pairs is full (a triangle per sample), ragged or nearly empty."""
+    s = sc.random_triangles(seed=41, triangles=triangles, width=width, height=height, shadow_size=128, texture_size=32)
+    if triangles > 10000:  # triangles of a pixel or less: four of them in most pixels
+        v = s.vertices[:, 0:3].reshape(-1, 3, 3)
+        s.vertices[:, 0:3] = (v[:, :1] + (v - v[:, :1]) * np.float32(0.12)).reshape(-1, 3)
+        s.draw_config["cull_enabled"] = 0
+    s.samples = 4
+    ref, out = run(s, oracle)
+    if triangles > 10000:
+        assert (np.ptp(out["ids"], axis=0) > 0).mean() > 0.5
+    assert np.array_equal(out["ids"], ref["ids"])
+    assert np.array_equal(out["vis_depth"].view(np.uint32), ref["depth"].view(np.uint32))
+    assert np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32)).max() <= COLOR_TOL
+
+
+@pytest.mark.gpu
 def test_shading_error_against_fp64_oracle(gpu, oracle):
     """The oracle also shades in float64; the GPU's 8-bit sRGB colour stays within
     1.5 levels of that (0.5 of it is the 8-bit rounding itself)."""
