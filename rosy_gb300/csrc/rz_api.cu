@@ -96,6 +96,9 @@ struct rz_ctx {
     cudaStream_t side = nullptr;  // shadow pass branch of the frame graph
     cudaStream_t vtx = nullptr;   // vertex stage, beside the camera pass's setup and raster
     cudaEvent_t vtx_fork = nullptr, vtx_join = nullptr;
+    // 4x multisampling: the other parts of the camera raster, beside the first
+    cudaStream_t msaa[kMsaaSamples - 1] = {nullptr, nullptr, nullptr};
+    cudaEvent_t msaa_fork = nullptr, msaa_join[kMsaaSamples - 1] = {nullptr, nullptr, nullptr};
     // read-back (rz_read_frame): device staging copies on the frame stream, then
     // device-to-host copies on their own stream so that the next frame renders meanwhile
     cudaStream_t copy_stream = nullptr;
@@ -791,8 +794,8 @@ PassParams pass_params(rz_ctx* c, int kind) {
     p.lookback_spins = c->lookback_spins;
     p.sample_x = 128;  // pixel centre
     p.sample_y = 128;
-    p.sample_plane = 0;
-    p.bb_hi = (kind != 0 && c->samples > 1) ? 32 : 128;
+    p.msaa = (kind != 0 && c->samples > 1) ? 1 : 0;
+    p.bb_hi = p.msaa ? 32 : 128;
     PassBuffers* pb;
     if (kind == 2) {  // blended list: cull none, records kept in submission order
         p.draws = c->d_blended_draws;
@@ -899,26 +902,33 @@ void enqueue_shadow(rz_ctx* c, cudaStream_t s, bool stamps) {
     }
 }
 
-// Camera passes of all views (5566-5653): visibility cleared to 0, opaque list,
-// then the vertex stage of the shading; the blended list's setup.
-// The camera raster: one launch per coverage sample, each into its plane of the
-// visibility buffer (the setup records are shared).
-void launch_camera_raster(rz_ctx* c, PassParams cp, cudaStream_t s) {
+// The camera raster. With 4x multisampling its work is dealt to one launch per
+// sample: each takes its part of the records, at all four samples (a record is
+// loaded and decoded once for the four). Outside stage timing the launches run side
+// by side on branches of their own, each with its part of the resident CTAs.
+int launch_camera_raster(rz_ctx* c, PassParams cp, cudaStream_t s, bool branches) {
     if (c->samples <= 1) {
         launch_raster(cp, c->sm_count, s);
-        return;
+        return RZ_OK;
     }
+    if (branches) RZ_CUDA(c, cudaEventRecord(c->msaa_fork, s), "camera raster fork");
     for (int k = 0; k < kMsaaSamples; ++k) {
-        cp.sample_x = kMsaaX[k];
-        cp.sample_y = kMsaaY[k];
-        cp.sample_plane = (uint32_t)k;
-        launch_raster(cp, c->sm_count, s);
+        cp.part = (uint32_t)k;
+        cudaStream_t b = k && branches ? c->msaa[k - 1] : s;
+        if (k && branches) RZ_CUDA(c, cudaStreamWaitEvent(b, c->msaa_fork, 0), "camera raster fork");
+        launch_raster(cp, c->sm_count, b, branches ? kMsaaSamples : 1);
+        if (k && branches) RZ_CUDA(c, cudaEventRecord(c->msaa_join[k - 1], b), "camera raster join");
     }
+    for (int k = 1; k < kMsaaSamples && branches; ++k)
+        RZ_CUDA(c, cudaStreamWaitEvent(s, c->msaa_join[k - 1], 0), "camera raster join");
+    return RZ_OK;
 }
 
+// Camera passes of all views (5566-5653): visibility cleared to 0, opaque list,
+// then the vertex stage of the shading; the blended list's setup.
 // The visibility buffer is zeroed by the opaque setup launch when there is one,
 // else by the clear launch.
-void enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh) {
+int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh) {
     ClearList cl{};
     cl.ptr[0] = &c->d_report->camera;  // the camera and blended headers and their error word
     cl.bytes[0] = sizeof(FrameReport) - offsetof(FrameReport, camera);
@@ -958,7 +968,8 @@ void enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& s
         launch_setup(cp, s);
         cp.clear_count = 0;
         if (stamps) stamp(c, 5);
-        launch_camera_raster(c, cp, s);
+        const int rc = launch_camera_raster(c, cp, s, !stamps);
+        if (rc != RZ_OK) return rc;
     } else if (stamps) {
         stamp(c, 5);
     }
@@ -975,12 +986,13 @@ void enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& s
         bs.tri_refs = nullptr;
         launch_vertex_range(bs, c->blended_varying_base, s);
     }
+    return RZ_OK;
 }
 
 // Per-view sequential launches: the same kernels, restricted to one view at a
 // time (its draws, its pixels, its targets), view after view. This is what the
 // batched frame is measured against.
-void enqueue_sequential(rz_ctx* c, cudaStream_t s, const ShadeParams& sh) {
+int enqueue_sequential(rz_ctx* c, cudaStream_t s, const ShadeParams& sh) {
     for (uint32_t vi = 0; vi < c->views.size(); ++vi) {
         const rz_ctx::ViewRange& rg = c->ranges[vi];
         ClearList cl{};
@@ -1018,7 +1030,8 @@ void enqueue_sequential(rz_ctx* c, cudaStream_t s, const ShadeParams& sh) {
             cp.tri_offset = rg.opaque_tri_base;
             cp.tri_total = rg.opaque_tris;
             launch_setup(cp, s);
-            launch_camera_raster(c, cp, s);
+            const int rc = launch_camera_raster(c, cp, s, false);
+            if (rc != RZ_OK) return rc;
         }
         ShadeParams v = sh;
         v.varying_count = rg.varying_end;
@@ -1027,6 +1040,7 @@ void enqueue_sequential(rz_ctx* c, cudaStream_t s, const ShadeParams& sh) {
         v.shade_blocks = rg.blocks;
         launch_shade(v, s);
     }
+    return RZ_OK;
 }
 
 // Enqueues one frame (everything after the scene/object uploads). With stage
@@ -1046,18 +1060,21 @@ int enqueue_frame(rz_ctx* c) {
         RZ_CUDA(c, cudaMemsetAsync(c->d_report, 0, sizeof(FrameReport), s), "clear frame report");
         launch_prep(c->d_shadow_draws, c->shadow_draw_count, c->d_objects, c->d_views, c->d_shadow_mvp, s);
         launch_prep_camera(c->d_opaque_draws, c->opaque_draw_count, c->d_objects, c->d_views, c->d_camera_consts, s);
-        enqueue_sequential(c, s, sh);
+        const int rc = enqueue_sequential(c, s, sh);
+        if (rc != RZ_OK) return rc;
     } else if (c->timing) {
         stamp(c, 0);
         enqueue_shadow(c, s, true);
         stamp(c, 3);
-        enqueue_camera(c, s, true, sh);
+        const int rc = enqueue_camera(c, s, true, sh);
+        if (rc != RZ_OK) return rc;
         stamp(c, 6);
     } else {
         RZ_CUDA(c, cudaEventRecord(c->fork, s), "fork");
         RZ_CUDA(c, cudaStreamWaitEvent(c->side, c->fork, 0), "fork");
         enqueue_shadow(c, c->side, false);
-        enqueue_camera(c, s, false, sh);
+        const int rc = enqueue_camera(c, s, false, sh);
+        if (rc != RZ_OK) return rc;
         RZ_CUDA(c, cudaEventRecord(c->join, c->side), "join");
         if (sources) {
             RZ_CUDA(c, cudaEventRecord(c->camera_done, s), "camera done");
@@ -1252,6 +1269,13 @@ int rz_create(rz_ctx** out, const rz_config* cfg) {
         cudaEventCreateWithFlags(&c->sources_done, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(RZ_GRAPHICS_INIT_FAILURE);
+    if (c->samples > 1) {
+        if (cudaEventCreateWithFlags(&c->msaa_fork, cudaEventDisableTiming) != cudaSuccess) return bail(RZ_GRAPHICS_INIT_FAILURE);
+        for (int k = 0; k < kMsaaSamples - 1; ++k)
+            if (cudaStreamCreateWithFlags(&c->msaa[k], cudaStreamNonBlocking) != cudaSuccess ||
+                cudaEventCreateWithFlags(&c->msaa_join[k], cudaEventDisableTiming) != cudaSuccess)
+                return bail(RZ_GRAPHICS_INIT_FAILURE);
+    }
     for (int k = 0; k < 2; ++k)
         if (cudaEventCreateWithFlags(&c->read_done[k], cudaEventDisableTiming) != cudaSuccess)
             return bail(RZ_GRAPHICS_INIT_FAILURE);
@@ -1307,6 +1331,8 @@ void rz_destroy(rz_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->side) cudaStreamSynchronize(c->side);
     if (c->vtx) cudaStreamSynchronize(c->vtx);
+    for (cudaStream_t b : c->msaa)
+        if (b) cudaStreamSynchronize(b);
     if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
     if (c->upload) cudaStreamSynchronize(c->upload);
     drop_graph(c);
@@ -1373,6 +1399,11 @@ void rz_destroy(rz_ctx* c) {
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->vtx) cudaStreamDestroy(c->vtx);
+    if (c->msaa_fork) cudaEventDestroy(c->msaa_fork);
+    for (int k = 0; k < kMsaaSamples - 1; ++k) {
+        if (c->msaa_join[k]) cudaEventDestroy(c->msaa_join[k]);
+        if (c->msaa[k]) cudaStreamDestroy(c->msaa[k]);
+    }
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }

@@ -109,8 +109,6 @@ constexpr int kMaxCascades = 4;
 // Standard sample positions of 4x multisampling (Vulkan standardSampleLocations),
 // in 1/256 pixel: (0.375, 0.125), (0.875, 0.375), (0.125, 0.625), (0.625, 0.875).
 constexpr int kMsaaSamples = 4;
-constexpr int32_t kMsaaX[kMsaaSamples] = {96, 224, 32, 160};
-constexpr int32_t kMsaaY[kMsaaSamples] = {32, 96, 160, 224};
 __host__ __device__ constexpr int32_t msaa_x(int k) { return k == 0 ? 96 : k == 1 ? 224 : k == 2 ? 32 : 160; }
 __host__ __device__ constexpr int32_t msaa_y(int k) { return k == 0 ? 32 : k == 1 ? 96 : k == 2 ? 160 : 224; }
 
@@ -174,10 +172,12 @@ struct PassParams {
     PassHeader* header;
     uint32_t* error_flags;
     uint32_t lookback_spins;  // bound of each look-back wait (ordered passes)
-    // coverage sample of this raster launch, in 1/256 pixel: the pixel centre
-    // (128, 128) or one of the standard 4x positions; camera-pass target plane
+    // coverage sample, in 1/256 pixel: the pixel centre (128, 128)
     int32_t sample_x, sample_y;
-    uint32_t sample_plane;
+    // 4x multisampled camera pass: every record at the four standard positions, each
+    // into its plane; the records are dealt to kMsaaSamples launches, of which this is `part`
+    int32_t msaa;
+    uint32_t part;
     int32_t bb_hi;  // smallest sample offset the setup boxed for (32 with 4x samples, else 128)
     // buffers the setup launch zeroes besides its own work (the depth target's
     // CLEAR load-op, folded into the launch that precedes the raster); none when
@@ -275,7 +275,8 @@ void launch_prep(const DrawRec* draws, uint32_t n, const rz_object* objects, con
 void launch_prep_camera(const DrawRec* draws, uint32_t n, const rz_object* objects, const ViewRec* views,
                         DrawConsts* out, cudaStream_t stream, const ClearList* clear = nullptr, int sm_count = 0);
 void launch_setup(const PassParams& p, cudaStream_t stream);
-void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream);
+// `share`: the launch is one of that many that run side by side (its grid is that part of the resident CTAs)
+void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int share = 1);
 void launch_vertex(const ShadeParams& p, cudaStream_t stream);
 // k_vertex over the varying records [first, varying_count) of the draws in p
 // (whose varying_base values start at `first`).

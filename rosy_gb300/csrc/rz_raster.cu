@@ -649,7 +649,8 @@ void launch_setup(const PassParams& p, cudaStream_t stream) {
 // With the top-left decision folded into the constant (E' = E - 1 on the other
 // edges) the test is E' >= 0 on all three edges.
 
-// The target of a view: visibility (camera pass) or shadow map, and its row pitch.
+// The target of a view: visibility (camera pass; of a multisampled view, its first
+// sample plane) or shadow map, and its row pitch.
 struct Target {
     void* ptr;
     int pitch;
@@ -658,9 +659,15 @@ struct Target {
 template <bool kWriteId>
 __device__ __forceinline__ Target view_target(const PassParams& P, uint32_t view) {
     const ViewRec& V = P.views[view & kViewMask];
-    if (kWriteId) return Target{V.vis + (size_t)P.sample_plane * (size_t)V.width * (size_t)V.height, V.width};
+    if (kWriteId) return Target{V.vis, V.width};
     return Target{V.shadow + (size_t)((view >> kViewBits) & kCascadeMask) * (size_t)V.shadow_w * (size_t)V.shadow_h,
                   V.shadow_w};
+}
+
+// Words between the sample planes of a multisampled view's visibility.
+__device__ __forceinline__ size_t plane_words(const PassParams& P, uint32_t view) {
+    const ViewRec& V = P.views[view & kViewMask];
+    return (size_t)V.width * (size_t)V.height;
 }
 
 // The stored depth of a fragment: the interpolated z plus the record's depth bias
@@ -702,7 +709,7 @@ __device__ __forceinline__ void write_fragment(const Target& T, int px, int py, 
 // One lane rasterises one small triangle: its extent is at most the pass's
 // small_extent (<= kMaxSmallExtent = 16 pixels = 4096 sub-pixels) each way, so
 // every edge value and product stays below 2^26 and fits in 32 bits.
-template <bool kWriteId>
+template <bool kWriteId, bool kMsaa>
 __device__ __forceinline__ void raster_small(const PassParams& P, const TriRecord* rec) {
     const int4* src = reinterpret_cast<const int4*>(rec);
     const int4 q0 = __ldg(src), q1 = __ldg(src + 1), q2 = __ldg(src + 2), q3 = __ldg(src + 3);
@@ -723,16 +730,43 @@ __device__ __forceinline__ void raster_small(const PassParams& P, const TriRecor
         // E' at (PX, PY) = c + dx*(PY - Y0) - dy*(PX - X0)
         c[i] = dy[i] * (X[a] - X[0]) - dx[i] * (Y[a] - Y[0]) - (tl ? 0 : 1);
     }
-    for (int py = py0; py <= py1; ++py) {
-        const int32_t ry = py * 256 + P.sample_y - Y[0];
-        for (int px = px0; px <= px1; ++px) {
-            const int32_t rx = px * 256 + P.sample_x - X[0];
-            const int32_t e0 = c[0] + dx[0] * ry - dy[0] * rx;
-            const int32_t e1 = c[1] + dx[1] * ry - dy[1] * rx;
-            const int32_t e2 = c[2] + dx[2] * ry - dy[2] * rx;
-            if ((e0 | e1 | e2) >= 0) {
-                const float z = biased_depth(fmaf(dzdx, (float)rx, fmaf(dzdy, (float)ry, z0)), bias);
-                write_fragment<kWriteId>(T, px, py, z, id);
+    if (kMsaa) {
+        // the four samples of a pixel: the edges at its corner plus constant offsets
+        int32_t off[kMsaaSamples][3];
+#pragma unroll
+        for (int k = 0; k < kMsaaSamples; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) off[k][i] = dx[i] * msaa_y(k) - dy[i] * msaa_x(k);
+        const size_t plane = plane_words(P, (uint32_t)q3.y);
+        for (int py = py0; py <= py1; ++py) {
+            const int32_t ry = py * 256 - Y[0];
+            for (int px = px0; px <= px1; ++px) {
+                const int32_t rx = px * 256 - X[0];
+                const int32_t e0 = c[0] + dx[0] * ry - dy[0] * rx;
+                const int32_t e1 = c[1] + dx[1] * ry - dy[1] * rx;
+                const int32_t e2 = c[2] + dx[2] * ry - dy[2] * rx;
+#pragma unroll
+                for (int k = 0; k < kMsaaSamples; ++k) {
+                    if (((e0 + off[k][0]) | (e1 + off[k][1]) | (e2 + off[k][2])) >= 0) {
+                        const float fx = (float)(rx + msaa_x(k)), fy = (float)(ry + msaa_y(k));
+                        const float z = biased_depth(fmaf(dzdx, fx, fmaf(dzdy, fy, z0)), bias);
+                        write_word<kWriteId>(target_word<kWriteId>(T, px, py) + k * plane, z, id);
+                    }
+                }
+            }
+        }
+    } else {
+        for (int py = py0; py <= py1; ++py) {
+            const int32_t ry = py * 256 + P.sample_y - Y[0];
+            for (int px = px0; px <= px1; ++px) {
+                const int32_t rx = px * 256 + P.sample_x - X[0];
+                const int32_t e0 = c[0] + dx[0] * ry - dy[0] * rx;
+                const int32_t e1 = c[1] + dx[1] * ry - dy[1] * rx;
+                const int32_t e2 = c[2] + dx[2] * ry - dy[2] * rx;
+                if ((e0 | e1 | e2) >= 0) {
+                    const float z = biased_depth(fmaf(dzdx, (float)rx, fmaf(dzdy, (float)ry, z0)), bias);
+                    write_fragment<kWriteId>(T, px, py, z, id);
+                }
             }
         }
     }
@@ -1009,26 +1043,92 @@ __device__ __forceinline__ void medium_walk(const Target& T, const LargeRecord& 
     }
 }
 
+// The walk over a medium record's stamps at the four standard sample positions:
+// the edge values at the pixels' corners, to which each sample adds constants (the
+// sums are the values medium_start computes for that sample, in wrapping 32-bit
+// arithmetic), the word of each sample a plane further. What a record segment costs
+// before its first stamp (decode, start values: 220 warp instructions for 4 stamps
+// of 13) is then paid once, not per sample: on the 1080p scene-scale frame the
+// camera raster issued 50.6 M warp instructions as four passes over the records,
+// and the frame goes from 307 to 286 us.
+template <bool kBoxCheck>
+__device__ __forceinline__ void medium_walk_msaa(const Target& T, size_t plane, const LargeRecord& L, uint32_t sx, uint32_t sy,
+                                                 uint32_t n, int lx, int ly) {
+    MediumWalk<true> w;
+    medium_start<true>(T, L, sx, sy, lx, ly, 0, 0, w);
+    int32_t off[kMsaaSamples][3];
+    float zrow[kMsaaSamples];
+#pragma unroll
+    for (int k = 0; k < kMsaaSamples; ++k) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            off[k][i] = (int32_t)((uint32_t)L.dx[i] * (uint32_t)msaa_y(k) - (uint32_t)L.dy[i] * (uint32_t)msaa_x(k));
+        zrow[k] = fmaf(L.dzdy, w.fy + (float)msaa_y(k), L.z0);
+    }
+    const size_t row_step = (size_t)kStampH * (size_t)T.pitch;
+    while (true) {
+        const uint32_t run = min(n, L.nsx - sx);
+        for (uint32_t j = 0; j < run; ++j) {
+            if (!kBoxCheck || (w.px <= L.px1 && w.py <= L.py1)) {
+#pragma unroll
+                for (int k = 0; k < kMsaaSamples; ++k) {
+                    const int32_t e0 = (int32_t)((uint32_t)w.e[0] + (uint32_t)off[k][0]);
+                    const int32_t e1 = (int32_t)((uint32_t)w.e[1] + (uint32_t)off[k][1]);
+                    const int32_t e2 = (int32_t)((uint32_t)w.e[2] + (uint32_t)off[k][2]);
+                    if ((e0 | e1 | e2) >= 0)
+                        write_word<true>(w.w + k * plane, biased_depth(fmaf(L.dzdx, w.fx + (float)msaa_x(k), zrow[k]), L.bias),
+                                         L.id);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 3; ++i) w.e[i] = (int32_t)((uint32_t)w.e[i] + (uint32_t)w.stepx[i]);
+            w.w += kStampW;
+            w.fx += (float)(kStampW * 256);
+            if (kBoxCheck) w.px += kStampW;
+        }
+        n -= run;
+        if (n == 0) return;
+        sx = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            w.er[i] = (int32_t)((uint32_t)w.er[i] + (uint32_t)w.stepy[i]);
+            w.e[i] = w.er[i];
+        }
+        w.wr += row_step;
+        w.w = w.wr;
+        w.fx = w.fxr;
+        w.fy += (float)(kStampH * 256);
+#pragma unroll
+        for (int k = 0; k < kMsaaSamples; ++k) zrow[k] = fmaf(L.dzdy, w.fy + (float)msaa_y(k), L.z0);
+        if (kBoxCheck) {
+            w.px = w.pxr;
+            w.py += kStampH;
+        }
+    }
+}
+
 // Persistent raster: each warp first takes batches of 32 small records (one per
 // lane), then chunks of kChunkStamps stamps of the large records, both in a
 // fixed grid-stride order. (A shared cursor that every warp bumps with an
 // atomic serialises on one L2 line: a raster launch with its work skipped took
 // 12 us that way on the 4096^2 shadow pass of 262,144 triangles, 6 us without.)
-template <bool kWriteId>
+template <bool kWriteId, bool kMsaa>
 __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
     __shared__ int4 s_stage[kRasterThreads / 32][2][kStageRecords][4];
     const int lane = threadIdx.x & 31;
     const int lx = lane & (kStampW - 1), ly = lane >> 3;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t warp_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // a multisampled pass's launches number their warps together
+    const uint32_t warps = ((gridDim.x * blockDim.x) >> 5) * (kMsaa ? kMsaaSamples : 1u);
+    const uint32_t warp_id = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kMsaa ? kMsaaSamples : 1u) + (kMsaa ? P.part : 0u);
     const uint64_t n_small = min(P.header->small_records, P.small_capacity);
     for (uint64_t base = (uint64_t)warp_id * 32u; base < n_small; base += (uint64_t)warps * 32u)
-        if (base + lane < n_small) raster_small<kWriteId>(P, P.small_records + base + lane);
+        if (base + lane < n_small) raster_small<kWriteId, kMsaa>(P, P.small_records + base + lane);
     const uint32_t chunks = P.header->chunks;
     const uint64_t total = P.header->stamps;
     const uint32_t n_rec = min(P.header->records, P.record_capacity);  // records the setup wrote
     uint32_t cur_view = 0xffffffffu;  // the view whose target T holds
     Target T{nullptr, 0};
+    size_t plane = 0;
     // chunk k's first record (r_cur, staged in buffer cb), the next chunk's (r_next)
     int cb = 0;
     uint32_t r_cur = warp_id < chunks ? P.chunk_map[warp_id] : n_rec;
@@ -1062,9 +1162,28 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
             const uint32_t sy = i ? i / L.nsx : 0u, sx = i - sy * L.nsx;  // a segment mostly starts at its record's first stamp
             if (L.view != cur_view) {
                 T = view_target<kWriteId>(P, L.view);
+                if (kMsaa) plane = plane_words(P, L.view);
                 cur_view = L.view;
             }
-            if (L.medium) {
+            if (kMsaa) {
+                if (L.medium) {
+                    if (L.clipped) medium_walk_msaa<true>(T, plane, L, sx, sy, n, lx, ly);
+                    else medium_walk_msaa<false>(T, plane, L, sx, sy, n, lx, ly);
+                } else {
+                    GenericEdges G;
+                    generic_edges(L, G);
+#pragma unroll 1
+                    for (int k = 0; k < kMsaaSamples; ++k) {
+                        const Target Tk{reinterpret_cast<TargetWord<kWriteId>*>(T.ptr) + k * plane, T.pitch};
+                        GenericWalk w;
+                        generic_start(L, G, sx, sy, msaa_x(k), msaa_y(k), w);
+                        for (uint32_t j = 0; j < n; ++j) {
+                            raster_stamp<kWriteId, true>(Tk, L, G, w, lx, ly, msaa_x(k), msaa_y(k));
+                            generic_next(L, w);
+                        }
+                    }
+                }
+            } else if (L.medium) {
                 MediumWalk<kWriteId> w;
                 medium_start<kWriteId>(T, L, sx, sy, lx, ly, P.sample_x, P.sample_y, w);
                 if (L.clipped) medium_walk<kWriteId, true>(T, L, sx, n, w);
@@ -1097,19 +1216,17 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream) {
-    // persistent grid: as many CTAs as can be resident at once
-    static int occ[2] = {0, 0};
-    const int t = p.write_id ? 1 : 0;
+void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int share) {
+    // persistent grid: as many CTAs as can be resident at once, with the launches beside this one
+    static int occ[3] = {0, 0, 0};
+    const int t = !p.write_id ? 0 : p.msaa ? 2 : 1;
+    void (*const kernel)(PassParams) = t == 0 ? k_raster<false, false> : t == 1 ? k_raster<true, false> : k_raster<true, true>;
     if (!occ[t]) {
         int n = 0;
-        if (p.write_id) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster<true>, kRasterThreads, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster<false>, kRasterThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kRasterThreads, 0);
         occ[t] = n > 0 ? n : 1;
     }
-    const int blocks = sm_count * occ[t];
-    if (p.write_id) k_raster<true><<<blocks, kRasterThreads, 0, stream>>>(p);
-    else k_raster<false><<<blocks, kRasterThreads, 0, stream>>>(p);
+    kernel<<<(sm_count * occ[t] + share - 1) / share, kRasterThreads, 0, stream>>>(p);
     note_launch();
 }
 

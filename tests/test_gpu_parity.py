@@ -8,7 +8,7 @@ import pytest
 
 from kat_scenes import flat_scene, one_surface_per_triangle
 from rosy_gb300 import scene as sc
-from rosy_gb300.graphics import render_scene
+from rosy_gb300.graphics import Graphics, render_scene
 
 COLOR_TOL = 1  # 1/255 per channel
 
@@ -238,6 +238,37 @@ def test_msaa_tiles_of_one_to_four_triangles(gpu, oracle, width, height, triangl
     assert np.array_equal(out["ids"], ref["ids"])
     assert np.array_equal(out["vis_depth"].view(np.uint32), ref["depth"].view(np.uint32))
     assert np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32)).max() <= COLOR_TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("chunk_stamps,small_extent,spread", [(8, 1, 1.0), (256, 16, 0.3), (32, 8, 0.08), (32, 16, 0.02)])
+def test_msaa_raster_parts(gpu, oracle, chunk_stamps, small_extent, spread):
+    """The four launches of a multisampled camera raster share out small, medium and screen-sized
+    records, boxes cut by the viewport among them: every sample's id and depth as the oracle's."""
+    s = sc.random_triangles(seed=43, triangles=900, width=307, height=205, shadow_size=64, texture_size=32)
+    v = s.vertices[:, 0:3].reshape(-1, 3, 3)
+    s.vertices[:, 0:3] = (1.4 * v[:, :1] + (v - v[:, :1]) * np.float32(spread)).reshape(-1, 3)
+    s.samples = 4
+    ref = oracle.render(s)
+    g = Graphics()
+    g.init(s.width, s.height, s.shadow_size, samples=4)
+    try:
+        g.set_asset(s)
+        g.set_graphic_objects(s.objects, s.surfaces)
+        g.set_draw_config(s.draw_config)
+        g.set_tuning(chunk_stamps, small_extent)
+        g.update(s.scene)
+        for timed in (False, True):  # side by side, then one after the other
+            g.set_stage_timing(timed)
+            g.render()
+            if g.sync_code() == 14:
+                g.render()
+            g.sync()
+            out = g.download()
+            assert np.array_equal(out["ids"], ref["ids"])
+            assert np.array_equal(out["vis_depth"].view(np.uint32), ref["depth"].view(np.uint32))
+    finally:
+        g.deinit()
 
 
 @pytest.mark.gpu
