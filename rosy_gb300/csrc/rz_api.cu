@@ -35,6 +35,8 @@ struct PassBuffers {
     uint32_t tile_capacity = 0;
     uint32_t* chunk_map = nullptr;
     uint32_t chunk_capacity = 0;
+    uint4* boxes = nullptr;  // blended pass: the boxes of the record groups
+    uint32_t box_capacity = 0;  // the record capacity they are sized for
 };
 
 template <class T>
@@ -198,7 +200,7 @@ struct rz_ctx {
     DrawConsts* d_camera_consts = nullptr;
     DrawConsts* d_blended_consts = nullptr;
     float4* d_varyings = nullptr;
-    uint4* d_tri_refs = nullptr;  // per opaque triangle: its draw and varying records (written by the camera setup)
+    uint4* d_tri_refs = nullptr;  // per opaque, then per blended triangle: its draw and varying records (written by the setups)
     uint32_t varying_count = 0, blended_varying_base = 0;
     bool layout_dirty = true;        // draw lists, pools and view table need a rebuild
 
@@ -267,6 +269,8 @@ void free_pass(PassBuffers& p) {
     dfree(p.small_records);
     dfree(p.tile_status);
     dfree(p.chunk_map);
+    dfree(p.boxes);
+    p.box_capacity = 0;
     p.record_capacity = p.small_capacity = p.tile_capacity = p.chunk_capacity = 0;
 }
 
@@ -298,6 +302,16 @@ int size_pass(rz_ctx* c, PassBuffers& p, uint32_t tris, uint64_t stamps_hint) {
         RZ_CUDA(c, dalloc(&p.chunk_map, (size_t)chunks), "chunk map");
         p.chunk_capacity = (uint32_t)chunks;
     }
+    return RZ_OK;
+}
+
+// The group boxes of a blended pass's records.
+int size_boxes(rz_ctx* c, PassBuffers& p) {
+    if (p.record_capacity <= p.box_capacity) return RZ_OK;
+    dfree(p.boxes);
+    p.box_capacity = 0;
+    RZ_CUDA(c, dalloc(&p.boxes, blend_box_count(p.record_capacity)), "blended record boxes");
+    p.box_capacity = p.record_capacity;
     return RZ_OK;
 }
 
@@ -743,7 +757,7 @@ int build_layout(rz_ctx* c) {
     RZ_CUDA(c, dalloc(&c->d_camera_consts, std::max<size_t>(opaque.size(), 1)), "camera constants");
     RZ_CUDA(c, dalloc(&c->d_blended_consts, std::max<size_t>(blended.size(), 1)), "blended constants");
     RZ_CUDA(c, dalloc(&c->d_varyings, std::max<size_t>((size_t)varyings, 1) * 8), "varying records");
-    RZ_CUDA(c, dalloc(&c->d_tri_refs, std::max<size_t>((size_t)opaque_tris, 1)), "triangle references");
+    RZ_CUDA(c, dalloc(&c->d_tri_refs, std::max<size_t>((size_t)opaque_tris + (size_t)blended_tris, 1)), "triangle references");
     for (int k = 0; k < 2; ++k) {
         std::vector<ViewRec> set = c->view_recs;
         for (ViewRec& r : set) {
@@ -777,6 +791,7 @@ int build_layout(rz_ctx* c) {
     int rc = size_pass(c, c->shadow_pass, c->shadow_tris, stamp_hint(c->shadow_tris, shadow));
     if (rc == RZ_OK) rc = size_pass(c, c->camera_pass, c->opaque_tris, stamp_hint(c->opaque_tris, pix));
     if (rc == RZ_OK && c->blended_tris) rc = size_pass(c, c->blended_pass, c->blended_tris, stamp_hint(c->blended_tris, pix));
+    if (rc == RZ_OK && c->blended_tris) rc = size_boxes(c, c->blended_pass);
     if (rc != RZ_OK) return rc;
     c->layout_dirty = false;
     return RZ_OK;
@@ -833,7 +848,7 @@ PassParams pass_params(rz_ctx* c, int kind) {
     p.tile_status = pb->tile_status;
     p.chunk_map = pb->chunk_map;
     p.chunk_capacity = pb->chunk_capacity;
-    p.tri_refs = kind == 1 ? c->d_tri_refs : nullptr;
+    p.tri_refs = kind == 1 ? c->d_tri_refs : kind == 2 ? c->d_tri_refs + c->opaque_tris : nullptr;
     return p;
 }
 
@@ -978,12 +993,14 @@ int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh
     if (c->blended_tris) {
         launch_prep_camera(c->d_blended_draws, c->blended_draw_count, c->d_objects, c->d_views, c->d_blended_consts, s);
         launch_setup(pass_params(c, 2), s);
+        launch_blend_boxes(c->blended_pass.records, &c->d_report->blended, c->blended_pass.record_capacity,
+                           c->blended_pass.boxes, s);
         ShadeParams bs = sh;
         bs.draws = c->d_blended_draws;
         bs.draw_count = c->blended_draw_count;
         bs.consts = c->d_blended_consts;
         bs.varying_count = c->varying_count;
-        bs.tri_refs = nullptr;
+        bs.tri_refs = c->d_tri_refs + c->opaque_tris;
         launch_vertex_range(bs, c->blended_varying_base, s);
     }
     return RZ_OK;
@@ -1096,8 +1113,9 @@ int enqueue_frame(rz_ctx* c) {
         bp.sh.draws = c->d_blended_draws;
         bp.sh.draw_count = c->blended_draw_count;
         bp.sh.consts = c->d_blended_consts;
-        bp.sh.tri_refs = nullptr;  // the blended triangles are looked up through their draws
+        bp.sh.tri_refs = c->d_tri_refs + c->opaque_tris;
         bp.records = c->blended_pass.records;
+        bp.boxes = c->blended_pass.boxes;
         bp.header = &c->d_report->blended;
         bp.error_flags = &c->d_report->camera_errors;
         bp.record_capacity = c->blended_pass.record_capacity;
@@ -1159,6 +1177,7 @@ int grow_queues(rz_ctx* c) {
     int rc = grow(c->shadow_pass, c->h_report->shadow);
     if (rc == RZ_OK) rc = grow(c->camera_pass, c->h_report->camera);
     if (rc == RZ_OK && c->blended_tris) rc = grow(c->blended_pass, c->h_report->blended);
+    if (rc == RZ_OK && c->blended_tris) rc = size_boxes(c, c->blended_pass);
     c->grow_records = c->grow_chunks = false;
     return rc;
 }

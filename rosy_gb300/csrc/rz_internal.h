@@ -185,8 +185,8 @@ struct PassParams {
     void* clear_ptr[2];
     size_t clear_bytes[2];
     uint32_t clear_count;
-    // opaque camera pass only (else null): per triangle that produced a record,
-    // its draw and its three varying record indices, for the shading
+    // camera passes only (else null): per triangle with valid indices, its draw and
+    // its three varying record indices, for the shading
     uint4* tri_refs;
 };
 
@@ -212,9 +212,8 @@ struct ShadeParams {
     int blended;                  // 1: k_shade stores the RGBA16F draw image (color16) for k_blend
     uint32_t samples;             // camera-pass samples per pixel of the views (1 or 4)
     uint32_t gbuffer;             // 1: the views have a G-buffer (ViewRec::gb_albedo)
-    // the opaque camera setup's per-triangle (draw, varying record of each vertex),
-    // indexed by pass-global triangle id; null for the blended list, whose
-    // triangles are then looked up through the draw list and the index buffer
+    // the camera setup's per-triangle (draw, varying record of each vertex), indexed
+    // by the triangle id of the pass (opaque or blended)
     const uint4* tri_refs;
 };
 
@@ -247,6 +246,7 @@ constexpr int32_t kDebugHalfWidth = 640;
 struct BlendParams {
     ShadeParams sh;               // blended draws, their constants and varyings
     const TriRecord* records;     // setup records of the blended triangles, in submission order
+    const uint4* boxes;           // the boxes of their groups (launch_blend_boxes)
     const PassHeader* header;
     const uint32_t* error_flags;  // the blended pass's flags: its records are not used after a look-back timeout
     uint32_t record_capacity;
@@ -281,6 +281,10 @@ void launch_vertex(const ShadeParams& p, cudaStream_t stream);
 // k_vertex over the varying records [first, varying_count) of the draws in p
 // (whose varying_base values start at `first`).
 void launch_vertex_range(const ShadeParams& p, uint32_t first, cudaStream_t stream);
+// The boxes of the groups of a pass's records, for launch_blend; blend_box_count of them at most.
+void launch_blend_boxes(const TriRecord* records, const PassHeader* header, uint32_t capacity, uint4* boxes,
+                        cudaStream_t stream);
+size_t blend_box_count(uint32_t capacity);
 void launch_blend(const BlendParams& p, cudaStream_t stream);
 // k_debug_prep: the overlay's `count` segments for each of the `view_count` views.
 void launch_debug_prep(const DebugPair* pairs, uint32_t count, const rz_debug_object* objects, const ViewRec* views,

@@ -753,19 +753,12 @@ __device__ bool shade_pixel(const ShadeParams& P, const ViewRec& VR, const rz_sc
                             int px, int py, float out[4], float* aux = nullptr, const PixelNdc* pn = nullptr) {
     uint32_t d;
     const float4* rec[3];
-    if (P.tri_refs) {  // the opaque list: the camera setup recorded the draw and the vertices
+    {  // the camera setup recorded the draw and the vertices
         const uint4 r = __ldg(&P.tri_refs[tri]);
         d = r.x;
         rec[0] = P.varyings + (size_t)r.y * kVaryingF4;
         rec[1] = P.varyings + (size_t)r.z * kVaryingF4;
         rec[2] = P.varyings + (size_t)r.w * kVaryingF4;
-    } else {
-        d = find_draw(P.draws, P.draw_count, tri);
-        const DrawRec& dl = P.draws[d];
-        const uint32_t t = tri - dl.tri_base;
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            rec[k] = P.varyings + (size_t)(__ldg(&P.indices[dl.first_index + 3u * t + k]) + dl.varying_base) * kVaryingF4;
     }
     const int32_t material = __ldg(&P.draws[d].material);
     const GpuMaterial* md = material >= 0 ? &P.materials[material] : nullptr;
@@ -1370,26 +1363,43 @@ void launch_subpixel_sources(const ShadeParams& p, cudaStream_t stream) {
 // blended list
 // ---------------------------------------------------------------------------
 
-// One CTA per 16x16 tile. The blended records overlapping the tile are
-// compacted into shared memory in submission order, then every pixel walks
-// them in that order: coverage with the raster's integer edge test, the
-// GREATER_OR_EQUAL test against the opaque depth (no write), fragmentMain
-// (discard honoured), and SRC_ALPHA / ONE_MINUS_SRC_ALPHA on colour, ONE / ZERO
-// on alpha, rounded to the RGBA16F draw image after each blend
+// One CTA per 16x16 tile. The blended records overlapping the tile are listed in
+// shared memory in submission order; every pixel takes from them, in that order, the
+// fragments that cover it (the raster's integer edge test) and pass the
+// GREATER_OR_EQUAL test against the opaque depth (no write); fragmentMain (discard
+// honoured); then SRC_ALPHA / ONE_MINUS_SRC_ALPHA on colour, ONE / ZERO on alpha,
+// rounded to the RGBA16F draw image after each blend
 // (src/Engine/Graphics.cpp:5654-5691). Then the sRGB blit.
-constexpr int kBlendBatch = 1024;
+//
+// Blending keeps the order; finding and shading the fragments does not need it.
+// * A tile does not look at every record: k_blend_boxes gives each group of 32
+//   consecutive records its box, a tile reads the boxes and then the records of the
+//   groups that meet it. Neighbours in the list are mostly neighbours on the screen
+//   (a mesh's triangles). Where they are not, every group meets every tile, and the
+//   tile tests the records it tested without the boxes, and 1/32 as many boxes.
+// * The fragments are shaded together: a pixel collects up to kBlendRound of them,
+//   the tile lists them (the first ones of all pixels, the second ones, ...), the
+//   block shades the list with all lanes busy, and each pixel blends its own in
+//   order. Shaded where they are met, a triangle of a few pixels ran the fragment
+//   stage for a few lanes of a warp.
+// 1279x717, 12,288 blended triangles (a median 4 square pixels) of 49,152: the frame
+// went from 636 to 125 us.
+constexpr int kBlendBatch = 512;   // records (or overlay segments) listed at a time
+constexpr int kBlendRound = 4;     // fragments a pixel collects before the tile shades them
+constexpr int kBlendGroup = 32;    // records of a group box
+constexpr int kBlendItems = 256 * kBlendRound;
 
 // Ordered compaction of the items [start, min(start + kBlendBatch, n)) that `hit`
-// selects (4 consecutive items per thread) into s_list, in item order; returns
+// selects (kPer consecutive items per thread) into s_list, in item order; returns
 // their count. Every thread of the 256-thread CTA calls it.
-template <class Hit>
+template <int kPer, class Hit>
 __device__ __forceinline__ uint32_t compact_batch(uint32_t start, uint32_t n, int tid, uint32_t* s_list,
                                                   uint32_t* s_count, Hit hit) {
     const int lane = tid & 31, warp = tid >> 5;
     uint32_t mask = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const uint32_t r = start + 4 * tid + k;
+    for (int k = 0; k < kPer; ++k) {
+        const uint32_t r = start + kPer * tid + k;
         if (r < n && hit(r)) mask |= 1u << k;
     }
     const uint32_t cnt = __popc(mask);
@@ -1409,8 +1419,8 @@ __device__ __forceinline__ uint32_t compact_batch(uint32_t start, uint32_t n, in
     }
     uint32_t pos = base + incl - cnt;
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (mask & (1u << k)) s_list[pos++] = start + 4 * tid + k;
+    for (int k = 0; k < kPer; ++k)
+        if (mask & (1u << k)) s_list[pos++] = start + kPer * tid + k;
     __syncthreads();
     return total;
 }
@@ -1436,10 +1446,101 @@ __device__ __forceinline__ bool debug_covers(const DebugSeg& s, int32_t PX, int3
     return true;
 }
 
-__global__ void __launch_bounds__(256) k_blend(BlendParams B) {
+// The box (pixels, inclusive) and the first and last view of every group of
+// kBlendGroup records: (x0 | y0 << 16, x1 | y1 << 16, view, view). One warp per group.
+__global__ void __launch_bounds__(256) k_blend_boxes(const TriRecord* __restrict__ records, const PassHeader* __restrict__ header,
+                                                     uint32_t capacity, uint4* __restrict__ boxes) {
+    const uint32_t n = min(header->records, capacity), groups = (n + kBlendGroup - 1) / kBlendGroup;
+    const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < groups; g += warps) {
+        const uint32_t r = g * kBlendGroup + lane;
+        uint32_t x0 = 0xffffu, y0 = 0xffffu, x1 = 0u, y1 = 0u, v0 = 0xffffffffu, v1 = 0u;
+        if (r < n) {
+            const TriRecord& rec = records[r];
+            x0 = rec.p0 & 0xffffu;
+            y0 = rec.p0 >> 16;
+            x1 = rec.p1 & 0xffffu;
+            y1 = rec.p1 >> 16;
+            v0 = v1 = rec.view & kViewMask;
+        }
+        x0 = __reduce_min_sync(0xffffffffu, x0);
+        y0 = __reduce_min_sync(0xffffffffu, y0);
+        x1 = __reduce_max_sync(0xffffffffu, x1);
+        y1 = __reduce_max_sync(0xffffffffu, y1);
+        v0 = __reduce_min_sync(0xffffffffu, v0);
+        v1 = __reduce_max_sync(0xffffffffu, v1);
+        if (lane == 0) boxes[g] = make_uint4(x0 | (y0 << 16), x1 | (y1 << 16), v0, v1);
+    }
+}
+
+__device__ __forceinline__ bool box_meets(uint32_t p0, uint32_t p1, int tx0, int ty0) {
+    const int x0 = p0 & 0xffff, y0 = p0 >> 16, x1 = p1 & 0xffff, y1 = p1 >> 16;
+    return x1 >= tx0 && x0 <= tx0 + 15 && y1 >= ty0 && y0 <= ty0 + 15;
+}
+
+// The samples of pixel (px, py) (bits; bit 0 without multisampling) that a blended
+// record covers and whose opaque depth it passes.
+template <bool kMsaa>
+__device__ __forceinline__ uint32_t blend_samples(const TriRecord& rec, int px, int py, const float* dst_depth) {
+    const int4* src = reinterpret_cast<const int4*>(&rec);
+    const int4 q0 = __ldg(src), q1 = __ldg(src + 1);
+    const float dzdy = __int_as_float(__ldg(reinterpret_cast<const int*>(src + 2)));
+    const int32_t X[3] = {q0.x, q0.z, q1.x}, Y[3] = {q0.y, q0.w, q1.y};
+    const float z0 = __int_as_float(q1.z), dzdx = __int_as_float(q1.w);
+    uint32_t pass = 0;
+#pragma unroll
+    for (int k = 0; k < (kMsaa ? kMsaaSamples : 1); ++k) {
+        const int32_t PX = px * 256 + (kMsaa ? msaa_x(k) : 128), PY = py * 256 + (kMsaa ? msaa_y(k) : 128);
+        bool in = true;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int a = (i + 1) % 3, b = (i + 2) % 3;
+            const int32_t dx = X[b] - X[a], dy = Y[b] - Y[a];
+            const bool tl = dy < 0 || (dy == 0 && dx > 0);
+            const int64_t E = (int64_t)dx * (int64_t)(PY - Y[a]) - (int64_t)dy * (int64_t)(PX - X[a]);
+            in = in && (E > 0 || (E == 0 && tl));
+        }
+        if (!in) continue;
+        float z = fmaf(dzdx, (float)(PX - X[0]), fmaf(dzdy, (float)(PY - Y[0]), z0));
+        if (!(z > 0.0f)) z = 0.0f;
+        if (z > 1.0f) z = 1.0f;
+        if (z >= dst_depth[k]) pass |= 1u << k;
+    }
+    return pass;
+}
+
+// Shades the listed fragments: item i is the triangle item_id[i] (id + 1) at pixel
+// item_px[i] (row * 16 + column) of the tile; its colour goes to item_out[i], and
+// item_id[i] becomes 0 where it is discarded.
+template <bool kLit>
+__device__ __forceinline__ void shade_fragments(const ShadeParams& P, const ViewRec& VR, const float* s_srgb, const TileNdc& tn,
+                                                int tx0, int ty0, int tid, int total, uint32_t* item_id,
+                                                const uint8_t* item_px, float4* item_out) {
+    const Sampler smp{&P, s_srgb};
+#pragma unroll 1
+    for (int i = tid; i < total; i += 256) {
+        const int t = item_px[i], lx = t & 15, ly = t >> 4;
+        const PixelNdc pn{tn.x[lx], tn.y[ly], tn.x[lx & ~1], tn.y[ly & ~1], tn.x[lx | 1], tn.y[ly | 1]};
+        float o[4];
+        if (shade_pixel<kLit>(P, VR, *VR.scene, smp, item_id[i] - 1u, tx0 + lx, ty0 + ly, o, nullptr, &pn))
+            item_out[i] = make_float4(o[0], o[1], o[2], o[3]);
+        else
+            item_id[i] = 0u;
+    }
+}
+
+template <bool kMsaa>
+__global__ void __launch_bounds__(256, 4) k_blend(BlendParams B) {
+    constexpr int kSamples = kMsaa ? kMsaaSamples : 1;
     __shared__ float s_srgb[256];
+    __shared__ uint32_t s_groups[256];
     __shared__ uint32_t s_list[kBlendBatch];
-    __shared__ uint32_t s_count[256 / 32 + 1];
+    __shared__ uint2 s_box[kBlendBatch];
+    __shared__ uint32_t s_count[kBlendRound][256 / 32];
+    __shared__ TileNdc s_ndc;
+    __shared__ uint32_t s_id[kBlendItems];
+    __shared__ uint8_t s_px[kBlendItems];
+    __shared__ float4 s_out[kBlendItems];
     __shared__ uint32_t s_view;
     const ShadeParams& P = B.sh;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -1455,102 +1556,142 @@ __global__ void __launch_bounds__(256) k_blend(BlendParams B) {
     const bool inside = px < VR.width && py < VR.height;
     const size_t p = inside ? (size_t)py * VR.width + px : 0;
     const size_t plane = (size_t)VR.width * VR.height;
-    const int nsamples = VR.samples > 1 ? kMsaaSamples : 1;
+    if (tid < 16) s_ndc.x[tid] = ndc(tx0 + tid, VR.width);
+    else if (tid < 32) s_ndc.y[tid - 16] = ndc(ty0 + tid - 16, VR.height);
     // per coverage sample: the RGBA16F value and the opaque depth it is tested against
-    float col[kMsaaSamples][4];
-    float dst_depth[kMsaaSamples];
+    float col[kSamples][4];
+    float dst_depth[kSamples];
 #pragma unroll
-    for (int k = 0; k < kMsaaSamples; ++k) {
+    for (int k = 0; k < kSamples; ++k) {
         dst_depth[k] = 0.f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) col[k][i] = 0.f;
-        if (inside && k < nsamples) {
+        if (inside) {
             const uint2 c = VR.color16[p + k * plane];
             const __half2 rg = *reinterpret_cast<const __half2*>(&c.x), ba = *reinterpret_cast<const __half2*>(&c.y);
             col[k][0] = __low2float(rg);
             col[k][1] = __high2float(rg);
             col[k][2] = __low2float(ba);
             col[k][3] = __high2float(ba);
-            dst_depth[k] = nsamples > 1 ? __uint_as_float((uint32_t)(VR.vis[p + k * plane] >> 32)) : VR.depth[p];
+            dst_depth[k] = kMsaa ? __uint_as_float((uint32_t)(VR.vis[p + k * plane] >> 32)) : VR.depth[p];
         }
     }
-    const Sampler smp{&P, s_srgb};
+    const bool lit = lit_view(*VR.scene);
     // a pass whose look-back gave up has records at unreliable slots: blend none of them
     const bool records_ok = !B.error_flags || !(*B.error_flags & kErrLookbackTimeout);
     const uint32_t n = records_ok ? min(B.header->records, B.record_capacity) : 0u;
+    const uint32_t groups = (n + kBlendGroup - 1) / kBlendGroup;
     const int lane = tid & 31, warp = tid >> 5;
-    for (uint32_t start = 0; start < n; start += kBlendBatch) {
-        // ordered compaction of the records whose box meets this tile (4 per thread)
-        uint32_t mask = 0;
+    for (uint32_t first = 0; first < groups; first += 256) {
+        const uint32_t ngroups = compact_batch<1>(first, groups, tid, s_groups, s_count[0], [&](uint32_t g) {
+            const uint4 b = __ldg(&B.boxes[g]);
+            return b.z <= view && view <= b.w && box_meets(b.x, b.y, tx0, ty0);
+        });
+        for (uint32_t gs = 0; gs < ngroups; gs += kBlendBatch / kBlendGroup) {
+            // the groups' records whose box meets the tile, in order: kPer groups per warp, a record per lane
+            constexpr int kPer = kBlendBatch / kBlendGroup / 8;
+            uint32_t hits[kPer], rec_of[kPer], found = 0;
+            uint2 box[kPer];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t r = start + 4 * tid + k;
-            if (r < n) {
-                const TriRecord& rec = B.records[r];
-                const int bx0 = rec.p0 & 0xffff, by0 = rec.p0 >> 16, bx1 = rec.p1 & 0xffff, by1 = rec.p1 >> 16;
-                if ((rec.view & kViewMask) == view && bx1 >= tx0 && bx0 <= tx0 + 15 && by1 >= ty0 && by0 <= ty0 + 15)
-                    mask |= 1u << k;
-            }
-        }
-        const uint32_t cnt = __popc(mask);
-        uint32_t incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        __syncthreads();
-        if (lane == 31) s_count[warp] = incl;
-        __syncthreads();
-        uint32_t base = 0, total = 0;
-        for (int w = 0; w < 8; ++w) {
-            if (w < warp) base += s_count[w];
-            total += s_count[w];
-        }
-        uint32_t pos = base + incl - cnt;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (mask & (1u << k)) s_list[pos++] = start + 4 * tid + k;
-        __syncthreads();
-        if (inside) {
-            for (uint32_t j = 0; j < total; ++j) {
-                const TriRecord& rec = B.records[s_list[j]];
-                const int bx0 = rec.p0 & 0xffff, by0 = rec.p0 >> 16, bx1 = rec.p1 & 0xffff, by1 = rec.p1 >> 16;
-                if (px < bx0 || px > bx1 || py < by0 || py > by1) continue;
-                const int32_t X[3] = {rec.X0, rec.X1, rec.X2}, Y[3] = {rec.Y0, rec.Y1, rec.Y2};
-                uint32_t pass = 0;  // samples covered and in front of the opaque depth
-                for (int k = 0; k < nsamples; ++k) {
-                    const int32_t PX = px * 256 + (nsamples > 1 ? msaa_x(k) : 128);
-                    const int32_t PY = py * 256 + (nsamples > 1 ? msaa_y(k) : 128);
-                    bool in = true;
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        const int a = (i + 1) % 3, b = (i + 2) % 3;
-                        const int32_t dx = X[b] - X[a], dy = Y[b] - Y[a];
-                        const bool tl = dy < 0 || (dy == 0 && dx > 0);
-                        const int64_t E = (int64_t)dx * (int64_t)(PY - Y[a]) - (int64_t)dy * (int64_t)(PX - X[a]);
-                        in = in && (E > 0 || (E == 0 && tl));
+            for (int q = 0; q < kPer; ++q) {
+                const uint32_t gi = gs + kPer * warp + q;
+                bool hit = false;
+                rec_of[q] = 0u;
+                box[q] = make_uint2(0u, 0u);
+                if (gi < ngroups) {
+                    rec_of[q] = s_groups[gi] * kBlendGroup + lane;
+                    if (rec_of[q] < n) {
+                        const TriRecord& rec = B.records[rec_of[q]];
+                        box[q] = make_uint2(rec.p0, rec.p1);
+                        hit = (rec.view & kViewMask) == view && box_meets(rec.p0, rec.p1, tx0, ty0);
                     }
-                    if (!in) continue;
-                    float z = fmaf(rec.dzdx, (float)(PX - rec.X0), fmaf(rec.dzdy, (float)(PY - rec.Y0), rec.z0));
-                    if (!(z > 0.0f)) z = 0.0f;
-                    if (z > 1.0f) z = 1.0f;
-                    if (z >= dst_depth[k]) pass |= 1u << k;
                 }
-                if (!pass) continue;
-                float s4[4];
-                if (!shade_pixel(P, VR, *VR.scene, smp, rec.id - 1u, px, py, s4)) continue;
-                const float a = s4[3];
+                hits[q] = __ballot_sync(0xffffffffu, hit);
+                found += __popc(hits[q]);
+            }
+            if (lane == 0) s_count[0][warp] = found;
+            __syncthreads();
+            uint32_t at = 0, total = 0;
+            for (int w = 0; w < 8; ++w) {
+                if (w < warp) at += s_count[0][w];
+                total += s_count[0][w];
+            }
 #pragma unroll
-                for (int k = 0; k < kMsaaSamples; ++k) {
-                    if (!(pass & (1u << k))) continue;
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) col[k][i] = half_round(s4[i] * a + col[k][i] * (1.0f - a));
-                    col[k][3] = half_round(a);
+            for (int q = 0; q < kPer; ++q) {
+                if ((hits[q] >> lane) & 1u) {
+                    const uint32_t i = at + __popc(hits[q] & ((1u << lane) - 1u));
+                    s_list[i] = rec_of[q];
+                    s_box[i] = box[q];
                 }
+                at += __popc(hits[q]);
+            }
+            __syncthreads();
+            uint32_t j = 0;  // the pixel's next record of the list
+            bool more = total != 0;
+            while (more) {
+                // up to kBlendRound fragments of the pixel, in order
+                uint32_t frag[kBlendRound], pass_of = 0, nf = 0;
+#pragma unroll
+                for (int r = 0; r < kBlendRound; ++r) frag[r] = 0u;
+                if (inside) {
+                    for (; j < total && nf < kBlendRound; ++j) {
+                        const uint2 b = s_box[j];
+                        const int bx0 = b.x & 0xffff, by0 = b.x >> 16, bx1 = b.y & 0xffff, by1 = b.y >> 16;
+                        if (px < bx0 || px > bx1 || py < by0 || py > by1) continue;
+                        const TriRecord& rec = B.records[s_list[j]];
+                        const uint32_t pass = blend_samples<kMsaa>(rec, px, py, dst_depth);
+                        if (!pass) continue;
+                        const uint32_t id = rec.id;
+#pragma unroll
+                        for (int r = 0; r < kBlendRound; ++r)
+                            if (nf == (uint32_t)r) frag[r] = id;
+                        pass_of |= pass << (4 * nf);
+                        ++nf;
+                    }
+                }
+                uint32_t before[kBlendRound];
+#pragma unroll
+                for (int r = 0; r < kBlendRound; ++r) {
+                    const uint32_t m = __ballot_sync(0xffffffffu, nf > (uint32_t)r);
+                    before[r] = __popc(m & ((1u << lane) - 1u));
+                    if (lane == 0) s_count[r][warp] = __popc(m);
+                }
+                __syncthreads();
+                uint64_t slots = 0;  // where the pixel's fragments sit in the list, 16 bits each
+                uint32_t items = 0;
+#pragma unroll
+                for (int r = 0; r < kBlendRound; ++r) {
+                    uint32_t i = items + before[r];
+                    for (int w = 0; w < 8; ++w) {
+                        if (w < warp) i += s_count[r][w];
+                        items += s_count[r][w];
+                    }
+                    slots |= (uint64_t)i << (16 * r);
+                    if (nf > (uint32_t)r) {
+                        s_id[i] = frag[r];
+                        s_px[i] = (uint8_t)tid;
+                    }
+                }
+                __syncthreads();
+                if (lit) shade_fragments<true>(P, VR, s_srgb, s_ndc, tx0, ty0, tid, (int)items, s_id, s_px, s_out);
+                else shade_fragments<false>(P, VR, s_srgb, s_ndc, tx0, ty0, tid, (int)items, s_id, s_px, s_out);
+                __syncthreads();
+                for (uint32_t r = 0; r < nf; ++r) {
+                    const uint32_t i = (uint32_t)(slots >> (16 * r)) & 0xffffu;
+                    if (s_id[i] == 0u) continue;  // discarded
+                    const float4 o = s_out[i];
+                    const float s4[3] = {o.x, o.y, o.z}, a = o.w;
+#pragma unroll
+                    for (int k = 0; k < kSamples; ++k) {
+                        if (!((pass_of >> (4 * r + k)) & 1u)) continue;
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) col[k][c] = half_round(s4[c] * a + col[k][c] * (1.0f - a));
+                        col[k][3] = half_round(a);
+                    }
+                }
+                more = __syncthreads_or(inside && j < total) != 0;
             }
         }
-        __syncthreads();
     }
     // Debug-line overlay after the blended list (src/Engine/Graphics.cpp:5694-5738): the same
     // blend state and depth test, depth writes off; a covered sample in front of the opaque
@@ -1558,10 +1699,9 @@ __global__ void __launch_bounds__(256) k_blend(BlendParams B) {
     if (B.debug_count) {
         const DebugSeg* __restrict__ segs = B.debug + (size_t)view * B.debug_count;
         for (uint32_t start = 0; start < B.debug_count; start += kBlendBatch) {
-            const uint32_t total = compact_batch(start, B.debug_count, tid, s_list, s_count, [&](uint32_t r) {
+            const uint32_t total = compact_batch<2>(start, B.debug_count, tid, s_list, s_count[0], [&](uint32_t r) {
                 const DebugSeg& sg = segs[r];
-                const int bx0 = sg.p0 & 0xffff, by0 = sg.p0 >> 16, bx1 = sg.p1 & 0xffff, by1 = sg.p1 >> 16;
-                return sg.live && bx1 >= tx0 && bx0 <= tx0 + 15 && by1 >= ty0 && by0 <= ty0 + 15;
+                return sg.live && box_meets(sg.p0, sg.p1, tx0, ty0);
             });
             if (inside) {
                 for (uint32_t j = 0; j < total; ++j) {
@@ -1569,15 +1709,16 @@ __global__ void __launch_bounds__(256) k_blend(BlendParams B) {
                     const int bx0 = sg.p0 & 0xffff, by0 = sg.p0 >> 16, bx1 = sg.p1 & 0xffff, by1 = sg.p1 >> 16;
                     if (px < bx0 || px > bx1 || py < by0 || py > by1) continue;
                     uint32_t pass = 0;  // samples covered and in front of the opaque depth
-                    for (int k = 0; k < nsamples; ++k) {
-                        const int32_t PX = px * 256 + (nsamples > 1 ? msaa_x(k) : 128);
-                        const int32_t PY = py * 256 + (nsamples > 1 ? msaa_y(k) : 128);
+#pragma unroll
+                    for (int k = 0; k < kSamples; ++k) {
+                        const int32_t PX = px * 256 + (kMsaa ? msaa_x(k) : 128);
+                        const int32_t PY = py * 256 + (kMsaa ? msaa_y(k) : 128);
                         float z;
                         if (debug_covers(sg, PX, PY, z) && z >= dst_depth[k]) pass |= 1u << k;
                     }
                     if (!pass) continue;
 #pragma unroll
-                    for (int k = 0; k < kMsaaSamples; ++k) {
+                    for (int k = 0; k < kSamples; ++k) {
                         if (!(pass & (1u << k))) continue;
 #pragma unroll
                         for (int i = 0; i < 3; ++i) col[k][i] = half_round(sg.rgb[i]);
@@ -1591,14 +1732,27 @@ __global__ void __launch_bounds__(256) k_blend(BlendParams B) {
     if (!inside) return;
     float o[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        o[i] = nsamples > 1 ? resolve4(col[0][i], col[1][i], col[2][i], col[3][i]) : col[0][i];
+    for (int i = 0; i < 4; ++i) {
+        if constexpr (kMsaa) o[i] = resolve4(col[0][i], col[1][i], col[2][i], col[3][i]);
+        else o[i] = col[0][i];
+    }
     VR.color[p] = encode_srgb8(o[0]) | (encode_srgb8(o[1]) << 8) | (encode_srgb8(o[2]) << 16) | (encode_unorm8(o[3]) << 24);
 }
 
+void launch_blend_boxes(const TriRecord* records, const PassHeader* header, uint32_t capacity, uint4* boxes,
+                        cudaStream_t stream) {
+    const uint32_t groups = (capacity + kBlendGroup - 1) / kBlendGroup;
+    if (groups == 0) return;
+    k_blend_boxes<<<std::min((groups + 7) / 8, 1024u), 256, 0, stream>>>(records, header, capacity, boxes);
+    note_launch();
+}
+
+size_t blend_box_count(uint32_t capacity) { return (capacity + (size_t)kBlendGroup - 1) / kBlendGroup; }
+
 void launch_blend(const BlendParams& p, cudaStream_t stream) {
     if (p.sh.shade_blocks == 0) return;
-    k_blend<<<p.sh.shade_blocks, dim3(16, 16), 0, stream>>>(p);
+    if (p.sh.samples > 1) k_blend<true><<<p.sh.shade_blocks, dim3(16, 16), 0, stream>>>(p);
+    else k_blend<false><<<p.sh.shade_blocks, dim3(16, 16), 0, stream>>>(p);
     note_launch();
 }
 

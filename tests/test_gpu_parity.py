@@ -272,6 +272,25 @@ def test_msaa_raster_parts(gpu, oracle, chunk_stamps, small_extent, spread):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("samples", [1, 4])
+@pytest.mark.parametrize("width,height,triangles,spread,mask", [
+    (48, 40, 24000, 0.05, False),  # over 8,192 records (a window of group boxes), hundreds to a tile
+    (33, 17, 1500, 0.8, True),     # tens of fragments to a pixel, some discarded
+    (16, 16, 31, 1.0, False),      # less than a group
+    (64, 1, 33, 1.0, False)])
+def test_blended_lists(gpu, oracle, samples, width, height, triangles, spread, mask):
+    """Blended lists of less than a group to several windows of groups, and pixels of many rounds."""
+    s = sc.random_triangles(seed=47, triangles=triangles, width=width, height=height, shadow_size=64, texture_size=32)
+    v = s.vertices[:, 0:3].reshape(-1, 3, 3)
+    s.vertices[:, 0:3] = (v[:, :1] + (v - v[:, :1]) * np.float32(spread)).reshape(-1, 3)
+    s = sc.with_blended(s, 0.95, alpha=0.3, mask_cutoff=0.4 if mask else None)
+    s.samples = samples
+    ref, out = run(s, oracle)
+    assert np.array_equal(out["ids"], ref["ids"])
+    assert np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32)).max() <= COLOR_TOL
+
+
+@pytest.mark.gpu
 def test_shading_error_against_fp64_oracle(gpu, oracle):
     """The oracle also shades in float64; the GPU's 8-bit sRGB colour stays within
     1.5 levels of that (0.5 of it is the 8-bit rounding itself)."""
