@@ -19,15 +19,15 @@
 //   weights transposed and the taps mirrored.
 //   weight gradient: D[(tap, cin), cout] = sum over pixels of
 //     X[pixel + offset(tap), cin] * dY[pixel, cout]
-//   One persistent CTA per half SM walks 64-pixel x 4-row tiles; it stages X
-//   transposed (8 pixels of one channel per 16 bytes) for the three horizontal
-//   shifts, laid out so that the (tap, channel) rows of an M block sit at a
-//   uniform stride, and accumulates D in tensor memory over all its tiles.
+//   One persistent CTA per SM walks 112-pixel x 4-row tiles of the same planes
+//   (here the contraction runs over the pixels, so the operands are MN-major) and
+//   accumulates D in tensor memory over all its tiles.
 //
-// Shared-memory operands use the canonical K-major layout without swizzle:
-// 8 x 16-byte core matrices; the descriptor's leading byte offset is the
-// distance between core matrices along K and the stride byte offset the
-// distance between 8-row groups along M (or N).
+// Shared-memory operands use the canonical layouts without swizzle: 8 x 16-byte
+// core matrices; the descriptor's leading byte offset is the distance between
+// core matrices along K and the stride byte offset the distance between groups of
+// 8 along M (or N). K-major, a core matrix is 8 rows of M (or N) by 8 of K;
+// MN-major, 8 of K by 8 of M (or N).
 //
 // Every wait on a copy or tensor-core completion barrier has a time limit
 // (about a second; rz_upsampler_set_wait_limit can shorten it); a wait that runs
@@ -52,7 +52,7 @@
 namespace rz {
 namespace up {
 
-constexpr int kThreads = 128;      // weight-gradient and self-test kernels
+constexpr int kThreads = 128;      // self-test kernel
 constexpr int kConvEpilogueWarps = 16;  // convolution: one epilogue warp per (TMEM lane quadrant, tile row),
 constexpr int kConvThreads = 32 * (kConvEpilogueWarps + 2);  // then a TMA warp and an MMA warp
 constexpr int kTileW = 128;  // conv: MMA rows (M = 128), one row segment of output pixels
@@ -63,8 +63,9 @@ constexpr int kConvStages = 4; // conv: halo buffers in flight (TMA loads ahead 
 // kTileOut + 1 (whose 3x3 window runs past the halo) are computed and dropped
 constexpr int kHaloW = kTileW;
 constexpr int kTileOut = kHaloW - 2;
-constexpr int kWgKP = 64;    // weight gradient: pixels per tile row (K chunk)
-constexpr int kWgRows = 4;   // weight gradient: rows per tile
+constexpr int kWgKP = 112;   // weight gradient: output pixels per tile row (7 MMA steps; with the halo one TMA box)
+constexpr int kWgRows = 4;   // weight gradient: output rows per tile
+constexpr int kWgThreads = 32 * 6;  // a TMA warp, an MMA warp, four for the bias gradient and the epilogue
 constexpr long long kWaitCycles = 2000000000ll;  // about one second at 2 GHz
 constexpr uint32_t kErrMmaTimeout = 1u << 0;
 
@@ -155,18 +156,6 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {  // 
 
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {  // one full warp
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-
-// 16-byte asynchronous global -> shared copy; valid == false writes zeros (src must still be a mapped address).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kPending>
-__device__ __forceinline__ void cp_async_wait_group() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -661,142 +650,211 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
 // ---- weight gradient ------------------------------------------------------------
 
 struct WgradArgs {
-    const __nv_bfloat16* x;   // planar [CIN / 8][H][W][8]: the layer's input
-    const __nv_bfloat16* dy;  // planar [N / 8][H][W][8]: gradient of the loss sum w.r.t. the pre-activation output
     float* dw;                // [N][9][CIN], accumulated
     float* db;                // [N], accumulated
     int W, H;
     uint32_t* err;
-    long long wait_cycles;    // bound of each wait for the previous tile's MMAs
+    long long wait_cycles;    // bound of each pipeline wait
 };
 
+// Shared memory of the weight gradient: a ring of stages, each with a tile's X halo
+// ([row][8-channel group][pixel], kWgRows + 2 rows of kHaloW pixels) and its dY rows
+// ([row][8-channel group][pixel], kWgKP pixels). An M block is 16 consecutive
+// (row, group) planes from output row r on: the three vertical taps' channels, then
+// planes of further rows (or of the dY that follows), whose products are not read.
 template <int CIN, int N>
 struct WgSmem {
     static constexpr int G = CIN / 8;
-    static constexpr int NB = (9 * CIN + 127) / 128;         // M blocks of 128 (tap, channel) rows
-    static constexpr uint32_t S_CG = kWgKP * 16;              // between 8-channel groups (M direction)
-    static constexpr uint32_t S_KX = G * S_CG;                // between horizontal shifts
-    static constexpr uint32_t S_ROW = 3 * S_KX;               // between halo rows
-    static constexpr uint32_t XT_USED = (kWgRows + 2) * S_ROW;
-    static constexpr uint32_t XT_READ = (kWgRows - 1) * S_ROW + 16 * NB * S_CG;  // end of the furthest M block read
-    static constexpr uint32_t XT_BYTES = XT_USED > XT_READ ? XT_USED : XT_READ;
-    static constexpr uint32_t S_COG = kWgKP * 16;             // between 8-channel groups of dY (N direction)
-    static constexpr uint32_t S_DYROW = (N / 8) * S_COG;
-    static constexpr uint32_t DY_OFF = (XT_BYTES + 127) / 128 * 128;
+    static constexpr int GN = N / 8;
+    static constexpr uint32_t S_G = kHaloW * 16;              // between channel planes of X (M direction)
+    static constexpr uint32_t S_ROW = G * S_G;                // between halo rows
+    static constexpr uint32_t X_BYTES = (kWgRows + 2) * S_ROW;
+    static constexpr uint32_t X_READ = (kWgRows - 1) * S_ROW + 16 * S_G;  // end of the furthest M block
+    static constexpr uint32_t S_COG = kWgKP * 16;             // between channel planes of dY (N direction)
+    static constexpr uint32_t S_DYROW = GN * S_COG;
+    static constexpr uint32_t DY_OFF = X_BYTES;
     static constexpr uint32_t DY_BYTES = kWgRows * S_DYROW;
-    static constexpr uint32_t BAR_OFF = (DY_OFF + DY_BYTES + 127) / 128 * 128;
-    static constexpr uint32_t BYTES = BAR_OFF + 16;
-    static constexpr uint32_t TMEM_COLS = tmem_cols_for(NB * N);
+    static constexpr uint32_t TX_BYTES = X_BYTES + DY_BYTES;  // what one tile's TMA loads write
+    static constexpr uint32_t STAGE = (TX_BYTES + 1023) / 1024 * 1024;
+    static constexpr int NS = 200 * 1024 / STAGE;             // 2 (32 -> 32 channels) or 3 tiles in flight
+    static constexpr uint32_t BAR_OFF = NS * STAGE;
+    static constexpr uint32_t NBAR = 2 * NS + 1;              // full, empty, done
+    static constexpr uint32_t BYTES = BAR_OFF + NBAR * 8 + 16;
+    static constexpr uint32_t TMEM_COLS = tmem_cols_for(kWgRows * 3 * N);  // an accumulator per tile row and horizontal tap
+    static_assert(X_READ <= STAGE, "an M block stays inside its stage");
+    static_assert(NS >= 2 && BYTES <= 227 * 1024, "the ring fits shared memory");
+    static_assert(S_COG % 128 == 0 && S_G % 128 == 0, "TMA destinations 128-byte aligned");
+    static_assert(kWgKP + 2 <= kHaloW && kWgKP % 16 == 0, "a tile row's halo is one box, its pixels whole MMA steps");
 };
 
+// Persistent, warp-specialised weight gradient. The activations lie as the tensor
+// cores want them for a contraction over pixels: a plane holds 8 channels of a pixel
+// in 16 bytes, pixels in a row, which is the MN-major layout without swizzle (8
+// pixels x 8 channels are one core matrix), so the tiles go from global to shared
+// memory by TMA and into the MMAs without a transposition. A horizontal tap is a
+// start address shifted by a pixel, the vertical taps are M rows.
+//   warp 0 (one thread)  TMA-loads tile j's X halo and dY into stage j % NS;
+//   warp 1 (one thread)  issues the tile's MMAs: per output row, 16 pixels and
+//                        horizontal tap one M = 128, N = cout, K = 16 MMA, into the
+//                        accumulator of that row and tap, which sums over all the
+//                        CTA's tiles (a row's own, so that a sum is short: with one
+//                        for the four rows the gradients of 957x539 were 8e-6 off the
+//                        float64 sums of the same bf16 values, 3e-6 as it is);
+//   warps 2-5            add up the tile's dY (the bias gradient), and at the end
+//                        add the accumulators to the gradient.
+// Borders and the pixels past a ragged edge are zeros from the tensor map.
+// Bound by the operand reads of N = 32 MMAs (4 KB of X per 32 cycles at 128 bytes a
+// cycle), 11 us a layer of 960x540. As a kernel that transposed X and dY through
+// 2-byte loads into registers, the four layers took 529 of a training step's 709
+// us; a step of two 960x540 frames goes from 1,250 to 555 us.
 template <int CIN, int N>
-__global__ void __launch_bounds__(kThreads) k_wgrad(WgradArgs a) {
+__global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __grid_constant__ CUtensorMap x_map,
+                                                         const __grid_constant__ CUtensorMap dy_map) {
     using L = WgSmem<CIN, N>;
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char* sX = smem;
-    unsigned char* sD = smem + L::DY_OFF;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::BAR_OFF + 8);
+    constexpr int NS = L::NS;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);  // [NS]
+    uint64_t* empty = full + NS;                                       // [NS]: the MMAs and the four summing warps
+    uint64_t* done = empty + NS;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::BAR_OFF + L::NBAR * 8);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tiles_x = (a.W + kWgKP - 1) / kWgKP;
+    const int ntiles = tiles_x * ((a.H + kWgRows - 1) / kWgRows);
+    const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     if (warp == 0) tmem_alloc(tmem_slot, L::TMEM_COLS);
-    if (tid == 0) mbar_init(bar, 1);
+    if (tid == 0) {
+        for (int b = 0; b < NS; ++b) {
+            mbar_init(&full[b], 1);
+            mbar_init(&empty[b], 1 + 4);
+        }
+        mbar_init(done, 1);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const int tiles_x = (a.W + kWgKP - 1) / kWgKP, tiles_y = (a.H + kWgRows - 1) / kWgRows;
-    const int ntiles = tiles_x * tiles_y;
-    const int ci = tid % CIN, xgroups = kThreads / CIN;
-    const int co = tid % N, dgroups = kThreads / N;
-    float dbsum = 0.0f;
     bool ok = true;
-    int iter = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++iter) {
-        if (iter > 0) ok = ok && mbar_wait(bar, (uint32_t)(iter - 1) & 1u, a.wait_cycles);
-        if (!__syncthreads_and(ok ? 1 : 0)) {
-            ok = false;
-            break;
-        }
-        const int x0 = (tile % tiles_x) * kWgKP, y0 = (tile / tiles_x) * kWgRows;
-        // X transposed, three horizontal shifts: 16 bytes = 8 pixels of one channel
-        for (int task = tid / CIN; task < (kWgRows + 2) * (kWgKP / 8); task += xgroups) {
-            const int r = task / (kWgKP / 8), pxg = task % (kWgKP / 8);
-            const int y = y0 - 1 + r;
-            const int xs = x0 + 8 * pxg - 1;
-            float v[10];
-#pragma unroll
-            for (int j = 0; j < 10; ++j) {
-                const int x = xs + j;
-                v[j] = (y >= 0 && y < a.H && x >= 0 && x < a.W)
-                           ? __bfloat162float(a.x[act_index(a.W, a.H, x, y, ci)])
-                           : 0.0f;
+    if (warp == 0 && lane == 0) {
+        int issued = 0;
+        for (int j = 0; j < my_tiles; ++j) {
+            const int buf = j % NS;
+            if (j >= NS && !mbar_wait(&empty[buf], (uint32_t)((j - NS) / NS) & 1u, a.wait_cycles)) {
+                ok = false;
+                break;
             }
+            const int tile = blockIdx.x + j * gridDim.x;
+            const int x0 = (tile % tiles_x) * kWgKP, y0 = (tile / tiles_x) * kWgRows;
+            unsigned char* X = smem + buf * L::STAGE;
+            unsigned char* D = X + L::DY_OFF;
+            mbar_expect_tx(&full[buf], L::TX_BYTES);
+            for (int r = 0; r < kWgRows + 2; ++r)
 #pragma unroll
-            for (int kx = 0; kx < 3; ++kx) {
-                const uint4 w = make_uint4(pack_bf16(v[kx], v[kx + 1]), pack_bf16(v[kx + 2], v[kx + 3]),
-                                           pack_bf16(v[kx + 4], v[kx + 5]), pack_bf16(v[kx + 6], v[kx + 7]));
-                *reinterpret_cast<uint4*>(sX + r * L::S_ROW + kx * L::S_KX + (ci / 8) * L::S_CG + pxg * 128 +
-                                          (ci % 8) * 16) = w;
-            }
-        }
-        // dY transposed: 16 bytes = 8 pixels of one output channel
-        for (int task = tid / N; task < kWgRows * (kWgKP / 8); task += dgroups) {
-            const int r = task / (kWgKP / 8), pxg = task % (kWgKP / 8);
-            const int y = y0 + r;
-            float v[8];
+                for (int g = 0; g < L::G; ++g)
+                    tma_load_3d(X + r * L::S_ROW + g * L::S_G, &x_map, &full[buf], 2 * (x0 - 1), y0 - 1 + r, g);
+            for (int r = 0; r < kWgRows; ++r)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int x = x0 + 8 * pxg + j;
-                v[j] = (y < a.H && x < a.W) ? __bfloat162float(a.dy[act_index(a.W, a.H, x, y, co)]) : 0.0f;
-                dbsum += v[j];
-            }
-            *reinterpret_cast<uint4*>(sD + r * L::S_DYROW + (co / 8) * L::S_COG + pxg * 128 + (co % 8) * 16) =
-                make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                for (int g = 0; g < L::GN; ++g)
+                    tma_load_3d(D + r * L::S_DYROW + g * L::S_COG, &dy_map, &full[buf], 2 * x0, y0 + r, g);
+            issued = j + 1;
         }
-        fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (tid == 0) {
-            constexpr uint32_t idesc = idesc_bf16(128, N);
-            const uint32_t xa = smem_u32(sX), da0 = smem_u32(sD);
+        // the copies still in flight land before the CTA exits
+        for (int j = issued - NS > 0 ? issued - NS : 0; j < issued; ++j)
+            if (!mbar_wait(&full[j % NS], (uint32_t)(j / NS) & 1u)) ok = false;
+    } else if (warp == 1 && lane == 0) {
+        constexpr uint32_t idesc = idesc_bf16(128, N) | (1u << 15) | (1u << 16);  // A and B MN-major
+        bool issued = false;
+        for (int j = 0; j < my_tiles; ++j) {
+            const int buf = j % NS;
+            if (!mbar_wait(&full[buf], (uint32_t)(j / NS) & 1u, a.wait_cycles)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            // MN-major: the leading offset leads to the next 8 pixels (K), the stride offset to the next 8 channels
+            const uint64_t dx0 = umma_desc(smem_u32(smem + buf * L::STAGE), 128, L::S_G);
+            const uint64_t dd0 = umma_desc(smem_u32(smem + buf * L::STAGE + L::DY_OFF), 128, L::S_COG);
+#pragma unroll 1
             for (int r = 0; r < kWgRows; ++r) {
 #pragma unroll
                 for (int s = 0; s < kWgKP / 16; ++s) {
-                    const uint64_t db = umma_desc(da0 + r * L::S_DYROW + s * 256, 128, L::S_COG);
-                    const uint32_t accum = (iter > 0 || r > 0 || s > 0) ? 1u : 0u;
+                    const uint64_t dd = dd0 + ((r * L::S_DYROW + s * 256) >> 4);
 #pragma unroll
-                    for (int b = 0; b < L::NB; ++b) {
-                        const uint64_t dx = umma_desc(xa + r * L::S_ROW + 16 * b * L::S_CG + s * 256, 128, L::S_CG);
-                        mma_bf16(tmem + b * N, dx, db, idesc, accum);
-                    }
+                    for (int dx = 0; dx < 3; ++dx)
+                        mma_bf16(tmem + (r * 3 + dx) * N, dx0 + ((r * L::S_ROW + s * 256 + dx * 16) >> 4), dd, idesc,
+                                 (j > 0 || s > 0) ? 1u : 0u);
                 }
             }
-            mma_commit(bar);
+            issued = true;
+            mma_commit(&empty[buf]);
         }
-    }
-    if (ok && iter > 0) ok = mbar_wait(bar, (uint32_t)(iter - 1) & 1u, a.wait_cycles);
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;
-    // after a wait ran out, the MMAs of the last tile (committed by thread 0) still
-    // complete before the tensor memory is freed
-    if (!ok && tid == 0 && iter > 0) mbar_wait(bar, (uint32_t)(iter - 1) & 1u);
-    tc_fence_after();
-    if (ok && iter > 0) {
-        for (int b = 0; b < L::NB; ++b) {
-            float acc[N];
+        // every MMA issued completes before the accumulators are read and the tensor memory is freed
+        if (issued) {
+            mma_commit(done);
+            if (!mbar_wait(done, 0)) ok = false;
+        }
+    } else if (warp >= 2) {
+        // the sums of 8 channels over the tile's rows (all of them, or a half where two warps share the channels)
+        constexpr int kShare = 4 / L::GN;  // warps per channel group
+        const int cg = (warp - 2) % L::GN, r0 = (warp - 2) / L::GN * (kWgRows / kShare);
+        float sum[8];
 #pragma unroll
-            for (int c = 0; c < N; c += 16) tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + b * N + c, acc + c);
-            const int m = 128 * b + 32 * warp + lane;
-            const int tap = m / CIN, c_in = m % CIN;
-            if (tap < 9) {
+        for (int c = 0; c < 8; ++c) sum[c] = 0.0f;
+        for (int j = 0; j < my_tiles; ++j) {
+            const int buf = j % NS;
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&full[buf], (uint32_t)(j / NS) & 1u, a.wait_cycles))) {
+                ok = false;
+                break;
+            }
+            const unsigned char* D = smem + buf * L::STAGE + L::DY_OFF + cg * L::S_COG;
+            for (int r = r0; r < r0 + kWgRows / kShare; ++r)
+                for (int px = lane; px < kWgKP; px += 32) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(D + r * L::S_DYROW + px * 16);
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int c = 0; c < N; ++c)
-                    if (acc[c] != 0.0f) atomicAdd(a.dw + ((size_t)c * 9 + tap) * CIN + c_in, acc[c]);
+                    for (int h = 0; h < 4; ++h) {
+                        sum[2 * h] += bf16_lo(w[h]);
+                        sum[2 * h + 1] += bf16_hi(w[h]);
+                    }
+                }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[buf]);
+        }
+        if (ok && my_tiles > 0) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xFFFFFFFFu, sum[c], o);
+                if (lane == 0) atomicAdd(a.db + 8 * cg + c, sum[c]);
             }
         }
-        if (dbsum != 0.0f) atomicAdd(a.db + co, dbsum);
-    } else if (!ok && tid == 0) {
-        atomicOr(a.err, kErrMmaTimeout);
+    }
+    if (!ok) atomicOr(a.err, kErrMmaTimeout);
+    tc_fence_before();
+    const bool all_ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    tc_fence_after();
+    if (all_ok && my_tiles > 0 && warp >= 2) {
+        const int quad = warp & 3;  // the TMEM lanes this warp may read
+        const int m = quad * 32 + lane, dy = m / 8 / L::G, c_in = m / 8 % L::G * 8 + m % 8;
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+            float acc[N];
+#pragma unroll
+            for (int c = 0; c < N; ++c) acc[c] = 0.0f;
+#pragma unroll
+            for (int r = 0; r < kWgRows; ++r)
+#pragma unroll
+                for (int c = 0; c < N; c += 16) {
+                    float row[16];
+                    tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (r * 3 + dx) * N + c, row);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) acc[c + i] += row[i];
+                }
+            if (dy < 3) {
+#pragma unroll
+                for (int c = 0; c < N; ++c)
+                    if (acc[c] != 0.0f) atomicAdd(a.dw + ((size_t)c * 9 + 3 * dy + dx) * CIN + c_in, acc[c]);
+            }
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -994,15 +1052,15 @@ void load_encode_tiled() {
 
 // Tensor map of a planar [C / 8][H][W][8] bf16 tensor viewed as [C / 8][H][2 W]
 // 8-byte elements (a pixel's 8 channels are two elements), with boxes of
-// {2 kHaloW elements, 1 row, 1 group}: each box is one contiguous 2,048-byte
-// run, so TMA moves whole rows rather than 16-byte pieces. Out-of-range
-// elements read as zero.
-bool encode_planar(CUtensorMap* map, const void* base, int C, int W, int H) {
+// {2 box_w elements, 1 row, 1 group}: each box is one contiguous run (2,048 bytes
+// for kHaloW pixels), so TMA moves whole rows rather than 16-byte pieces.
+// Out-of-range elements read as zero.
+bool encode_planar(CUtensorMap* map, const void* base, int C, int W, int H, int box_w = kHaloW) {
     std::call_once(g_encode_once, load_encode_tiled);
     if (!g_encode_tiled) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)W * 2, (cuuint64_t)H, (cuuint64_t)(C / 8)};
     const cuuint64_t strides[2] = {(cuuint64_t)W * 16, (cuuint64_t)W * H * 16};
-    const cuuint32_t box[3] = {(cuuint32_t)(2 * kHaloW), 1, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * box_w), 1, 1};
     const cuuint32_t elem[3] = {1, 1, 1};
     return g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void*>(base), dims, strides, box, elem,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1020,10 +1078,13 @@ bool launch_conv(const rz_upsampler* u, const ConvArgs& a, cudaStream_t s) {
 }
 
 template <int CIN, int N>
-void launch_wgrad(const rz_upsampler* u, const WgradArgs& a, cudaStream_t s) {
+bool launch_wgrad(const rz_upsampler* u, const WgradArgs& a, const __nv_bfloat16* x, const __nv_bfloat16* dy, cudaStream_t s) {
+    CUtensorMap x_map, dy_map;
+    if (!encode_planar(&x_map, x, CIN, a.W, a.H) || !encode_planar(&dy_map, dy, N, a.W, a.H, kWgKP)) return false;
     const int tiles = ((a.W + kWgKP - 1) / kWgKP) * ((a.H + kWgRows - 1) / kWgRows);
-    const int grid = std::min(tiles, 2 * std::max(u->sms, 1));
-    k_wgrad<CIN, N><<<grid, kThreads, WgSmem<CIN, N>::BYTES, s>>>(a);
+    const int grid = std::min(tiles, std::max(u->sms, 1));
+    k_wgrad<CIN, N><<<grid, kWgThreads, WgSmem<CIN, N>::BYTES, s>>>(a, x_map, dy_map);
+    return true;
 }
 
 bool gbuffer_ok(const rz_upsampler* u, const rz_gbuffer* g) {
@@ -1166,44 +1227,36 @@ int rz_upsampler_accumulate(rz_upsampler* u, const rz_gbuffer* in, const void* t
     w.wait_cycles = u->wait_cycles;
     ConvArgs d = conv_args(u, W, H);
     // layer 3
-    w.x = u->d_act[2];
-    w.dy = u->d_dy3;
     w.dw = u->d_grads + layer_woff(3);
     w.db = u->d_grads + layer_boff(3);
-    launch_wgrad<32, 16>(u, w, s);
+    if (!launch_wgrad<32, 16>(u, w, u->d_act[2], u->d_dy3, s)) return RZ_ERROR;
     d.in = u->d_dy3;
     d.wimg = u->d_img + dgrad_img_off(3);
     d.mask_src = u->d_act[2];
     d.out = u->d_dyA;
     if (!launch_conv<16, 32, kEpiMask>(u, d, s)) return RZ_ERROR;
     // layer 2
-    w.x = u->d_act[1];
-    w.dy = u->d_dyA;
     w.dw = u->d_grads + layer_woff(2);
     w.db = u->d_grads + layer_boff(2);
-    launch_wgrad<32, 32>(u, w, s);
+    if (!launch_wgrad<32, 32>(u, w, u->d_act[1], u->d_dyA, s)) return RZ_ERROR;
     d.in = u->d_dyA;
     d.wimg = u->d_img + dgrad_img_off(2);
     d.mask_src = u->d_act[1];
     d.out = u->d_dyB;
     if (!launch_conv<32, 32, kEpiMask>(u, d, s)) return RZ_ERROR;
     // layer 1
-    w.x = u->d_act[0];
-    w.dy = u->d_dyB;
     w.dw = u->d_grads + layer_woff(1);
     w.db = u->d_grads + layer_boff(1);
-    launch_wgrad<32, 32>(u, w, s);
+    if (!launch_wgrad<32, 32>(u, w, u->d_act[0], u->d_dyB, s)) return RZ_ERROR;
     d.in = u->d_dyB;
     d.wimg = u->d_img + dgrad_img_off(1);
     d.mask_src = u->d_act[0];
     d.out = u->d_dyA;
     if (!launch_conv<32, 32, kEpiMask>(u, d, s)) return RZ_ERROR;
     // layer 0
-    w.x = u->d_feat;
-    w.dy = u->d_dyA;
     w.dw = u->d_grads + layer_woff(0);
     w.db = u->d_grads + layer_boff(0);
-    launch_wgrad<16, 32>(u, w, s);
+    if (!launch_wgrad<16, 32>(u, w, u->d_feat, u->d_dyA, s)) return RZ_ERROR;
     u->values += (uint64_t)4 * W * H * 3;
     return cudaGetLastError() == cudaSuccess ? RZ_OK : RZ_ERROR;
 }

@@ -277,6 +277,40 @@ def test_upsampler_gradients_match_oracle(gpu, w, h):
     hi.deinit()
 
 
+@pytest.mark.parametrize("w,h", [(1, 1), (3, 5), (16, 4), (111, 3), (112, 4), (113, 5), (126, 9), (225, 8), (1230, 61)])
+def test_weight_gradient_tiles(gpu, w, h):
+    """Every layer's weight and bias gradients at the edges of the 112 x 4 tiles (and, at 1230 x 61, with more
+    tiles than SMs) against the oracle's float64 sums. The operands are the same bf16 values up to roundings of
+    fp32 against float64 sums that fall on the other side of a bf16 step (2^-8 of a value, a few in a thousand),
+    so 1e-3 of a layer's norm holds for sums of them; fp32 accumulation adds below 1e-5."""
+    import torch
+
+    from rosy_gb300 import _abi
+
+    rng = np.random.default_rng(100 * w + h)
+    gb = {"color": rng.integers(0, 256, (h, w, 4), np.uint8), "albedo": rng.integers(0, 256, (h, w, 4), np.uint8),
+          "depth": (0.3 * rng.random((h, w))).astype(np.float32), "normal": (rng.random((h, w, 2)) - 0.5).astype(np.float16),
+          "sources": rng.integers(0, 65536, (h, w), np.uint16)}
+    target = rng.integers(0, 256, (2 * h, 2 * w, 4), np.uint8)
+    p = _params(5)
+    ref, _ = U.gradients(p, gb, target)
+    dev = {k: torch.from_numpy(v.view(np.int16) if k == "sources" else v).cuda() for k, v in gb.items()}
+    tgt = torch.from_numpy(target).cuda()
+    torch.cuda.synchronize()
+    g = _abi.RzGbuffer(color_rgba8=dev["color"].data_ptr(), depth_f32=dev["depth"].data_ptr(),
+                       albedo_rgba8=dev["albedo"].data_ptr(), normal_oct_f16x2=dev["normal"].data_ptr(),
+                       sources_u16=dev["sources"].data_ptr(), width=w, height=h)
+    u = up.Upsampler(0, w, h)
+    u.set_params(p)
+    u.accumulate(g, tgt.data_ptr())
+    got, _, _ = u.grads()
+    assert u.status() == 0
+    for (wo, bo), (_, cout) in zip(U.OFFSETS, U.LAYERS):
+        for a, b in ((got[wo:bo], ref[wo:bo]), (got[bo:bo + cout], ref[bo:bo + cout])):
+            assert np.linalg.norm(a - b) <= 1e-3 * np.linalg.norm(b)
+    u.close()
+
+
 def test_training_steps_lower_the_loss(gpu):
     import torch
 
