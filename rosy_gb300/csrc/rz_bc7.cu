@@ -17,28 +17,36 @@
 // ((64 - w) * e0 + w * e1 + 32) >> 6 with w from the 2-, 3- or 4-bit weight
 // table; anchor texels store their index with one bit fewer.
 //
-// Work: one CTA per tile of 64 x 4 blocks (256 x 16 texels). Each thread reads
-// one block (a 16-byte load); the tile's blocks are counting-sorted by mode in
-// shared memory, so that a warp almost always decodes 32 blocks of one mode with
-// the code specialised for that mode: every field sits at a compile-time bit
-// position (a funnel shift and a mask), and the index streams are made uniform
-// by inserting the anchors' missing high bits. Decoded texels are staged in
-// shared memory and the tile leaves as 16 rows of 1 KB, coalesced. Tables
-// (partition maps, anchors) are a kernel parameter copied to shared memory.
-// Algorithmic traffic: 16 bytes read + 64 written per block (the HBM roofline);
-// the decode arithmetic (integer ALU issue) bounds it before HBM does.
+// Work: one CTA per tile of 32 x 16 blocks (128 x 64 texels), two blocks per thread
+// (16-byte loads). The tile's blocks are counting-sorted by mode in shared memory,
+// so that most warps decode 32 blocks of one mode with the code specialised for
+// that mode (with eight modes in a tile of 256 blocks nearly every warp held two):
+// every field sits at a compile-time bit position (a funnel shift and a mask), and
+// the index streams are made uniform by inserting the anchors' missing high bits. A
+// texel is two multiply-adds on endpoint ramps prepared per subset and a byte
+// permute (struct Ramp). Decoded texels are staged in shared memory and the tile
+// leaves as 64 rows of 512 bytes, coalesced; rows stored straight from the decoder,
+// 16 bytes each, left half-written sectors behind and were slower (62 us below).
+// Tables (partition maps, anchors) are a kernel parameter copied to shared memory.
+// Algorithmic traffic: 16 bytes read + 64 written per block (the HBM roofline); the
+// decode arithmetic (integer-ALU issue, 63 %) bounds it before HBM does. 4096 x 4096
+// texels of mixed modes, back to back: 58 us with three lerps a texel in 64 x 4
+// block tiles, 46 with the ramps, 39 with these tiles, 34 with the subset picked by
+// multiply-adds (2,460 GB/s).
 #include "rz_device.cuh"
 
 namespace rz {
 
 namespace {
 
-constexpr int kBc7Threads = 256;   // one thread per block of a tile
-constexpr int kTileBX = 64;        // a tile: 64 x 4 blocks = 256 x 16 texels
-constexpr int kTileBY = 4;
+constexpr int kBc7Threads = 256;
+constexpr int kTileBX = 32;        // a tile: 32 x 16 blocks = 128 x 64 texels
+constexpr int kTileBY = 16;
+constexpr int kTileBlocks = kTileBX * kTileBY;
+constexpr int kPerThread = kTileBlocks / kBc7Threads;
 constexpr int kStagePitch = 4 * kTileBX + 4;  // staged texel row (u32), padded against bank conflicts
+static_assert(kPerThread == 2, "two blocks per thread");
 constexpr int kBc7MaxLevels = 16;
-static_assert(kTileBX * kTileBY == kBc7Threads, "one thread per block of a tile");
 
 // Subset of every texel (2 bits per texel, texel 0 lowest) and the anchor texels
 // other than texel 0: entries [0, 64) are the two-subset partitions (anchor
@@ -161,16 +169,46 @@ __device__ __forceinline__ uint64_t insert_zero(uint64_t x, uint32_t p) {
     return low | ((x ^ low) << 1);
 }
 
-// Interpolation weight (out of 64) of a 2-, 3- or 4-bit index: the format's
-// tables {0, 21, 43, 64}, {0, 9, 18, 27, 37, 46, 55, 64} and {0, 4, 9, ..., 60, 64}
-// are floor((64 i + c) / (2^IB - 1)) with c = 1, 3, 7; the division is a
-// multiply by a rounded-up 2^16 / (2^IB - 1), exact for these small numerators
-// (checked against every table entry).
+// Interpolation weight (out of 64) of a 2-, 3- or 4-bit index. The tables of four
+// and eight weights are bytes of one or two registers, picked by a byte permute
+// (index 0's weight is 0, so the other bytes of the result, picked by the index's
+// zero nibbles, are 0 too); the 4-bit table {0, 4, 9, ..., 60, 64} is
+// floor((64 i + 7) / 15), the division a multiply by a rounded-up 2^16 / 15, exact
+// for these numerators (checked against every table entry).
 template <int IB>
 __device__ __forceinline__ uint32_t weight_of(uint32_t i) {
-    constexpr uint32_t c = IB == 2 ? 1u : IB == 3 ? 3u : 7u;
-    constexpr uint32_t m = IB == 2 ? 21846u : IB == 3 ? 9363u : 4370u;
-    return ((64u * i + c) * m) >> 16;
+    if constexpr (IB == 2) return __byte_perm(0x402B1500u, 0u, i);                   // 0, 21, 43, 64
+    else if constexpr (IB == 3) return __byte_perm(0x1B120900u, 0x40372E25u, i);     // 0, 9, 18, 27, 37, 46, 55, 64
+    else return (i * (64u * 4370u) + 7u * 4370u) >> 16;
+}
+
+// An endpoint pair prepared for interpolation, two channels in the 16-bit lanes of
+// a register (R and B, G and A): base = 256 e0 + 128 and step = 4 (e1 - e0) per
+// lane. base + w * step is 4 ((64 - w) e0 + w e1 + 32) in every lane, between 128
+// and 65,408, so the lanes neither borrow nor carry in the sum (steps may be
+// negative; the sum of the two lanes is what the wrapping arithmetic gives), and the
+// interpolated byte ((64 - w) e0 + w e1 + 32) >> 6 is each lane's upper byte.
+struct Ramp {
+    uint32_t rb, rb_step, ga, ga_step;
+};
+
+// p + on * d in every field, on 0 or 1: a texel's subset picked by multiply-adds
+// (the decoder is short of integer-ALU issue, not of multiply-adds).
+__device__ __forceinline__ void add_ramp(Ramp& p, const Ramp& d, uint32_t on) {
+    p.rb += on * d.rb;
+    p.rb_step += on * d.rb_step;
+    p.ga += on * d.ga;
+    p.ga_step += on * d.ga_step;
+}
+
+__device__ __forceinline__ Ramp make_ramp(uint32_t e0, uint32_t e1) {
+    constexpr uint32_t M = 0x00FF00FFu;
+    Ramp r;
+    r.rb = (e0 & M) * 256u + 0x00800080u;
+    r.rb_step = ((e1 & M) - (e0 & M)) * 4u;
+    r.ga = (e0 & ~M) + 0x00800080u;
+    r.ga_step = (((e1 >> 8) & M) - ((e0 >> 8) & M)) * 4u;
+    return r;
 }
 
 // Widens the three colour bytes of a packed endpoint from N (5..8) bits to 8 by
@@ -192,14 +230,14 @@ __device__ __forceinline__ uint32_t widen1(uint32_t v) {
     else return (v << (8 - N)) | (v >> (2 * N - 8));
 }
 
-// One block of mode M to its 4 x 4 RGBA8 texels, row r at out + r * pitch (16-byte
-// aligned). The layout follows the mode: partition, rotation and index-selection
-// fields after the mode bits, colour endpoints channel-major, alpha endpoints,
-// P-bits, then the primary and (modes 4, 5) secondary index streams. Rows are a
-// loop (the streams and the subset map shift down after each), the four texels
-// of a row unrolled: the eight decoders stay small enough for the instruction cache.
+// One block of mode M to its 4 x 4 RGBA8 texels, row r at out + r * kStagePitch
+// (16-byte aligned). The layout follows the mode: partition, rotation and index-selection fields after the mode bits, colour
+// endpoints channel-major, alpha endpoints, P-bits, then the primary and (modes 4,
+// 5) secondary index streams. Rows are a loop (the streams and the subset map shift
+// down after each), the four texels of a row unrolled: the eight decoders stay
+// small enough for the instruction cache.
 template <int M>
-__device__ __forceinline__ void decode_mode(const uint4& q, const Bc7Tables& T, uint32_t* out, int pitch) {
+__device__ __forceinline__ void decode_mode(const uint4& q, const Bc7Tables& T, uint32_t* out) {
     constexpr int NS = kModeFields[M][0], PB = kModeFields[M][1], RB = kModeFields[M][2], ISB = kModeFields[M][3];
     constexpr int CB = kModeFields[M][4], AB = kModeFields[M][5], PK = kModeFields[M][6];
     constexpr int IB = kModeFields[M][7], IB2 = kModeFields[M][8];
@@ -240,131 +278,167 @@ __device__ __forceinline__ void decode_mode(const uint4& q, const Bc7Tables& T, 
     }
     uint64_t s2 = 0;
     if constexpr (IB2 != 0) s2 = insert_zero(field64(q, I0 + L1, L2), IB2 - 1);
-    const uint32_t sel = rot == 0 ? 0x3210u : rot == 1 ? 0x0213u : rot == 2 ? 0x1230u : 0x2310u;
+    Ramp ramp[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        ramp[k] = make_ramp(E[2 * k], E[2 * k + 1]);
+        if (k > 0) {  // as the difference to the first
+            ramp[k].rb -= ramp[0].rb;
+            ramp[k].rb_step -= ramp[0].rb_step;
+            ramp[k].ga -= ramp[0].ga;
+            ramp[k].ga_step -= ramp[0].ga_step;
+        }
+    }
+    // modes 4 and 5: alpha steps on its own weight
+    uint32_t g_step = 0, a_step = 0;
+    if constexpr (IB2 != 0) {
+        g_step = (((E[1] >> 8) & 0xFFu) - ((E[0] >> 8) & 0xFFu)) * 4u;
+        a_step = ((E[1] >> 24) - (E[0] >> 24)) << 18;
+    }
+    // the upper bytes of the lanes in the order R, G, B, A, or alpha swapped with R, G or B
+    const uint32_t sel = rot == 0 ? 0x7351u : rot == 1 ? 0x1357u : rot == 2 ? 0x5371u : 0x3751u;
 #pragma unroll 1
     for (int r = 0; r < 4; ++r) {
         uint32_t v[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            uint32_t e0 = E[0], e1 = E[1];
+            Ramp p = ramp[0];
             if constexpr (NS >= 2) {
-                const uint32_t s = (map >> (2 * c)) & 3u;
-                if constexpr (NS == 2) {
-                    e0 = s ? E[2] : E[0];
-                    e1 = s ? E[3] : E[1];
-                } else {
-                    e0 = s == 0 ? E[0] : s == 1 ? E[2] : E[4];
-                    e1 = s == 0 ? E[1] : s == 1 ? E[3] : E[5];
-                }
+                add_ramp(p, ramp[1], (map >> (2 * c)) & 1u);
+                if constexpr (NS == 3) add_ramp(p, ramp[2], (map >> (2 * c + 1)) & 1u);
             }
             const uint32_t w1 = weight_of<IB>((uint32_t)(s1 >> (IB * c)) & ((1u << IB) - 1u));
-            uint32_t wc = w1, wa = w1;
+            uint32_t rb, ga;
             if constexpr (IB2 != 0) {
                 const uint32_t w2 = weight_of<IB2>((uint32_t)(s2 >> (IB2 * c)) & ((1u << IB2) - 1u));
-                wc = isb ? w2 : w1;  // the index-selection bit (mode 4) gives the colour the secondary set
-                wa = isb ? w1 : w2;
+                const uint32_t wc = isb ? w2 : w1;  // the index-selection bit (mode 4) gives the colour the secondary set
+                const uint32_t wa = isb ? w1 : w2;
+                rb = p.rb + wc * p.rb_step;
+                ga = p.ga + wc * g_step + wa * a_step;
+            } else {
+                rb = p.rb + w1 * p.rb_step;
+                ga = p.ga + w1 * p.ga_step;
             }
-            // R and B in two 16-bit lanes: (64 - w) * 255 + w * 255 + 32 < 2^16, so the lanes never carry
-            const uint32_t rb = (((64u - wc) * (e0 & 0x00FF00FFu) + wc * (e1 & 0x00FF00FFu) + 0x00200020u) >> 6) & 0x00FF00FFu;
-            const uint32_t g = ((64u - wc) * ((e0 >> 8) & 0xFFu) + wc * ((e1 >> 8) & 0xFFu) + 32u) >> 6;
-            const uint32_t a = ((64u - wa) * (e0 >> 24) + wa * (e1 >> 24) + 32u) >> 6;
-            const uint32_t t = rb | g << 8 | a << 24;
-            v[c] = RB ? __byte_perm(t, 0u, sel) : t;
+            v[c] = __byte_perm(rb, ga, RB ? sel : 0x7351u);
         }
-        *reinterpret_cast<uint4*>(out + r * pitch) = make_uint4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<uint4*>(out + r * kStagePitch) = make_uint4(v[0], v[1], v[2], v[3]);
         map >>= 8;
         s1 >>= 4 * IB;
         if constexpr (IB2 != 0) s2 >>= 4 * IB2;
     }
 }
 
-__device__ __forceinline__ void decode_block(const uint4& q, const Bc7Tables& T, uint32_t* out, int pitch) {
+__device__ __forceinline__ void decode_block(const uint4& q, const Bc7Tables& T, uint32_t* out) {
     const uint32_t m8 = q.x & 0xFFu;
     switch (m8 ? __ffs(m8) - 1 : 8) {
-        case 0: decode_mode<0>(q, T, out, pitch); break;
-        case 1: decode_mode<1>(q, T, out, pitch); break;
-        case 2: decode_mode<2>(q, T, out, pitch); break;
-        case 3: decode_mode<3>(q, T, out, pitch); break;
-        case 4: decode_mode<4>(q, T, out, pitch); break;
-        case 5: decode_mode<5>(q, T, out, pitch); break;
-        case 6: decode_mode<6>(q, T, out, pitch); break;
-        case 7: decode_mode<7>(q, T, out, pitch); break;
+        case 0: decode_mode<0>(q, T, out); break;
+        case 1: decode_mode<1>(q, T, out); break;
+        case 2: decode_mode<2>(q, T, out); break;
+        case 3: decode_mode<3>(q, T, out); break;
+        case 4: decode_mode<4>(q, T, out); break;
+        case 5: decode_mode<5>(q, T, out); break;
+        case 6: decode_mode<6>(q, T, out); break;
+        case 7: decode_mode<7>(q, T, out); break;
         default:  // the reserved mode
-            for (int r = 0; r < 4; ++r) *reinterpret_cast<uint4*>(out + r * pitch) = make_uint4(0u, 0u, 0u, 0u);
+            for (int r = 0; r < 4; ++r) *reinterpret_cast<uint4*>(out + r * kStagePitch) = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
-__global__ void __launch_bounds__(kBc7Threads) k_bc7_decode(const Bc7Job job, const Bc7Tables tables) {
+__global__ void __launch_bounds__(kBc7Threads) k_bc7_decode(const __grid_constant__ Bc7Job job,
+                                                            const __grid_constant__ Bc7Tables tables) {
     __shared__ Bc7Tables T;
-    __shared__ Bc7Level L[kBc7MaxLevels];
-    __shared__ uint4 s_blk[kBc7Threads];
-    __shared__ uint16_t s_src[kBc7Threads];
-    __shared__ uint32_t s_count[10], s_off[10];
+    // the sorted blocks, then (once every thread has its own) the decoded tile
     __shared__ __align__(16) uint32_t s_out[4 * kTileBY][kStagePitch];
-    const int tid = threadIdx.x;
+    __shared__ uint16_t s_src[kTileBlocks];
+    __shared__ uint32_t s_count[16], s_off[16];
+    uint4* const s_blk = reinterpret_cast<uint4*>(&s_out[0][0]);
+    const int tid = threadIdx.x, lane = tid & 31;
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&tables);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&T);
-        for (uint32_t i = tid; i < sizeof(Bc7Tables) / 4; i += blockDim.x) dst[i] = src[i];
-        const uint32_t* ls = reinterpret_cast<const uint32_t*>(job.L);
-        uint32_t* ld = reinterpret_cast<uint32_t*>(L);
-        for (uint32_t i = tid; i < sizeof(job.L) / 4; i += blockDim.x) ld[i] = ls[i];
-        if (tid < 10) s_count[tid] = 0;
+        for (uint32_t i = tid; i < sizeof(Bc7Tables) / 4; i += kBc7Threads) dst[i] = src[i];
+        if (tid < 16) s_count[tid] = 0;
     }
-    __syncthreads();
     const uint32_t tile = blockIdx.x;
     uint32_t l = 0;
-    while (l + 1 < job.levels && tile >= L[l + 1].tile0) ++l;
-    const Bc7Level& lv = L[l];
+    while (l + 1 < job.levels && tile >= job.L[l + 1].tile0) ++l;
+    const Bc7Level& lv = job.L[l];
     const uint32_t lt = tile - lv.tile0;
     const uint32_t tbx = (lt % lv.tiles_x) * kTileBX, tby = (lt / lv.tiles_x) * kTileBY;
-    // this thread's block, and its mode (9: outside the level)
-    uint4 q = make_uint4(0u, 0u, 0u, 0u);
-    uint32_t mode = 9;
-    {
-        const uint32_t bx = tbx + tid % kTileBX, by = tby + tid / kTileBX;
+    // this thread's blocks, and their modes (9: outside the level)
+    uint4 q[kPerThread];
+    uint32_t mode[kPerThread], rank[kPerThread];
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+        const int i = tid + k * kBc7Threads;
+        const uint32_t bx = tbx + i % kTileBX, by = tby + i / kTileBX;
+        q[k] = make_uint4(0u, 0u, 0u, 0u);
+        mode[k] = 9;
         if (bx < lv.bw && by < lv.bh) {
-            q = __ldg(job.blocks + lv.block0 + (size_t)by * lv.bw + bx);
-            const uint32_t m8 = q.x & 0xFFu;
-            mode = m8 ? __ffs(m8) - 1 : 8;
+            q[k] = __ldg(job.blocks + lv.block0 + (size_t)by * lv.bw + bx);
+            const uint32_t m8 = q[k].x & 0xFFu;
+            mode[k] = m8 ? __ffs(m8) - 1 : 8;
         }
     }
-    // counting sort of the tile's blocks by mode
-    const uint32_t rank = atomicAdd(&s_count[mode], 1u);
     __syncthreads();
-    if (tid == 0) {
+    // counting sort of the tile's blocks by mode: a warp's lanes of a mode take their places with one atomic
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+        uint32_t same = 0xffffffffu;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const uint32_t v = __ballot_sync(0xffffffffu, (mode[k] >> b) & 1u);
+            same &= (mode[k] >> b) & 1u ? v : ~v;
+        }
+        const int leader = __ffs(same) - 1;
+        uint32_t at = 0;
+        if (lane == leader) at = atomicAdd(&s_count[mode[k]], (uint32_t)__popc(same));
+        rank[k] = __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    if (tid < 16) {
         uint32_t acc = 0;
-        for (int m = 0; m < 10; ++m) {
-            s_off[m] = acc;
-            acc += s_count[m];
-        }
+        for (int m = 0; m < tid; ++m) acc += s_count[m];
+        s_off[tid] = acc;
     }
     __syncthreads();
-    const uint32_t pos = s_off[mode] + rank;
-    s_blk[pos] = q;
-    s_src[pos] = (uint16_t)tid;
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+        const uint32_t pos = s_off[mode[k]] + rank[k];
+        s_blk[pos] = q[k];
+        s_src[pos] = (uint16_t)(tid + k * kBc7Threads);
+    }
     __syncthreads();
-    // decode the sorted blocks into the staged tile
-    {
-        const uint32_t src = s_src[tid];
-        const uint32_t sbx = src % kTileBX, sby = src / kTileBX;
-        if (tbx + sbx < lv.bw && tby + sby < lv.bh) decode_block(s_blk[tid], T, &s_out[4 * sby][4 * sbx], kStagePitch);
+    uint32_t src[kPerThread];
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+        q[k] = s_blk[tid + k * kBc7Threads];
+        src[k] = s_src[tid + k * kBc7Threads];
+    }
+    __syncthreads();
+    // decode the sorted blocks that lie inside the level into the staged tile
+    const uint32_t inside = s_off[9];
+#pragma unroll 1
+    for (int k = 0; k < kPerThread; ++k) {
+        const uint32_t at = k ? src[1] : src[0];
+        if ((uint32_t)(tid + k * kBc7Threads) < inside)
+            decode_block(k ? q[1] : q[0], T, &s_out[4 * (at / kTileBX)][4 * (at % kTileBX)]);
     }
     __syncthreads();
     // the tile's texel rows, four texels per thread, consecutive threads on consecutive texels
-    for (int i = tid; i < 4 * kTileBY * kTileBX; i += kBc7Threads) {
-        const int r = i / kTileBX, g = i % kTileBX;
-        const uint32_t y = 4 * tby + r, x = 4 * (tbx + g);
-        if (y >= lv.h || x >= lv.w) continue;
-        uint32_t* dst = job.texels + lv.texel0 + (size_t)y * lv.w + x;
-        const uint4 v = *reinterpret_cast<const uint4*>(&s_out[r][4 * g]);
-        if (lv.vec && x + 4 <= lv.w) {
+    const uint32_t rows = min(4u * kTileBY, lv.h - 4 * tby), x = 4 * (tbx + tid % kTileBX);
+    if (x >= lv.w) return;
+    const uint32_t cols = lv.w - x;
+    uint32_t* dst = job.texels + lv.texel0 + (size_t)(4 * tby + tid / kTileBX) * lv.w + x;
+    for (uint32_t r = tid / kTileBX; r < rows; r += kBc7Threads / kTileBX, dst += (size_t)(kBc7Threads / kTileBX) * lv.w) {
+        const uint4 v = *reinterpret_cast<const uint4*>(&s_out[r][4 * (tid % kTileBX)]);
+        if (lv.vec) {
             *reinterpret_cast<uint4*>(dst) = v;
         } else {
             dst[0] = v.x;
-            if (x + 1 < lv.w) dst[1] = v.y;
-            if (x + 2 < lv.w) dst[2] = v.z;
-            if (x + 3 < lv.w) dst[3] = v.w;
+            if (cols > 1) dst[1] = v.y;
+            if (cols > 2) dst[2] = v.z;
+            if (cols > 3) dst[3] = v.w;
         }
     }
 }

@@ -60,6 +60,16 @@ def test_partial_blocks_match_oracle(gpu, w, h):
     assert np.array_equal(_decode(blocks, w, h), oracle.bc7_decode(blocks, w, h))
 
 
+@pytest.mark.parametrize("w,h", [(124, 60), (127, 63), (128, 64), (129, 65), (260, 3), (4, 132), (257, 129)])
+def test_tile_edges_match_oracle(gpu, w, h):
+    """Images at the edges of the 128 x 64 texel tiles, reserved-mode blocks among them."""
+    rng = np.random.default_rng(w * 1000 + h)
+    n = ((w + 3) // 4) * ((h + 3) // 4)
+    pool = np.concatenate([bc7.mixed_blocks(rng, n), bc7.blocks_of_mode(rng, 8, 1 + n // 16)])
+    blocks = pool[rng.permutation(len(pool))[:n]]
+    assert np.array_equal(_decode(blocks, w, h), oracle.bc7_decode(blocks, w, h))
+
+
 def test_large_image_matches_texture_unit(gpu):
     """4096 x 4096 texels (a million blocks, all modes) against the texture unit."""
     rng = np.random.default_rng(7)
