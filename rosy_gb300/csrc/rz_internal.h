@@ -96,10 +96,9 @@ static_assert(sizeof(TriRecord) == 64, "TriRecord is 64 bytes");
 constexpr uint32_t kViewBits = 24;
 constexpr uint32_t kCascadeMask = 3u;     // cascade = (view >> kViewBits) & kCascadeMask
 // Large records also carry raster facts the setup computed once, so that the
-// raster decodes them instead of recomputing them for every chunk a record
-// meets: view bits 26-28 the top-left bias of edges 0-2 (1: not a top-left
-// edge), 29 medium, 30 box cut by the viewport, 31 near origin; stamp_offset
-// bits 40-63 the stamps per row of the record's box.
+// raster decodes them instead of recomputing them: view bits 26-28 the top-left
+// bias of edges 0-2 (1: not a top-left edge), 29 near origin, 30 box cut by the
+// viewport; stamp_offset bits 40-63 the stamps per row of the record's box.
 constexpr uint32_t kRecFlagShift = 26;
 constexpr uint32_t kRecViewMask = (1u << kRecFlagShift) - 1u;  // view index and cascade
 constexpr int kStampOffsetBits = 40;
@@ -174,11 +173,11 @@ struct PassParams {
     uint32_t lookback_spins;  // bound of each look-back wait (ordered passes)
     // coverage sample, in 1/256 pixel: the pixel centre (128, 128)
     int32_t sample_x, sample_y;
+    int32_t bb_hi;  // smallest sample offset the setup boxed for (32 with 4x samples, else 128)
     // 4x multisampled camera pass: every record at the four standard positions, each
     // into its plane; the records are dealt to kMsaaSamples launches, of which this is `part`
     int32_t msaa;
     uint32_t part;
-    int32_t bb_hi;  // smallest sample offset the setup boxed for (32 with 4x samples, else 128)
     // buffers the setup launch zeroes besides its own work (the depth target's
     // CLEAR load-op, folded into the launch that precedes the raster); none when
     // clear_count is 0

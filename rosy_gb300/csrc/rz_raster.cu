@@ -16,7 +16,8 @@
 //    with a decoupled look-back across CTAs; each record also marks the work
 //    chunks (kChunkStamps stamps) that start inside it.
 //  * k_raster: persistent warps take chunks of stamps, so tiny and huge
-//    triangles are balanced alike. A lane is a pixel of the stamp; coverage is
+//    triangles are balanced alike. A lane prepares a stamp (edges, bounds), then
+//    the warp takes those that are left with a lane per pixel; coverage is
 //    the integer edge-function test with the top-left rule, and the depth test
 //    is a 64-bit atomicMax on (depth_bits << 32 | id). Because depths are
 //    non-negative floats their bit patterns order like the values, so the max
@@ -190,39 +191,38 @@ __device__ __forceinline__ uint32_t record_stamps(const TriRecord& r) {
     return (uint32_t)((px1 - px0) / kStampW + 1) * (uint32_t)((py1 - py0) / kStampH + 1);
 }
 
-// Triangles up to this extent (pixels, each way) take the incremental 32-bit
-// path: every edge value over the bounding box plus a stamp of overhang is
-// below 2 * ((90 + 8) * 256)^2 < 2^31.
-constexpr int kMediumExtent = 90;
+// The raster facts of a large record (packed by the setup, decoded by the raster):
+// the edges' top-left bias, whether the stamps may be taken together (near: float
+// offsets from vertex 0 are exact over the box, and edges are below 2^26 so that a
+// stamp's edge values fit 32 bits), whether its edge functions themselves fit 32
+// bits (small: an extent of at most 90 pixels each way), whether the viewport cut its
+// box, and its stamps per row. Pixels past an uncut box edge lie outside the triangle's extent, so the
+// edge test alone rejects the stamps' overhang there; only a cut box needs the check.
+constexpr uint32_t kFactNear = 8u, kFactCut = 16u, kFactSmall = 32u;
+// every edge value over the box plus a stamp of overhang is below 2 * ((90 + 8) * 256)^2 < 2^31
+constexpr int kSmallEdges = 90;
 
-// The raster facts of a large record (packed by the setup, decoded by
-// load_large): the edges' top-left bias, whether the 32-bit incremental walk
-// applies (medium), whether the viewport cut its box (clipped), whether float
-// offsets from vertex 0 are exact over the box (near_origin), and its stamps per row.
 __device__ __forceinline__ uint32_t large_facts(const TriRecord& r, int32_t bb_hi, uint32_t& nsx) {
     const int32_t X[3] = {r.X0, r.X1, r.X2}, Y[3] = {r.Y0, r.Y1, r.Y2};
     const int px0 = (int)(r.p0 & 0xffff), py0 = (int)(r.p0 >> 16), px1 = (int)(r.p1 & 0xffff), py1 = (int)(r.p1 >> 16);
     uint32_t flags = 0;
+    bool near_origin = true;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int a = (i + 1) % 3, b = (i + 2) % 3;
         const int32_t dx = X[b] - X[a], dy = Y[b] - Y[a];
         if (!(dy < 0 || (dy == 0 && dx > 0))) flags |= 1u << i;
+        near_origin = near_origin && abs(dx) < (1 << 26) && abs(dy) < (1 << 26);
     }
     const int32_t lo_x = px0 * 256 - X[0], hi_x = px1 * 256 + 256 - X[0] + kStampW * 256;
     const int32_t lo_y = py0 * 256 - Y[0], hi_y = py1 * 256 + 256 - Y[0] + kStampH * 256;
     const int32_t lim = 1 << 23;
-    const bool near_origin = lo_x > -lim && hi_x < lim && lo_y > -lim && hi_y < lim;
+    near_origin = near_origin && lo_x > -lim && hi_x < lim && lo_y > -lim && hi_y < lim;
     const int32_t max_x = max(X[0], max(X[1], X[2])), max_y = max(Y[0], max(Y[1], Y[2]));
-    const int32_t ex = max_x - min(X[0], min(X[1], X[2]));
-    const int32_t ey = max_y - min(Y[0], min(Y[1], Y[2]));
-    // Pixels past an uncut box edge lie outside the triangle's extent, so the edge
-    // test alone rejects the stamps' overhang there; only a cut box needs the check.
-    const bool clipped = ((max_x - bb_hi) >> 8) > px1 || ((max_y - bb_hi) >> 8) > py1;
-    const bool medium = near_origin && ex <= kMediumExtent * 256 && ey <= kMediumExtent * 256;
-    flags |= (medium ? 8u : 0u) | (clipped ? 16u : 0u) | (near_origin ? 32u : 0u);
+    const bool cut = ((max_x - bb_hi) >> 8) > px1 || ((max_y - bb_hi) >> 8) > py1;
+    const bool small = max_x - min(X[0], min(X[1], X[2])) <= kSmallEdges * 256 && max_y - min(Y[0], min(Y[1], Y[2])) <= kSmallEdges * 256;
     nsx = (uint32_t)((px1 - px0) / kStampW + 1);
-    return flags;
+    return flags | (small ? kFactSmall : 0u) | (near_origin ? kFactNear : 0u) | (cut ? kFactCut : 0u);
 }
 
 
@@ -777,10 +777,7 @@ struct LargeRecord {
     int32_t X[3], Y[3];
     int32_t dx[3], dy[3];
     uint32_t tl_bias[3];  // 0 on top-left edges, 1 otherwise
-    bool medium;          // extent <= kMediumExtent px and near_origin: incremental 32-bit walk
-    bool clipped;         // the box was cut by the viewport: pixels past px1 / py1 may be inside the triangle
-    bool near_origin;     // |PX - X0|, |PY - Y0| < 2^23 over the box: float offsets exact
-    int32_t X0, Y0;
+    bool near_origin, cut, small;  // see large_facts
     float z0, dzdx, dzdy, bias;
     int px0, py0, px1, py1;
     uint32_t id, nsx, view;
@@ -795,8 +792,6 @@ __device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const
     L.Y[1] = q0.w;
     L.X[2] = q1.x;
     L.Y[2] = q1.y;
-    L.X0 = q0.x;
-    L.Y0 = q0.y;
     L.z0 = __int_as_float(q1.z);
     L.dzdx = __int_as_float(q1.w);
     L.dzdy = __int_as_float(q2.x);
@@ -818,9 +813,9 @@ __device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const
         L.dy[i] = L.Y[b] - L.Y[a];
         L.tl_bias[i] = (flags >> i) & 1u;
     }
-    L.medium = (flags & 8u) != 0;
-    L.clipped = (flags & 16u) != 0;
-    L.near_origin = (flags & 32u) != 0;
+    L.near_origin = (flags & kFactNear) != 0;
+    L.cut = (flags & kFactCut) != 0;
+    L.small = (flags & kFactSmall) != 0;
 }
 
 __device__ __forceinline__ void load_large(const TriRecord* rec, LargeRecord& L) {
@@ -829,11 +824,11 @@ __device__ __forceinline__ void load_large(const TriRecord* rec, LargeRecord& L)
 }
 
 // Record staging of the chunk walk: a warp copies the records a chunk starts
-// with (one per lane, kStageRecords at most) into shared memory with cp.async
+// with (one per lane, the first few of them) into shared memory with cp.async
 // while it rasterises the chunk before, so that a segment finds its record
 // there instead of waiting for a dependent global load.
 constexpr int kRasterThreads = 256;
-constexpr int kStageRecords = 32;
+constexpr int kStageRecordsMax = 16;  // a chunk of 32 stamps rarely holds more; 8 where the stamps take more room (4x samples)
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -842,9 +837,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 
 // Lane `lane` copies record r0 + lane when it exists (below n_rec); one commit
 // group per call, also when it copies nothing.
+template <int kRecords>
 __device__ __forceinline__ void stage_records(int4 (*buf)[4], const TriRecord* records, uint32_t r0, uint32_t n_rec,
                                               int lane) {
-    if ((uint64_t)r0 + (uint64_t)lane < (uint64_t)n_rec) {
+    if (lane < kRecords && (uint64_t)r0 + (uint64_t)lane < (uint64_t)n_rec) {
         const int4* src = reinterpret_cast<const int4*>(records + r0 + lane);
 #pragma unroll
         for (int i = 0; i < 4; ++i) cp_async16(&buf[lane][i], src + i);
@@ -852,269 +848,148 @@ __device__ __forceinline__ void stage_records(int4 (*buf)[4], const TriRecord* r
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-// Edge constants of the generic (64-bit) path.
-struct GenericEdges {
-    int64_t c[3];                    // E' at sub-pixel (0, 0): E'(P) = c + dx*PY - dy*PX
-    int64_t max_off[3], min_off[3];  // range of the lane offsets over the stamp
-    bool short_edges;                // all |dx|, |dy| < 2^18: partial-edge values and lane offsets fit in 32 bits
+// Up to 32 stamps as the lanes of a warp (their pixels) read them from shared memory.
+// A 16-byte broadcast takes four cycles of the shared-memory return path, so a stamp
+// is kept to its own values, and its record's are read when the record changes.
+template <int kSamples>
+struct StampWork {
+    int4 e[kSamples][32];  // per sample: floor(E' / 256) of the three edges at the stamp's first pixel, clamped;
+                           // [0].w: the first pixel's word in the target
+    float2 at[32];         // offset of the first pixel's sample from vertex 0
+    int4 edges[32];        // the record's dx and -dy of edges 0 and 1 (edge 2's are minus their sums)
+    int4 plane[32];        // the record's z0, dz/dx, dz/dy, and its id (camera) or depth bias (shadow)
+    uint2 box[32];         // the lanes whose pixel lies in the record's box; the record's view field
 };
 
-__device__ __forceinline__ void generic_edges(const LargeRecord& L, GenericEdges& G) {
-    bool short_edges = true;
+constexpr uint32_t kAllLanes = 0xffffffffu;
+
+// The edges of stamp (sx, sy) of a record whose stamps may be taken together, per
+// sample, at its first pixel: floor(E' / 256), clamped. Returns false if no pixel of
+// the stamp passes all three edges' bounds.
+//
+// The edge function of a pixel lx right of and ly below the stamp's first pixel is
+// E' = E0 + 256 (dx ly - dy lx), so E' >= 0 exactly when floor(E0 / 256) + dx ly -
+// dy lx >= 0. Edges are below 2^26, so the lane term stays below 2^30 in size, and
+// the 64-bit floor may be clamped to +-2^30 without a change of that sign.
+template <int kSamples, class Int>  // Int: the type that holds the record's edge values
+__device__ __forceinline__ bool stamp_edges(const LargeRecord& L, int32_t PX, int32_t PY, int32_t (&q)[kSamples][3]) {
+    uint32_t rejected = 0;  // samples
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int a = (i + 1) % 3;
         const int32_t dx = L.dx[i], dy = L.dy[i];
-        G.c[i] = (int64_t)dy * L.X[a] - (int64_t)dx * L.Y[a] - L.tl_bias[i];
-        G.max_off[i] = (dx > 0 ? (int64_t)dx * ((kStampH - 1) * 256) : 0) + (dy < 0 ? -(int64_t)dy * ((kStampW - 1) * 256) : 0);
-        G.min_off[i] = (dx < 0 ? (int64_t)dx * ((kStampH - 1) * 256) : 0) + (dy > 0 ? -(int64_t)dy * ((kStampW - 1) * 256) : 0);
-        short_edges = short_edges && abs(dx) < (1 << 18) && abs(dy) < (1 << 18);
-    }
-    G.short_edges = short_edges;
-}
-
-// Rasterises stamp (sx, sy) of a large record: lane = pixel (lane & 7, lane >> 3).
-// Walk over the stamps of a generic record in raster order: the 64-bit edge
-// values at the current stamp's origin sample, advanced by exact constant steps
-// (one stamp right, or back to the row start and one stamp down).
-struct GenericWalk {
-    int64_t e[3], er[3];  // edge values at the current stamp's / the row's first stamp's origin sample
-    int sx0, sy0;         // origin pixel of the current stamp
-    uint32_t sx;
-};
-
-__device__ __forceinline__ void generic_start(const LargeRecord& L, const GenericEdges& G, uint32_t sx, uint32_t sy,
-                                              int32_t ox, int32_t oy, GenericWalk& w) {
-    w.sx = sx;
-    w.sx0 = L.px0 + (int)sx * kStampW;
-    w.sy0 = L.py0 + (int)sy * kStampH;
-    const int32_t PXo = w.sx0 * 256 + ox, PYo = w.sy0 * 256 + oy, PXr = L.px0 * 256 + ox;
+        const Int E = (Int)dx * (PY - L.Y[a]) - (Int)dy * (PX - L.X[a]) - (Int)L.tl_bias[i];
+        const int32_t most = max(dx, 0) * (kStampH - 1) + max(-dy, 0) * (kStampW - 1);  // of the lane term
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        w.e[i] = G.c[i] + (int64_t)L.dx[i] * PYo - (int64_t)L.dy[i] * PXo;
-        w.er[i] = G.c[i] + (int64_t)L.dx[i] * PYo - (int64_t)L.dy[i] * PXr;
-    }
-}
-
-__device__ __forceinline__ void generic_next(const LargeRecord& L, GenericWalk& w) {
-    if (++w.sx == L.nsx) {
-        w.sx = 0;
-        w.sx0 = L.px0;
-        w.sy0 += kStampH;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            w.er[i] += (int64_t)L.dx[i] * (kStampH * 256);
-            w.e[i] = w.er[i];
-        }
-    } else {
-        w.sx0 += kStampW;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) w.e[i] -= (int64_t)L.dy[i] * (kStampW * 256);
-    }
-}
-
-template <bool kWriteId, bool kBoxCheck>
-__device__ __forceinline__ void raster_stamp(const Target& T, const LargeRecord& L, const GenericEdges& G,
-                                             const GenericWalk& w, int lx, int ly, int32_t ox, int32_t oy) {
-    const int sx0 = w.sx0, sy0 = w.sy0;
-    const int32_t PXo = sx0 * 256 + ox, PYo = sy0 * 256 + oy;
-    const int64_t* eo = w.e;
-    bool reject = false, accept = true;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        reject |= eo[i] + G.max_off[i] < 0;
-        accept &= eo[i] + G.min_off[i] >= 0;
-    }
-    if (reject) return;
-    const int px = sx0 + lx, py = sy0 + ly;
-    bool in = !kBoxCheck || (px <= L.px1 && py <= L.py1);
-    if (!accept) {
-        if (G.short_edges) {
-            // partial edges: |eo| < 2^30 and the lane offset < 2^30, so 32 bits suffice
-            int32_t hi = 0;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const bool edge_accept = eo[i] + G.min_off[i] >= 0;
-                const int32_t e = (int32_t)eo[i] + L.dx[i] * (ly * 256) - L.dy[i] * (lx * 256);
-                hi |= edge_accept ? 0 : e;
-            }
-            in = in && hi >= 0;
-        } else {
-            int32_t hi = 0;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const int64_t e = eo[i] + (int64_t)L.dx[i] * (ly * 256) - (int64_t)L.dy[i] * (lx * 256);
-                hi |= (int32_t)(e >> 32);
-            }
-            in = in && hi >= 0;
+        for (int k = 0; k < kSamples; ++k) {
+            Int f = (kSamples > 1 ? E + (Int)dx * msaa_y(k) - (Int)dy * msaa_x(k) : E) >> 8;
+            if (sizeof(Int) > 4) f = max(min(f, (Int)1 << 30), -((Int)1 << 30));
+            q[k][i] = (int32_t)f;
+            if (q[k][i] + most < 0) rejected |= 1u << k;
         }
     }
-    if (!in) return;
-    float fx, fy;
-    if (L.near_origin) {
-        // exact: both terms are integers below 2^24
-        fx = (float)(PXo - L.X0) + (float)(lx * 256);
-        fy = (float)(PYo - L.Y0) + (float)(ly * 256);
-    } else {
-        fx = (float)(px * 256 + ox - L.X0);
-        fy = (float)(py * 256 + oy - L.Y0);
-    }
-    const float z = biased_depth(fmaf(L.dzdx, fx, fmaf(L.dzdy, fy, L.z0)), L.bias);
-    write_fragment<kWriteId>(T, px, py, z, L.id);
+    return rejected != (1u << kSamples) - 1u;
 }
 
-// Incremental walk over the stamps of a medium record in raster order. Each
-// lane holds its edge values, its float offsets from vertex 0 and the address of
-// its pixel's word; moving one stamp right adds a constant, moving to the next
-// stamp row restarts from the row's first stamp. The float offsets stay exact
-// integers below 2^24, so the depth is bit-identical to
-// fma(dzdx, (float)(PX-X0), fma(dzdy, (float)(PY-Y0), z0)).
-template <bool kWriteId>
-struct MediumWalk {
-    int32_t e[3], er[3], stepx[3], stepy[3];
-    float fx, fxr, fy, zrow;
-    int px, pxr, py;
-    TargetWord<kWriteId>* w;   // the lane's pixel in the current stamp
-    TargetWord<kWriteId>* wr;  // and in the row's first stamp
-};
+// Leaves the stamp at (sx0, sy0) with edges q as entry i of w.
+template <bool kWriteId, int kSamples>
+__device__ __forceinline__ void put_stamp(const PassParams& P, const LargeRecord& L, int sx0, int sy0, int32_t PX, int32_t PY,
+                                          const int32_t (&q)[kSamples][3], int i, StampWork<kSamples>& w) {
+    const int pitch = kWriteId ? P.views[L.view & kViewMask].width : P.views[L.view & kViewMask].shadow_w;
+#pragma unroll
+    for (int k = 0; k < kSamples; ++k) w.e[k][i] = make_int4(q[k][0], q[k][1], q[k][2], sy0 * pitch + sx0);
+    w.at[i] = make_float2((float)(PX - L.X[0]), (float)(PY - L.Y[0]));
+    w.edges[i] = make_int4(L.dx[0], L.dx[1], -L.dy[0], -L.dy[1]);
+    w.plane[i] = make_int4(__float_as_int(L.z0), __float_as_int(L.dzdx), __float_as_int(L.dzdy),
+                           kWriteId ? (int)L.id : __float_as_int(L.bias));
+    const int nx = min(L.px1 - sx0, kStampW - 1), ny = min(L.py1 - sy0, kStampH - 1);  // last column and row in the box
+    w.box[i] = make_uint2(((0xffu >> (kStampW - 1 - nx)) * 0x01010101u) & (kAllLanes >> (8 * (kStampH - 1 - ny))), L.view);
+}
 
-// Edge values relative to vertex 0 in wrapping 32-bit arithmetic: for a medium
-// triangle the true value at every pixel of the walk fits in int32, so the
-// wrapped result equals it.
+// The n stamps of w, one after the other, a pixel per lane (column lx, row ly). Bit i
+// of `heads`: stamp i is the first of its record; of `cut`: its record's box is cut.
+// Offsets from vertex 0 are integers below 2^24, so their float sums are exact.
+template <bool kWriteId, int kSamples, bool kCut>
+__device__ __forceinline__ void raster_stamps(const PassParams& P, const StampWork<kSamples>& w, int n, uint32_t heads,
+                                              uint32_t cut, int lane, int lx, int ly) {
+    uint32_t cur_view = kAllLanes;  // the view whose target is held
+    int32_t l0 = 0, l1 = 0, lane_word = 0;
+    int4 plane{};
+    size_t sample_words = 0;
+    TargetWord<kWriteId>* base = nullptr;
+    const float fx = (float)(lx * 256), fy = (float)(ly * 256);
+    for (int i = 0; i < n; ++i, heads >>= 1, cut >>= 1) {
+        if (heads & 1u) {
+            const int4 d = w.edges[i];
+            l0 = d.x * ly + d.z * lx;
+            l1 = d.y * ly + d.w * lx;
+            plane = w.plane[i];
+            const uint32_t view = w.box[i].y;
+            if (view != cur_view) {
+                cur_view = view;
+                const Target T = view_target<kWriteId>(P, view);
+                base = reinterpret_cast<TargetWord<kWriteId>*>(T.ptr);
+                lane_word = ly * T.pitch + lx;
+                if (kSamples > 1) sample_words = plane_words(P, view);
+            }
+        }
+        const float2 at = w.at[i];
+        int4 e = w.e[0][i];
+        auto* const word = base + (e.w + lane_word);
+        if (kCut && (cut & 1u) && !((w.box[i].x >> lane) & 1u)) continue;
+#pragma unroll
+        for (int k = 0; k < kSamples; ++k) {
+            if (k) e = w.e[k][i];
+            // the third edge's lane term is minus the sum of the others'
+            if (((e.x + l0) | (e.y + l1) | (e.z - l0 - l1)) < 0) continue;
+            const float px = at.x + (kSamples > 1 ? fx + (float)msaa_x(k) : fx);
+            const float py = at.y + (kSamples > 1 ? fy + (float)msaa_y(k) : fy);
+            const float z = fmaf(__int_as_float(plane.y), px, fmaf(__int_as_float(plane.z), py, __int_as_float(plane.x)));
+            write_word<kWriteId>(word + k * sample_words, biased_depth(z, kWriteId ? 0.0f : __int_as_float(plane.w)),
+                                 kWriteId ? (uint32_t)plane.w : 0u);
+        }
+    }
+}
+
+// A pixel of a stamp of any record: 64-bit edge functions, float offsets rounded once.
 template <bool kWriteId>
-__device__ __forceinline__ void medium_start(const Target& T, const LargeRecord& L, uint32_t sx, uint32_t sy, int lx, int ly,
-                                             int32_t ox, int32_t oy, MediumWalk<kWriteId>& w) {
-    w.pxr = L.px0 + lx;
-    w.px = w.pxr + (int)sx * kStampW;
-    w.py = L.py0 + (int)sy * kStampH + ly;
-    const int32_t rx = w.px * 256 + ox - L.X0, ry = w.py * 256 + oy - L.Y0, rxr = w.pxr * 256 + ox - L.X0;
+__device__ __forceinline__ void raster_far_pixel(const Target& T, const LargeRecord& L, int px, int py, int32_t ox, int32_t oy) {
+    if (px > L.px1 || py > L.py1) return;
+    const int32_t PX = px * 256 + ox, PY = py * 256 + oy;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const int a = (i + 1) % 3;
-        const uint32_t dx = (uint32_t)L.dx[i], dy = (uint32_t)L.dy[i];
-        const uint32_t c = dy * (uint32_t)(L.X[a] - L.X0) - dx * (uint32_t)(L.Y[a] - L.Y0) - L.tl_bias[i];
-        w.e[i] = (int32_t)(c + dx * (uint32_t)ry - dy * (uint32_t)rx);
-        w.er[i] = (int32_t)(c + dx * (uint32_t)ry - dy * (uint32_t)rxr);
-        w.stepx[i] = (int32_t)(0u - dy * (uint32_t)(kStampW * 256));
-        w.stepy[i] = (int32_t)(dx * (uint32_t)(kStampH * 256));
+        if ((int64_t)L.dx[i] * ((int64_t)PY - L.Y[a]) - (int64_t)L.dy[i] * ((int64_t)PX - L.X[a]) - (int64_t)L.tl_bias[i] < 0) return;
     }
-    w.fx = (float)rx;
-    w.fxr = (float)rxr;
-    w.fy = (float)ry;
-    w.zrow = fmaf(L.dzdy, w.fy, L.z0);
-    w.wr = target_word<kWriteId>(T, w.pxr, w.py);
-    w.w = w.wr + (int)sx * kStampW;
-}
-
-// n stamps of the walk from stamp column sx: runs along a stamp row, then the
-// move to the next row.
-template <bool kWriteId, bool kBoxCheck>
-__device__ __forceinline__ void medium_walk(const Target& T, const LargeRecord& L, uint32_t sx, uint32_t n,
-                                            MediumWalk<kWriteId>& w) {
-    const size_t row_step = (size_t)kStampH * (size_t)T.pitch;
-    while (true) {
-        const uint32_t run = min(n, L.nsx - sx);
-        for (uint32_t j = 0; j < run; ++j) {
-            if (((w.e[0] | w.e[1] | w.e[2]) >= 0) && (!kBoxCheck || (w.px <= L.px1 && w.py <= L.py1)))
-                write_word<kWriteId>(w.w, biased_depth(fmaf(L.dzdx, w.fx, w.zrow), L.bias), L.id);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) w.e[i] = (int32_t)((uint32_t)w.e[i] + (uint32_t)w.stepx[i]);
-            w.w += kStampW;
-            w.fx += (float)(kStampW * 256);
-            if (kBoxCheck) w.px += kStampW;
-        }
-        n -= run;
-        if (n == 0) return;
-        sx = 0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            w.er[i] = (int32_t)((uint32_t)w.er[i] + (uint32_t)w.stepy[i]);
-            w.e[i] = w.er[i];
-        }
-        w.wr += row_step;
-        w.w = w.wr;
-        w.fx = w.fxr;
-        w.fy += (float)(kStampH * 256);
-        w.zrow = fmaf(L.dzdy, w.fy, L.z0);
-        if (kBoxCheck) {
-            w.px = w.pxr;
-            w.py += kStampH;
-        }
-    }
-}
-
-// The walk over a medium record's stamps at the four standard sample positions:
-// the edge values at the pixels' corners, to which each sample adds constants (the
-// sums are the values medium_start computes for that sample, in wrapping 32-bit
-// arithmetic), the word of each sample a plane further. What a record segment costs
-// before its first stamp (decode, start values: 220 warp instructions for 4 stamps
-// of 13) is then paid once, not per sample: on the 1080p scene-scale frame the
-// camera raster issued 50.6 M warp instructions as four passes over the records,
-// and the frame goes from 307 to 286 us.
-template <bool kBoxCheck>
-__device__ __forceinline__ void medium_walk_msaa(const Target& T, size_t plane, const LargeRecord& L, uint32_t sx, uint32_t sy,
-                                                 uint32_t n, int lx, int ly) {
-    MediumWalk<true> w;
-    medium_start<true>(T, L, sx, sy, lx, ly, 0, 0, w);
-    int32_t off[kMsaaSamples][3];
-    float zrow[kMsaaSamples];
-#pragma unroll
-    for (int k = 0; k < kMsaaSamples; ++k) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            off[k][i] = (int32_t)((uint32_t)L.dx[i] * (uint32_t)msaa_y(k) - (uint32_t)L.dy[i] * (uint32_t)msaa_x(k));
-        zrow[k] = fmaf(L.dzdy, w.fy + (float)msaa_y(k), L.z0);
-    }
-    const size_t row_step = (size_t)kStampH * (size_t)T.pitch;
-    while (true) {
-        const uint32_t run = min(n, L.nsx - sx);
-        for (uint32_t j = 0; j < run; ++j) {
-            if (!kBoxCheck || (w.px <= L.px1 && w.py <= L.py1)) {
-#pragma unroll
-                for (int k = 0; k < kMsaaSamples; ++k) {
-                    const int32_t e0 = (int32_t)((uint32_t)w.e[0] + (uint32_t)off[k][0]);
-                    const int32_t e1 = (int32_t)((uint32_t)w.e[1] + (uint32_t)off[k][1]);
-                    const int32_t e2 = (int32_t)((uint32_t)w.e[2] + (uint32_t)off[k][2]);
-                    if ((e0 | e1 | e2) >= 0)
-                        write_word<true>(w.w + k * plane, biased_depth(fmaf(L.dzdx, w.fx + (float)msaa_x(k), zrow[k]), L.bias),
-                                         L.id);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) w.e[i] = (int32_t)((uint32_t)w.e[i] + (uint32_t)w.stepx[i]);
-            w.w += kStampW;
-            w.fx += (float)(kStampW * 256);
-            if (kBoxCheck) w.px += kStampW;
-        }
-        n -= run;
-        if (n == 0) return;
-        sx = 0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            w.er[i] = (int32_t)((uint32_t)w.er[i] + (uint32_t)w.stepy[i]);
-            w.e[i] = w.er[i];
-        }
-        w.wr += row_step;
-        w.w = w.wr;
-        w.fx = w.fxr;
-        w.fy += (float)(kStampH * 256);
-#pragma unroll
-        for (int k = 0; k < kMsaaSamples; ++k) zrow[k] = fmaf(L.dzdy, w.fy + (float)msaa_y(k), L.z0);
-        if (kBoxCheck) {
-            w.px = w.pxr;
-            w.py += kStampH;
-        }
-    }
+    const float z = fmaf(L.dzdx, (float)(PX - L.X[0]), fmaf(L.dzdy, (float)(PY - L.Y[0]), L.z0));
+    write_fragment<kWriteId>(T, px, py, biased_depth(z, L.bias), L.id);
 }
 
 // Persistent raster: each warp first takes batches of 32 small records (one per
-// lane), then chunks of kChunkStamps stamps of the large records, both in a
-// fixed grid-stride order. (A shared cursor that every warp bumps with an
-// atomic serialises on one L2 line: a raster launch with its work skipped took
-// 12 us that way on the 4096^2 shadow pass of 262,144 triangles, 6 us without.)
+// lane), then chunks of chunk_stamps stamps of the large records, both in a fixed
+// grid-stride order. (A shared cursor that every warp bumps with an atomic
+// serialises on one L2 line: a raster launch with its work skipped took 12 us that
+// way on the 4096^2 shadow pass of 262,144 triangles, 6 us without.)
+//
+// A chunk goes 32 stamps at a time, of as many records as they belong to. Each lane
+// first prepares one stamp: finds its record, evaluates the edges at the stamp's
+// first pixel, drops it if an edge rejects it whole, and leaves what the pixels need
+// in shared memory. Then the warp takes the stamps that are left one after the
+// other, a pixel per lane. What is the same for all pixels of a stamp is so computed
+// once instead of by 32 lanes, a record costs nothing beyond its stamps (the chunks
+// of a shadow pass of 262,144 triangles hold 3.4 records each, 100-odd instructions
+// to decode and start), and an empty stamp (over a third of a triangle's box) costs
+// a thirty-second of its preparation. Against one lane per pixel throughout, with
+// 64-bit edges for triangles above 90 pixels: 640x360 triangle soup frame 89 -> 43
+// us, 3840x2160 with a million triangles and four cascades 975 -> 856 us, 1080p
+// scene-scale shadow raster 70 -> 62 us (now the shared-memory path is 76 % busy:
+// broadcasts, then the atomics). Four CTAs per SM were slower (62 -> 69 us).
 template <bool kWriteId, bool kMsaa>
 __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
+    constexpr int kSamples = kMsaa ? kMsaaSamples : 1;
+    constexpr int kStageRecords = kMsaa ? kStageRecordsMax / 2 : kStageRecordsMax;
     __shared__ int4 s_stage[kRasterThreads / 32][2][kStageRecords][4];
+    __shared__ StampWork<kSamples> s_work[kRasterThreads / 32];
     const int lane = threadIdx.x & 31;
     const int lx = lane & (kStampW - 1), ly = lane >> 3;
     // a multisampled pass's launches number their warps together
@@ -1126,89 +1001,100 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
     const uint32_t chunks = P.header->chunks;
     const uint64_t total = P.header->stamps;
     const uint32_t n_rec = min(P.header->records, P.record_capacity);  // records the setup wrote
-    uint32_t cur_view = 0xffffffffu;  // the view whose target T holds
-    Target T{nullptr, 0};
-    size_t plane = 0;
+    StampWork<kSamples>& work = s_work[threadIdx.x >> 5];
     // chunk k's first record (r_cur, staged in buffer cb), the next chunk's (r_next)
     int cb = 0;
     uint32_t r_cur = warp_id < chunks ? P.chunk_map[warp_id] : n_rec;
-    stage_records(s_stage[threadIdx.x >> 5][0], P.records, r_cur, n_rec, lane);
+    stage_records<kStageRecords>(s_stage[threadIdx.x >> 5][0], P.records, r_cur, n_rec, lane);
     uint32_t r_next = (uint64_t)warp_id + warps < chunks ? P.chunk_map[warp_id + warps] : n_rec;
     for (uint32_t k = warp_id; k < chunks; k += warps) {
-        uint64_t s = (uint64_t)k * P.chunk_stamps;
-        const uint64_t s_end = (s + P.chunk_stamps < total) ? (s + P.chunk_stamps) : total;
+        const uint64_t s0 = (uint64_t)k * P.chunk_stamps;
+        const uint64_t s_end = (s0 + P.chunk_stamps < total) ? (s0 + P.chunk_stamps) : total;
         // stage the next chunk's records while this one is rasterised, and fetch
         // the chunk map entry of the one after
-        stage_records(s_stage[threadIdx.x >> 5][cb ^ 1], P.records, r_next, n_rec, lane);
+        stage_records<kStageRecords>(s_stage[threadIdx.x >> 5][cb ^ 1], P.records, r_next, n_rec, lane);
         const uint64_t k_after = (uint64_t)k + 2u * (uint64_t)warps;
         const uint32_t r_after = k_after < chunks ? P.chunk_map[k_after] : n_rec;
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this lane's copies of chunk k
         __syncwarp();                                          // and every other lane's
-        int4 (*const st)[4] = s_stage[threadIdx.x >> 5][cb];
-        uint32_t r = r_cur;
-        while (s < s_end) {
-            if (r >= P.record_capacity) break;
+        const int4 (*const st)[4] = s_stage[threadIdx.x >> 5][cb];
+        uint32_t r_first = r_cur;  // the record of the first of the 32 stamps
+        for (uint64_t s = s0; s < s_end; s += 32) {
+            // the stamps' records: lane l looks where record r_first + l starts, and each
+            // stamp's record is the last that starts at or before it (a record has a stamp)
+            uint32_t starts = 0;
+            if (lane > 0 && (uint64_t)r_first + lane < n_rec) {
+                const uint32_t j = r_first - r_cur + lane;
+                const int4 q3 = j < (uint32_t)kStageRecords ? st[j][3] : __ldg(reinterpret_cast<const int4*>(P.records + r_first + lane) + 3);
+                const uint64_t begin = (uint64_t)(uint32_t)q3.z | ((uint64_t)((uint32_t)q3.w & 0xffu) << 32);
+                if (begin > s && begin < s + 32) starts = 1u << (uint32_t)(begin - s);
+            }
+            starts = __reduce_or_sync(kAllLanes, starts);
+            const uint32_t r = r_first + __popc(starts & (kAllLanes >> (31 - lane)));
+            uint32_t r_after_this = r;  // the record of the stamp after this one
+            bool live = false, far = false;
+            int sx0 = 0, sy0 = 0;
+            int32_t PX = 0, PY = 0;  // the sample of the stamp's first pixel (its corner with 4x samples)
+            int32_t q[kSamples][3];
             LargeRecord L;
-            const uint32_t j = r - r_cur;
-            if (j < (uint32_t)kStageRecords && r < n_rec) decode_large(st[j][0], st[j][1], st[j][2], st[j][3], L);
-            else load_large(P.records + r, L);
-            if (s < L.begin || s >= L.end) {  // cannot happen with a consistent chunk map
-                atomicOr(P.error_flags, kErrStampOverflow);
-                break;
+            if (s + lane < s_end && r < n_rec) {
+                const uint32_t j = r - r_cur;
+                if (j < (uint32_t)kStageRecords) decode_large(st[j][0], st[j][1], st[j][2], st[j][3], L);
+                else load_large(P.records + r, L);
+                if (s + lane >= L.begin && s + lane < L.end) {
+                    // stamp i of the record, below 2^24: the quotient by stamps per row, off by one at most
+                    const int i = (int)(s + lane - L.begin), nsx = (int)L.nsx;
+                    int sy = (int)__fdividef((float)i, (float)nsx), sx = i - sy * nsx;
+                    if (sx < 0) {
+                        --sy;
+                        sx += nsx;
+                    } else if (sx >= nsx) {
+                        ++sy;
+                        sx -= nsx;
+                    }
+                    sx0 = L.px0 + sx * kStampW;
+                    sy0 = L.py0 + sy * kStampH;
+                    PX = sx0 * 256 + (kMsaa ? 0 : P.sample_x);
+                    PY = sy0 * 256 + (kMsaa ? 0 : P.sample_y);
+                    if (s + lane + 1 == L.end) ++r_after_this;
+                    far = !L.near_origin;
+                    live = !far;
+                } else {  // cannot happen with a consistent chunk map
+                    atomicOr(P.error_flags, kErrStampOverflow);
+                }
             }
-            const uint64_t seg_end = s_end < L.end ? s_end : L.end;
-            const uint32_t n = (uint32_t)(seg_end - s);
-            const uint32_t i = (uint32_t)(s - L.begin);
-            const uint32_t sy = i ? i / L.nsx : 0u, sx = i - sy * L.nsx;  // a segment mostly starts at its record's first stamp
-            if (L.view != cur_view) {
-                T = view_target<kWriteId>(P, L.view);
-                if (kMsaa) plane = plane_words(P, L.view);
-                cur_view = L.view;
+            if (__all_sync(kAllLanes, !live || L.small)) live = live && stamp_edges<kSamples, int32_t>(L, PX, PY, q);
+            else live = live && stamp_edges<kSamples, int64_t>(L, PX, PY, q);
+            // the stamps that are left, in order: entry `at`; the first one of its record is a head
+            const uint32_t left = __ballot_sync(kAllLanes, live), below = left & ((1u << lane) - 1u);
+            const int at = __popc(below);
+            uint32_t head = 0, cut = 0;
+            if (live) {
+                put_stamp<kWriteId, kSamples>(P, L, sx0, sy0, PX, PY, q, at, work);
+                // record starts after the stamp left before this one
+                const uint32_t since = below ? starts & (kAllLanes >> (31 - lane)) & ~(kAllLanes >> __clz(below)) : kAllLanes;
+                head = since ? 1u << at : 0u;
+                cut = L.cut ? 1u << at : 0u;
             }
-            if (kMsaa) {
-                if (L.medium) {
-                    if (L.clipped) medium_walk_msaa<true>(T, plane, L, sx, sy, n, lx, ly);
-                    else medium_walk_msaa<false>(T, plane, L, sx, sy, n, lx, ly);
-                } else {
-                    GenericEdges G;
-                    generic_edges(L, G);
+            const uint32_t heads = __reduce_or_sync(kAllLanes, head), cuts = __reduce_or_sync(kAllLanes, cut);
+            __syncwarp();
+            if (cuts) raster_stamps<kWriteId, kSamples, true>(P, work, __popc(left), heads, cuts, lane, lx, ly);
+            else raster_stamps<kWriteId, kSamples, false>(P, work, __popc(left), heads, 0u, lane, lx, ly);
+            for (uint32_t m = __ballot_sync(kAllLanes, far); m; m &= m - 1) {
+                const int j = __ffs(m) - 1;
+                load_large(P.records + __shfl_sync(kAllLanes, r, j), L);
+                const int px = __shfl_sync(kAllLanes, sx0, j) + lx, py = __shfl_sync(kAllLanes, sy0, j) + ly;
+                const Target T = view_target<kWriteId>(P, L.view);
+                const size_t plane = kMsaa ? plane_words(P, L.view) : 0;
 #pragma unroll 1
-                    for (int k = 0; k < kMsaaSamples; ++k) {
-                        const Target Tk{reinterpret_cast<TargetWord<kWriteId>*>(T.ptr) + k * plane, T.pitch};
-                        GenericWalk w;
-                        generic_start(L, G, sx, sy, msaa_x(k), msaa_y(k), w);
-                        for (uint32_t j = 0; j < n; ++j) {
-                            raster_stamp<kWriteId, true>(Tk, L, G, w, lx, ly, msaa_x(k), msaa_y(k));
-                            generic_next(L, w);
-                        }
-                    }
-                }
-            } else if (L.medium) {
-                MediumWalk<kWriteId> w;
-                medium_start<kWriteId>(T, L, sx, sy, lx, ly, P.sample_x, P.sample_y, w);
-                if (L.clipped) medium_walk<kWriteId, true>(T, L, sx, n, w);
-                else medium_walk<kWriteId, false>(T, L, sx, n, w);
-            } else {
-                GenericEdges G;
-                generic_edges(L, G);
-                GenericWalk w;
-                generic_start(L, G, sx, sy, P.sample_x, P.sample_y, w);
-                if (L.clipped) {
-                    for (uint32_t j = 0; j < n; ++j) {
-                        raster_stamp<kWriteId, true>(T, L, G, w, lx, ly, P.sample_x, P.sample_y);
-                        generic_next(L, w);
-                    }
-                } else {
-                    for (uint32_t j = 0; j < n; ++j) {
-                        raster_stamp<kWriteId, false>(T, L, G, w, lx, ly, P.sample_x, P.sample_y);
-                        generic_next(L, w);
-                    }
+                for (int i = 0; i < kSamples; ++i) {
+                    const Target Ti{reinterpret_cast<TargetWord<kWriteId>*>(T.ptr) + i * plane, T.pitch};
+                    raster_far_pixel<kWriteId>(Ti, L, px, py, kMsaa ? msaa_x(i) : P.sample_x, kMsaa ? msaa_y(i) : P.sample_y);
                 }
             }
-            s = seg_end;
-            ++r;
+            r_first = __shfl_sync(kAllLanes, r_after_this, 31);
+            __syncwarp();  // every lane is done with the stamps (and, at the chunk's end, its records)
         }
-        __syncwarp();  // every lane is done with this buffer before it is staged again
         r_cur = r_next;
         r_next = r_after;
         cb ^= 1;

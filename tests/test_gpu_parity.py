@@ -272,6 +272,33 @@ def test_msaa_raster_parts(gpu, oracle, chunk_stamps, small_extent, spread):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("chunk_stamps,small_extent", [(8, 1), (16, 4), (33, 2), (64, 1), (256, 16)])
+@pytest.mark.parametrize("spread,fov", [(0.03, 60.0), (0.3, 60.0), (1.0, 60.0), (1.0, 1.5)])
+def test_raster_chunks(gpu, oracle, chunk_stamps, small_extent, spread, fov):
+    """Chunks of fewer and of more than 32 stamps, of records of one stamp (more records than are staged) to
+    screen-sized ones, boxes cut by the viewport, and (narrow field of view) vertices far outside it."""
+    s = sc.random_triangles(seed=53, triangles=1500, width=318, height=211, shadow_size=190, texture_size=32, fov_deg=fov)
+    v = s.vertices[:, 0:3].reshape(-1, 3, 3)
+    s.vertices[:, 0:3] = (v[:, :1] + (v - v[:, :1]) * np.float32(spread)).reshape(-1, 3)
+    ref = oracle.render(s)
+    g = Graphics()
+    g.init(s.width, s.height, s.shadow_size)
+    try:
+        g.set_asset(s)
+        g.set_graphic_objects(s.objects, s.surfaces)
+        g.set_draw_config(s.draw_config)
+        g.set_tuning(chunk_stamps, small_extent)
+        g.update(s.scene)
+        g.render()
+        if g.sync_code() == 14:
+            g.render()
+        g.sync()
+        check_parity(s, ref, g.download())
+    finally:
+        g.deinit()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("samples", [1, 4])
 @pytest.mark.parametrize("width,height,triangles,spread,mask", [
     (48, 40, 24000, 0.05, False),  # over 8,192 records (a window of group boxes), hundreds to a tile
