@@ -201,7 +201,7 @@ struct rz_ctx {
     DrawConsts* d_camera_consts = nullptr;
     DrawConsts* d_blended_consts = nullptr;
     float4* d_varyings = nullptr;
-    uint4* d_tri_refs = nullptr;  // per opaque, then per blended triangle: its draw and varying records (written by the setups)
+    uint4* d_tri_refs = nullptr;  // per opaque, then per blended triangle: its material and varying records (written by the setups)
     uint32_t varying_count = 0, blended_varying_base = 0;
     bool layout_dirty = true;        // draw lists, pools and view table need a rebuild
 

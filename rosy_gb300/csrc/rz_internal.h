@@ -184,8 +184,8 @@ struct PassParams {
     void* clear_ptr[2];
     size_t clear_bytes[2];
     uint32_t clear_count;
-    // camera passes only (else null): per triangle with valid indices, its draw and
-    // its three varying record indices, for the shading
+    // camera passes only (else null): per triangle with valid indices, its draw's
+    // material and its three varying record indices, for the shading
     uint4* tri_refs;
 };
 
@@ -211,7 +211,7 @@ struct ShadeParams {
     int blended;                  // 1: k_shade stores the RGBA16F draw image (color16) for k_blend
     uint32_t samples;             // camera-pass samples per pixel of the views (1 or 4)
     uint32_t gbuffer;             // 1: the views have a G-buffer (ViewRec::gb_albedo)
-    // the camera setup's per-triangle (draw, varying record of each vertex), indexed
+    // the camera setup's per-triangle (material, varying record of each vertex), indexed
     // by the triangle id of the pass (opaque or blended)
     const uint4* tri_refs;
 };

@@ -298,7 +298,7 @@ __device__ __forceinline__ void setup_triangle(const PassParams& P, uint32_t tri
         atomicOr(P.error_flags, kErrBadIndex);
         return;
     }
-    emit.source(d, vi[0] - dr.vertex_base + dr.varying_base, vi[1] - dr.vertex_base + dr.varying_base,
+    emit.source((uint32_t)dr.material, vi[0] - dr.vertex_base + dr.varying_base, vi[1] - dr.vertex_base + dr.varying_base,
                 vi[2] - dr.vertex_base + dr.varying_base);
     const ViewRec& VR = P.views[dr.view];
     ViewState V;
@@ -381,14 +381,14 @@ struct CountEmit {
     uint32_t small = 0;
     TriRecord first;       // the first record, kept for the common case of exactly one
     bool first_small = false;
-    uint4* refs = nullptr; // opaque camera pass: where the triangle's draw and vertex records go
+    uint4* refs = nullptr; // camera passes: where the triangle's material and vertex records go
     uint32_t tri = 0;
-    // every triangle with valid indices stores its draw and the varying records of
-    // its vertices: a triangle that owns a pixel of the visibility buffer is one of
+    // every triangle with valid indices stores its material and the varying records
+    // of its vertices: a triangle that owns a pixel of the visibility buffer is one of
     // them, and the shading finds them here (one load instead of a search of the
-    // draw list and the index buffer)
-    __device__ void source(uint32_t d, uint32_t v0, uint32_t v1, uint32_t v2) {
-        if (refs) refs[tri] = make_uint4(d, v0, v1, v2);
+    // draw list and the index buffer, and no dependent load of the draw's material)
+    __device__ void source(uint32_t material, uint32_t v0, uint32_t v1, uint32_t v2) {
+        if (refs) refs[tri] = make_uint4(material, v0, v1, v2);
     }
     __device__ void operator()(const TriRecord& r, bool is_small) {
         if (recs + small == 0) {

@@ -56,6 +56,41 @@ __device__ __forceinline__ V3 mulm3v(const float* N, V3 v) {
     return {N[0] * v.x + N[3] * v.y + N[6] * v.z, N[1] * v.x + N[4] * v.y + N[7] * v.z, N[2] * v.x + N[5] * v.y + N[8] * v.z};
 }
 
+// Two floats in a register pair, and the packed operations on them: each half rounds
+// as the scalar operation does, in one instruction instead of two (the fragment stage
+// is short of issue slots, not of multipliers).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 both(float x) { return pack2(x, x); }
+__device__ __forceinline__ void unpack2(F2 p, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// The products: a * b - 0, whose sums round like a * b. The assembler contracts a packed
+// multiply and the add after it into one multiply-add (whatever -fmad says, and with a
+// literal -0 too), which rounds once; it does not know this value.
+__constant__ unsigned long long c_minus_zeros = 0x8000000080000000ull;
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return fma2(a, b, F2{c_minus_zeros}); }
+__device__ __forceinline__ F2 mix2(F2 x, F2 y, F2 w) { return x + w * (y - x); }
+
 // ---------------------------------------------------------------------------
 // per-draw constants
 // ---------------------------------------------------------------------------
@@ -238,15 +273,13 @@ __device__ __forceinline__ int wrap_coord(int i, int size, int mode) {
     return size - 1 - a;
 }
 
-// Where a texture.Sample call reads: the level(s), the wrapped texel columns
-// and rows and the filter weights. It depends only on the texture's size and
+// Where a texture.Sample call reads: the level(s), their wrapped texels and the
+// filter weights. It depends only on the texture's size and
 // level count, the sampler and the uv/derivatives, so textures that share those
 // share one SampleCoords (the three material textures usually do).
 struct LevelCoords {
-    uint32_t off;   // texel offset of the level
-    int w;          // level width (row pitch)
-    int x0, x1, y0, y1;
-    float a, b;     // bilinear weights (unused for nearest)
+    uint32_t i00, i10, i01, i11;  // the texels, from the texture's first
+    float a, b;                   // bilinear weights (unused for nearest)
 };
 
 struct SampleCoords {
@@ -262,15 +295,12 @@ struct SampleCoords {
 __device__ __forceinline__ void level_coords(const TexDesc& t, int level, bool linear, SamplerBits st, float u, float v,
                                              LevelCoords& c) {
     const int w = max(1, (int)(t.width >> level)), h = max(1, (int)(t.height >> level));
-    c.off = t.level_off[level];
-    c.w = w;
+    const uint32_t off = t.level_off[level];
     const int wu = (st >> 4) & 3, wv = (st >> 6) & 3;
     if (!linear) {
         const int i = (int)floorf(u * (float)w), j = (int)floorf(v * (float)h);
-        c.x0 = wrap_coord(i, w, wu);
-        c.y0 = wrap_coord(j, h, wv);
-        c.x1 = c.x0;
-        c.y1 = c.y0;
+        c.i00 = off + (uint32_t)wrap_coord(j, h, wv) * (uint32_t)w + (uint32_t)wrap_coord(i, w, wu);
+        c.i10 = c.i01 = c.i11 = c.i00;
         c.a = c.b = 0.0f;
         return;
     }
@@ -279,10 +309,12 @@ __device__ __forceinline__ void level_coords(const TexDesc& t, int level, bool l
     c.a = uu - fi;
     c.b = vv - fj;
     const int i0 = (int)fi, j0 = (int)fj;
-    c.x0 = wrap_coord(i0, w, wu);
-    c.x1 = wrap_coord(i0 + 1, w, wu);
-    c.y0 = wrap_coord(j0, h, wv);
-    c.y1 = wrap_coord(j0 + 1, h, wv);
+    const uint32_t x0 = (uint32_t)wrap_coord(i0, w, wu), x1 = (uint32_t)wrap_coord(i0 + 1, w, wu);
+    const uint32_t r0 = off + (uint32_t)wrap_coord(j0, h, wv) * (uint32_t)w, r1 = off + (uint32_t)wrap_coord(j0 + 1, h, wv) * (uint32_t)w;
+    c.i00 = r0 + x0;
+    c.i10 = r0 + x1;
+    c.i01 = r1 + x0;
+    c.i11 = r1 + x1;
 }
 
 // Level selection of texture.Sample with implicit derivatives (Vulkan LOD rules).
@@ -329,73 +361,96 @@ __device__ __forceinline__ void sample_coords(const TexDesc& t, SamplerBits st, 
     }
 }
 
-// byte / 255 rounded to nearest: the product with the rounded reciprocal and one
-// residual step, exact for every byte (it equals the IEEE quotient, as a table
-// of (float)b / 255.0f would, without the shared-memory lookup and its bank
-// conflicts).
+// byte / 255 rounded to nearest: the reciprocal as two floats, the small part's
+// product in the addend of the large one's; exact for every byte (it equals the IEEE
+// quotient, as a table of (float)b / 255.0f would, without the shared-memory lookup
+// and its bank conflicts).
 __device__ __forceinline__ float unorm8(uint32_t b) {
     const float x = (float)b, r = 1.0f / 255.0f;
-    const float q = x * r;
-    return fmaf(fmaf(-q, 255.0f, x), r, q);
+    const float rest = (float)(1.0 / 255.0 - (double)r);
+    return fmaf(x, r, x * rest);
+}
+
+__device__ __forceinline__ F2 unorm8x2(uint32_t lo, uint32_t hi) {
+    const float r = 1.0f / 255.0f, rest = (float)(1.0 / 255.0 - (double)r);
+    const F2 x = pack2((float)lo, (float)hi);
+    return fma2(x, both(r), x * both(rest));
 }
 
 struct Sampler {
     const ShadeParams* P;
     const float* srgb;   // shared-memory table: sRGB byte -> linear
 
-    __device__ __forceinline__ void texel(const TexDesc& t, uint32_t off, int w, int i, int j, float out[4]) const {
-        const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(t.base) + off + (uint32_t)j * (uint32_t)w + (uint32_t)i);
+    // The channels of a texel that a caller reads: G and B always, R (and alpha) on demand.
+    enum { kGB = 0, kRGB = 1, kRGBA = 2 };
+    struct Texel {
+        F2 gb, ra;
+    };
+
+    template <int kChannels>
+    __device__ __forceinline__ Texel decode(bool is_srgb, uint32_t v) const {
         const uint32_t r = v & 0xffu, g = (v >> 8) & 0xffu, b = (v >> 16) & 0xffu, a = v >> 24;
-        if (t.srgb) {
-            out[0] = srgb[r];
-            out[1] = srgb[g];
-            out[2] = srgb[b];
+        Texel o;
+        o.ra.v = 0;
+        if (is_srgb) {
+            o.gb = pack2(srgb[g], srgb[b]);
+            if (kChannels == kRGB) o.ra = both(srgb[r]);
+            if (kChannels == kRGBA) o.ra = pack2(srgb[r], unorm8(a));
         } else {
-            out[0] = unorm8(r);
-            out[1] = unorm8(g);
-            out[2] = unorm8(b);
+            o.gb = unorm8x2(g, b);
+            if (kChannels == kRGB) o.ra = both(unorm8(r));
+            if (kChannels == kRGBA) o.ra = unorm8x2(r, a);
         }
-        out[3] = unorm8(a);
+        return o;
     }
 
-    __device__ __forceinline__ void fetch_level(const TexDesc& t, const LevelCoords& c, bool linear, float out[4]) const {
-        if (!linear) {
-            texel(t, c.off, c.w, c.x0, c.y0, out);
-            return;
-        }
-        float t00[4], t10[4], t01[4], t11[4];
-        texel(t, c.off, c.w, c.x0, c.y0, t00);
-        texel(t, c.off, c.w, c.x1, c.y0, t10);
-        texel(t, c.off, c.w, c.x0, c.y1, t01);
-        texel(t, c.off, c.w, c.x1, c.y1, t11);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float top = t00[k] + c.a * (t10[k] - t00[k]);
-            const float bot = t01[k] + c.a * (t11[k] - t01[k]);
-            out[k] = top + c.b * (bot - top);
-        }
+    __device__ __forceinline__ void load_level(const TexDesc& t, const LevelCoords& c, uint32_t q[4]) const {
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(t.base);
+        q[0] = __ldg(p + c.i00);
+        q[1] = __ldg(p + c.i10);
+        q[2] = __ldg(p + c.i01);
+        q[3] = __ldg(p + c.i11);
+    }
+
+    template <int kChannels>
+    __device__ __forceinline__ Texel filter_level(bool is_srgb, const LevelCoords& c, bool linear, const uint32_t q[4]) const {
+        Texel o = decode<kChannels>(is_srgb, q[0]);
+        if (!linear) return o;
+        const Texel t10 = decode<kChannels>(is_srgb, q[1]), t01 = decode<kChannels>(is_srgb, q[2]), t11 = decode<kChannels>(is_srgb, q[3]);
+        const F2 a = both(c.a), b = both(c.b);
+        o.gb = mix2(mix2(o.gb, t10.gb, a), mix2(t01.gb, t11.gb, a), b);
+        if (kChannels != kGB) o.ra = mix2(mix2(o.ra, t10.ra, a), mix2(t01.ra, t11.ra, a), b);
+        return o;
     }
 
     // texture.Sample(sampler, uv) with implicit derivatives. `cache` holds the
     // coordinates of the previous call and is reused when the texture's size,
-    // levels and sampler match.
-    __device__ void sample(uint32_t tex_index, uint32_t sampler_index, const Frag& f, SampleCoords& cache, float out[4]) const {
-        if (tex_index >= P->texture_count) {  // absent image: robust null descriptor reads 0
-            out[0] = out[1] = out[2] = out[3] = 0.0f;
-            return;
-        }
+    // levels and sampler match. Channels that the caller does not read are 0.
+    template <int kChannels>
+    __device__ __forceinline__ void sample(uint32_t tex_index, uint32_t sampler_index, const Frag& f, SampleCoords& cache,
+                                           float out[4]) const {
+        out[0] = out[1] = out[2] = out[3] = 0.0f;
+        if (tex_index >= P->texture_count) return;  // absent image: robust null descriptor reads 0
         const TexDesc& t = P->textures[tex_index];
         const SamplerBits st = P->samplers[min(sampler_index, P->sampler_count)];
         if (!(cache.valid && cache.width == t.width && cache.height == t.height && cache.levels == t.levels &&
               cache.st == st))
             sample_coords(t, st, f.uv, f.duvdx, f.duvdy, cache);
-        fetch_level(t, cache.l0, cache.linear, out);
+        const bool is_srgb = t.srgb != 0;
+        uint32_t q0[4], q1[4];  // both levels' texels before either is filtered: one trip to memory, not two
+        load_level(t, cache.l0, q0);
+        if (cache.two) load_level(t, cache.l1, q1);
+        Texel o = filter_level<kChannels>(is_srgb, cache.l0, cache.linear, q0);
         if (cache.two) {
-            float b[4];
-            fetch_level(t, cache.l1, cache.linear, b);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) out[k] = out[k] + cache.delta * (b[k] - out[k]);
+            const Texel hi = filter_level<kChannels>(is_srgb, cache.l1, cache.linear, q1);
+            const F2 d = both(cache.delta);
+            o.gb = mix2(o.gb, hi.gb, d);
+            if (kChannels != kGB) o.ra = mix2(o.ra, hi.ra, d);
         }
+        unpack2(o.gb, out[1], out[2]);
+        float alpha;
+        if (kChannels != kGB) unpack2(o.ra, out[0], alpha);
+        if (kChannels == kRGBA) out[3] = alpha;
     }
 };
 
@@ -420,6 +475,11 @@ __device__ __forceinline__ float sample_cmp(const float* __restrict__ shadow, in
 // positions are computed one by one (as the single-tap path would), and when
 // they fall on consecutive columns/rows - the usual case - the 16 compares of
 // the shared 4x4 block are done once; otherwise each tap reads its own texels.
+// Away from the map's border the block is four row pointers and constant offsets,
+// and where it is all lit or all in shadow, as in most of a frame, the taps are
+// what their sums would be: 9 ones or 9 zeros. (A block beyond float range is not
+// consecutive, so the weights here are in [0, 1).)
+// the taps took about 250: MEASURED
 __device__ float pcf3x3(const float* __restrict__ shadow, int S, const float csm[4]) {
     const float o = 1.0f / (float)S;
     int xi[3], yj[3];
@@ -438,13 +498,26 @@ __device__ float pcf3x3(const float* __restrict__ shadow, int S, const float csm
     float result = 0.0f;
     if (xi[1] == xi[0] + 1 && xi[2] == xi[0] + 2 && yj[1] == yj[0] + 1 && yj[2] == yj[0] + 2) {
         float c[4][4];
+        if (xi[0] >= 0 && yj[0] >= 0 && xi[0] + 3 < S && yj[0] + 3 < S) {
+            const float* row = shadow + (yj[0] * S + xi[0]);  // S <= 16384
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-            const size_t row = (size_t)min(max(yj[0] + y, 0), S - 1) * S;
+            for (int y = 0; y < 4; ++y, row += S) {
 #pragma unroll
-            for (int x = 0; x < 4; ++x)
-                c[y][x] = dref >= __ldg(&shadow[row + min(max(xi[0] + x, 0), S - 1)]) ? 1.0f : 0.0f;
+                for (int x = 0; x < 4; ++x) c[y][x] = dref >= __ldg(row + x) ? 1.0f : 0.0f;
+            }
+        } else {
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const int row = min(max(yj[0] + y, 0), S - 1) * S;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) c[y][x] = dref >= __ldg(shadow + (row + min(max(xi[0] + x, 0), S - 1))) ? 1.0f : 0.0f;
+            }
         }
+        float lit = 0.0f;
+#pragma unroll
+        for (int y = 0; y < 4; ++y) lit += (c[y][0] + c[y][1]) + (c[y][2] + c[y][3]);
+        if (lit == 16.0f) return 9.0f * (1.0f / 9.0f);
+        if (lit == 0.0f) return 0.0f;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
 #pragma unroll
@@ -539,43 +612,59 @@ __device__ __forceinline__ const float* select_cascade(const ViewRec& VR, const 
 // compiled into this copy. A view takes the same branches at every pixel, and
 // the shading kernel runs the specialised copy for such views: the code its
 // warps execute is then smaller (fewer instruction-fetch stalls).
-template <bool kLit = false>
-__device__ bool fragment_main(const ViewRec& VR, const rz_scene_data& sd, const GpuMaterial* md, const Frag& bv,
-                              const Sampler& smp, float out[4], float* albedo = nullptr) {
+// `late` interpolates the rest of bv (all but uv, its derivatives and csm) once the
+// shadow and the textures have been read: while they are, few values are held.
+template <bool kLit, class Late>
+__device__ __forceinline__ bool fragment_main(const ViewRec& VR, const rz_scene_data& sd, const GpuMaterial* md, Frag& bv, Late late,
+                                              const Sampler& smp, float out[4], float* albedo = nullptr) {
+    float shadowFactor = 1.0f;
+    if (kLit) {
+        float cc[4];
+        const float* map = select_cascade(VR, bv.csm, cc);
+        shadowFactor = pcf(map, VR.shadow_w, cc, VR.pcf_mode);
+    }
+    float sampledRoughness = 0.0f, sampledMetallic = 0.0f;
+    float normalTexel[4], colorTexel[4];
+    bool has_normal = false, has_color = false;
+    if (md) {
+        SampleCoords cache;
+        cache.valid = false;
+        has_normal = sd.normal_maps_enabled == 1 && md->tex[1] != RZ_INVALID_INDEX;
+        has_color = md->tex[0] != RZ_INVALID_INDEX;
+        if (has_normal) smp.sample<Sampler::kRGB>(md->tex[1], md->sampler[1], bv, cache, normalTexel);
+        if (has_color) smp.sample<Sampler::kRGBA>(md->tex[0], md->sampler[0], bv, cache, colorTexel);
+        float s[4];
+        const int mr = md->tex[3] != RZ_INVALID_INDEX ? 3 : 2;  // the mixmap, else the metallic-roughness texture
+        smp.sample<Sampler::kGB>(md->tex[mr], md->sampler[mr], bv, cache, s);
+        sampledRoughness = s[1];
+        sampledMetallic = s[2];
+    }
+    late(bv);
     const V3 ambientLight{sd.ambient_color[0], sd.ambient_color[1], sd.ambient_color[2]};
     float outFragColor[4] = {bv.color[0], bv.color[1], bv.color[2], bv.color[3]};
     float imageTextureColor[4] = {outFragColor[0], outFragColor[1], outFragColor[2], outFragColor[3]};
     float alpha = bv.color[3];
-    float sampledRoughness = 0.0f, sampledMetallic = 0.0f;
     V3 lightNormal = fnormalize(bv.normal);
     const V3 lightDir = fnormalize(bv.lightDir);
     const V3 bitangent = bv.bitangent;
-    SampleCoords cache;
-    cache.valid = false;
     if (md) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) outFragColor[k] = md->color[k];
 #pragma unroll
         for (int k = 0; k < 4; ++k) imageTextureColor[k] = outFragColor[k];
         alpha = fminf(md->color[3], alpha);
-        if (sd.normal_maps_enabled == 1 && md->tex[1] != RZ_INVALID_INDEX) {
-            float s[4];
-            smp.sample(md->tex[1], md->sampler[1], bv, cache, s);
-            const V3 m{s[0] * 2.0f - 1.0f, s[1] * 2.0f - 1.0f, s[2] * 2.0f - 1.0f};
+        if (has_normal) {
+            const V3 m{normalTexel[0] * 2.0f - 1.0f, normalTexel[1] * 2.0f - 1.0f, normalTexel[2] * 2.0f - 1.0f};
             const V3 n = fnormalize(bv.normal);
             const V3 t = fnormalize(bv.tangent - n * dot(bv.tangent, n));
             const V3 b = fnormalize(cross(bv.normal, bv.tangent) * bv.sigma);
             lightNormal = fnormalize(t * m.x + b * m.y + n * m.z);
         }
-        if (md->tex[0] != RZ_INVALID_INDEX) {
-            smp.sample(md->tex[0], md->sampler[0], bv, cache, imageTextureColor);
+        if (has_color) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) imageTextureColor[k] = colorTexel[k];
             alpha = fminf(imageTextureColor[3], alpha);
         }
-        float s[4];
-        if (md->tex[3] != RZ_INVALID_INDEX) smp.sample(md->tex[3], md->sampler[3], bv, cache, s);
-        else smp.sample(md->tex[2], md->sampler[2], bv, cache, s);
-        sampledRoughness = s[1];
-        sampledMetallic = s[2];
     }
     if (albedo) {
 #pragma unroll
@@ -618,9 +707,7 @@ __device__ bool fragment_main(const ViewRec& VR, const rz_scene_data& sd, const 
         outFragColor[3] = alpha;
     }
     if (kLit || sd.light_enabled > 0) {
-        float shadowFactor = 1.0f;
-        if (kLit || sd.shadows_enabled == 1)
-        {
+        if (!kLit && sd.shadows_enabled == 1) {
             float cc[4];
             const float* map = select_cascade(VR, bv.csm, cc);
             shadowFactor = pcf(map, VR.shadow_w, cc, VR.pcf_mode);
@@ -684,8 +771,10 @@ __device__ __forceinline__ float half_round(float x) { return __half2float(__flo
 
 // Varying record of one (draw, vertex): the vertex-stage outputs the fragment
 // stage reads plus the clip position, 32 floats:
-//   0-2 normal, 3-5 viewDir, 6-8 lightDir, 9-11 tangent, 12 sigma, 13-16 color,
-//   17-18 uv, 19-22 csm.near, 23-25 worldNormal, 26-28 bitangent, 29-31 clip x, y, w.
+//   0-2 normal, 3-5 viewDir, 6-8 lightDir, 9-11 tangent, 12 sigma, 13 color.a,
+//   14-16 color.rgb, 17 csm.near.w (not read), 18-19 uv, 20-22 csm.near.xyz, 23-25 worldNormal,
+//   26-28 bitangent, 29-31 clip x, y, w.
+// The fragment stage interpolates it two floats at a time.
 constexpr int kVaryingF4 = 8;
 
 __device__ __forceinline__ uint32_t find_draw_by_varying(const DrawRec* __restrict__ draws, uint32_t n, uint32_t i) {
@@ -724,9 +813,9 @@ __global__ void __launch_bounds__(256) k_vertex(ShadeParams P, uint32_t first) {
     dst[0] = make_float4(o.normal.x, o.normal.y, o.normal.z, o.viewDir.x);
     dst[1] = make_float4(o.viewDir.y, o.viewDir.z, o.lightDir.x, o.lightDir.y);
     dst[2] = make_float4(o.lightDir.z, o.tangent.x, o.tangent.y, o.tangent.z);
-    dst[3] = make_float4(o.sigma, o.color[0], o.color[1], o.color[2]);
-    dst[4] = make_float4(o.color[3], o.uv[0], o.uv[1], o.csm[0]);
-    dst[5] = make_float4(o.csm[1], o.csm[2], o.csm[3], o.worldNormal.x);
+    dst[3] = make_float4(o.sigma, o.color[3], o.color[0], o.color[1]);
+    dst[4] = make_float4(o.color[2], o.csm[3], o.uv[0], o.uv[1]);
+    dst[5] = make_float4(o.csm[0], o.csm[1], o.csm[2], o.worldNormal.x);
     dst[6] = make_float4(o.worldNormal.y, o.worldNormal.z, o.bitangent.x, o.bitangent.y);
     dst[7] = make_float4(o.bitangent.z, clip.x, clip.y, clip.w);
 }
@@ -751,16 +840,11 @@ void launch_vertex_range(const ShadeParams& p, uint32_t first, cudaStream_t stre
 template <bool kLit = false>
 __device__ bool shade_pixel(const ShadeParams& P, const ViewRec& VR, const rz_scene_data& sd, const Sampler& smp, uint32_t tri,
                             int px, int py, float out[4], float* aux = nullptr, const PixelNdc* pn = nullptr) {
-    uint32_t d;
-    const float4* rec[3];
-    {  // the camera setup recorded the draw and the vertices
-        const uint4 r = __ldg(&P.tri_refs[tri]);
-        d = r.x;
-        rec[0] = P.varyings + (size_t)r.y * kVaryingF4;
-        rec[1] = P.varyings + (size_t)r.z * kVaryingF4;
-        rec[2] = P.varyings + (size_t)r.w * kVaryingF4;
-    }
-    const int32_t material = __ldg(&P.draws[d].material);
+    // the camera setup recorded the material and the vertices
+    const uint4 ref = __ldg(&P.tri_refs[tri]);
+    const float4* const rec[3] = {P.varyings + (size_t)ref.y * kVaryingF4, P.varyings + (size_t)ref.z * kVaryingF4,
+                                  P.varyings + (size_t)ref.w * kVaryingF4};
+    const int32_t material = (int32_t)ref.x;
     const GpuMaterial* md = material >= 0 ? &P.materials[material] : nullptr;
     float4 clip[3];
 #pragma unroll
@@ -791,76 +875,71 @@ __device__ bool shade_pixel(const ShadeParams& P, const ViewRec& VR, const rz_sc
     barycentrics_n(clip[0], clip[1], clip[2], xq1, yq, bqx);
     barycentrics_n(clip[0], clip[1], clip[2], xq, yq1, bqy);
     const bool debug_extra = (!kLit && (sd.fragment_output == 1 || sd.fragment_output == 7)) || aux != nullptr;
+    // what the shadow and the textures need: uv here and at the quad's pixels, csm
     Frag f;
-    float u0[2], ux[2], uy[2];
+    F2 uv{}, uv0{}, uvx{}, uvy{}, csm_xy{};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const float4 a0 = __ldg(rec[k] + 0), a1 = __ldg(rec[k] + 1), a2 = __ldg(rec[k] + 2);
-        const float4 a3 = __ldg(rec[k] + 3), a4 = __ldg(rec[k] + 4), a5 = __ldg(rec[k] + 5);
-        float4 a6 = make_float4(0.f, 0.f, 0.f, 0.f), a7 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (debug_extra) {
-            a6 = __ldg(rec[k] + 6);
-            a7 = __ldg(rec[k] + 7);
-        }
-        const V3 normal{a0.x, a0.y, a0.z}, viewDir{a0.w, a1.x, a1.y}, lightDir{a1.z, a1.w, a2.x};
-        const V3 tangent{a2.y, a2.z, a2.w}, worldNormal{a5.w, a6.x, a6.y}, bitangent{a6.z, a6.w, a7.x};
-        const float sigma = a3.x;
-        const float color[4] = {a3.y, a3.z, a3.w, a4.x};
-        const float uv[2] = {a4.y, a4.z};
-        const float csm[4] = {a4.w, a5.x, a5.y, a5.z};
-        const float w = b[k];
-        if (k == 0) {
-            f.normal = normal * w;
-            f.worldNormal = worldNormal * w;
-            f.viewDir = viewDir * w;
-            f.lightDir = lightDir * w;
-            f.tangent = tangent * w;
-            f.bitangent = bitangent * w;
+        const float4 q5 = __ldg(rec[k] + 5);
+        const F2 tex{__ldg(reinterpret_cast<const ulonglong2*>(rec[k] + 4)).y}, xy = pack2(q5.x, q5.y);
+        const F2 w = both(b[k]), wq = both(bq0[k]), wx = both(bqx[k]), wy = both(bqy[k]);
+        uv = k == 0 ? tex * w : uv + tex * w;
+        uv0 = k == 0 ? tex * wq : uv0 + tex * wq;
+        uvx = k == 0 ? tex * wx : uvx + tex * wx;
+        uvy = k == 0 ? tex * wy : uvy + tex * wy;
+        csm_xy = k == 0 ? xy * w : csm_xy + xy * w;
+        f.csm[2] = k == 0 ? q5.z * b[k] : f.csm[2] + q5.z * b[k];
+    }
+    unpack2(uv, f.uv[0], f.uv[1]);
+    unpack2(uvx - uv0, f.duvdx[0], f.duvdx[1]);
+    unpack2(uvy - uv0, f.duvdy[0], f.duvdy[1]);
+    unpack2(csm_xy, f.csm[0], f.csm[1]);
+    f.csm[3] = 0.0f;  // not read
+    auto late = [&](Frag& v) {
+        F2 acc[8], extra[2];
+        float wnx = 0.0f, bz = 0.0f, c2 = 0.0f;
+        extra[0].v = extra[1].v = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) f.color[i] = color[i] * w;
+        for (int k = 0; k < 3; ++k) {
+            const F2 w = both(b[k]);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                f.uv[i] = uv[i] * w;
-                u0[i] = uv[i] * bq0[0];
-                ux[i] = uv[i] * bqx[0];
-                uy[i] = uv[i] * bqy[0];
+            for (int i = 0; i < 4; ++i) {
+                const ulonglong2 q = __ldg(reinterpret_cast<const ulonglong2*>(rec[k] + i));
+                acc[2 * i] = k == 0 ? F2{q.x} * w : acc[2 * i] + F2{q.x} * w;
+                acc[2 * i + 1] = k == 0 ? F2{q.y} * w : acc[2 * i + 1] + F2{q.y} * w;
             }
-            f.sigma = sigma * w;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) f.csm[i] = csm[i] * w;
-        } else {
-            f.normal = f.normal + normal * w;
-            f.worldNormal = f.worldNormal + worldNormal * w;
-            f.viewDir = f.viewDir + viewDir * w;
-            f.lightDir = f.lightDir + lightDir * w;
-            f.tangent = f.tangent + tangent * w;
-            f.bitangent = f.bitangent + bitangent * w;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) f.color[i] = f.color[i] + color[i] * w;
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                f.uv[i] = f.uv[i] + uv[i] * w;
-                u0[i] = u0[i] + uv[i] * bq0[k];
-                ux[i] = ux[i] + uv[i] * bqx[k];
-                uy[i] = uy[i] + uv[i] * bqy[k];
+            const float blue = __ldg(&rec[k][4].x);
+            c2 = k == 0 ? blue * b[k] : c2 + blue * b[k];
+            if (debug_extra) {
+                const float wx = __ldg(&rec[k][5].w), z = __ldg(&rec[k][7].x);
+                const ulonglong2 q = __ldg(reinterpret_cast<const ulonglong2*>(rec[k] + 6));
+                wnx = k == 0 ? wx * b[k] : wnx + wx * b[k];
+                extra[0] = k == 0 ? F2{q.x} * w : extra[0] + F2{q.x} * w;
+                extra[1] = k == 0 ? F2{q.y} * w : extra[1] + F2{q.y} * w;
+                bz = k == 0 ? z * b[k] : bz + z * b[k];
             }
-            f.sigma = f.sigma + sigma * w;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) f.csm[i] = f.csm[i] + csm[i] * w;
         }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        f.duvdx[i] = ux[i] - u0[i];
-        f.duvdy[i] = uy[i] - u0[i];
-    }
-    if (aux) {
-        const V3 n = fnormalize(f.worldNormal);
-        aux[3] = n.x;
-        aux[4] = n.y;
-        aux[5] = n.z;
-    }
-    return fragment_main<kLit>(VR, sd, md, f, smp, out, aux);
+        unpack2(acc[0], v.normal.x, v.normal.y);
+        unpack2(acc[1], v.normal.z, v.viewDir.x);
+        unpack2(acc[2], v.viewDir.y, v.viewDir.z);
+        unpack2(acc[3], v.lightDir.x, v.lightDir.y);
+        unpack2(acc[4], v.lightDir.z, v.tangent.x);
+        unpack2(acc[5], v.tangent.y, v.tangent.z);
+        unpack2(acc[6], v.sigma, v.color[3]);
+        unpack2(acc[7], v.color[0], v.color[1]);
+        v.color[2] = c2;
+        v.worldNormal.x = wnx;
+        unpack2(extra[0], v.worldNormal.y, v.worldNormal.z);
+        unpack2(extra[1], v.bitangent.x, v.bitangent.y);
+        v.bitangent.z = bz;
+        if (aux) {
+            const V3 n = fnormalize(v.worldNormal);
+            aux[3] = n.x;
+            aux[4] = n.y;
+            aux[5] = n.z;
+        }
+    };
+    return fragment_main<kLit>(VR, sd, md, f, late, smp, out, aux);
 }
 
 // Whether a view renders the default output with the light, its shadow and the
@@ -925,7 +1004,15 @@ __device__ __forceinline__ PixelNdc pixel_ndc(const ShadeParams& P, const ViewRe
     return pn;
 }
 
-__global__ void __launch_bounds__(256, 4) k_shade(ShadeParams P) {
+// Bound by instruction issue and the latency of its dependent reads (visibility,
+// vertex records, texels, shadow map) about alike: 55 % issue active, 5.4 of 11
+// cycles between a warp's instructions on memory. So the fragment stage reads the
+// shadow and the textures while it holds little, interpolates the rest after them
+// (two floats per instruction), and six CTAs of 42 registers hide more latency than
+// four of 64 did when everything was interpolated first (then five were no faster).
+// 1080p scene-scale frame: 166 -> 155 us with the kernel so, 4x MSAA 278 -> 256,
+// 32 views 171 -> 154.
+__global__ void __launch_bounds__(256, 6) k_shade(ShadeParams P) {
     __shared__ float s_srgb[256];
     __shared__ uint32_t s_view;
     {
@@ -1025,7 +1112,7 @@ __device__ __forceinline__ void shade_items(const ShadeParams& P, const ViewRec&
 }
 
 template <bool kAux>  // the views have a G-buffer
-__global__ void __launch_bounds__(256, 4) k_shade_msaa(ShadeParams P) {
+__global__ void __launch_bounds__(256, 5) k_shade_msaa(ShadeParams P) {
     __shared__ float s_srgb[256];
     __shared__ uint32_t s_view;
     __shared__ TileNdc s_ndc;
@@ -1530,7 +1617,7 @@ __device__ __forceinline__ void shade_fragments(const ShadeParams& P, const View
 }
 
 template <bool kMsaa>
-__global__ void __launch_bounds__(256, 4) k_blend(BlendParams B) {
+__global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
     constexpr int kSamples = kMsaa ? kMsaaSamples : 1;
     __shared__ float s_srgb[256];
     __shared__ uint32_t s_groups[256];
