@@ -195,6 +195,10 @@ struct rz_ctx {
     DrawRec* d_shadow_draws = nullptr;
     DrawRec* d_opaque_draws = nullptr;
     DrawRec* d_blended_draws = nullptr;
+    // the draw of every 256th triangle of the shadow, opaque and blended lists, then of every
+    // 256th varying record of the opaque and the blended draws
+    uint32_t* d_draw_tables = nullptr;
+    size_t table_at[5] = {0, 0, 0, 0, 0};
     uint32_t shadow_draw_count = 0, opaque_draw_count = 0, blended_draw_count = 0;
     uint32_t shadow_tris = 0, opaque_tris = 0, blended_tris = 0;
     float* d_shadow_mvp = nullptr;
@@ -749,6 +753,7 @@ int build_layout(rz_ctx* c) {
     dfree(c->d_shadow_draws);
     dfree(c->d_opaque_draws);
     dfree(c->d_blended_draws);
+    dfree(c->d_draw_tables);
     dfree(c->d_shadow_mvp);
     dfree(c->d_camera_consts);
     dfree(c->d_blended_consts);
@@ -782,6 +787,23 @@ int build_layout(rz_ctx* c) {
         RZ_CUDA(c, cudaMemcpy(c->d_opaque_draws, opaque.data(), opaque.size() * sizeof(DrawRec), cudaMemcpyHostToDevice), "upload draws");
     if (!blended.empty())
         RZ_CUDA(c, cudaMemcpy(c->d_blended_draws, blended.data(), blended.size() * sizeof(DrawRec), cudaMemcpyHostToDevice), "upload draws");
+    // entry g: the last draw whose first triangle (or varying record) is at most 256 g
+    std::vector<uint32_t> tables;
+    auto add_table = [&](int which, const std::vector<DrawRec>& list, uint64_t end, uint32_t DrawRec::*base) {
+        c->table_at[which] = tables.size();
+        uint32_t d = 0;
+        for (uint64_t at = 0; at < std::max<uint64_t>(end, 1); at += 256) {
+            while (d + 1 < list.size() && list[d + 1].*base <= at) ++d;
+            tables.push_back(d);
+        }
+    };
+    add_table(0, shadow_list, shadow_tris, &DrawRec::tri_base);
+    add_table(1, opaque, opaque_tris, &DrawRec::tri_base);
+    add_table(2, blended, blended_tris, &DrawRec::tri_base);
+    add_table(3, opaque, blended_varying_base, &DrawRec::varying_base);
+    add_table(4, blended, varyings, &DrawRec::varying_base);
+    RZ_CUDA(c, dalloc(&c->d_draw_tables, tables.size()), "draw tables");
+    RZ_CUDA(c, cudaMemcpy(c->d_draw_tables, tables.data(), tables.size() * 4, cudaMemcpyHostToDevice), "upload draw tables");
     c->shadow_draw_count = (uint32_t)shadow_list.size();
     c->opaque_draw_count = (uint32_t)opaque.size();
     c->blended_draw_count = (uint32_t)blended.size();
@@ -846,6 +868,7 @@ PassParams pass_params(rz_ctx* c, int kind) {
         p.header = &c->d_report->shadow;
         pb = &c->shadow_pass;
     }
+    p.draw_table = c->d_draw_tables + c->table_at[kind == 2 ? 2 : kind];
     p.records = pb->records;
     p.record_capacity = pb->record_capacity;
     p.small_records = pb->small_records;
@@ -866,6 +889,8 @@ ShadeParams shade_params(rz_ctx* c) {
     sh.shade_blocks = c->shade_blocks;
     sh.draws = c->d_opaque_draws;
     sh.draw_count = c->opaque_draw_count;
+    sh.draw_table = c->d_draw_tables + c->table_at[1];
+    sh.varying_table = c->d_draw_tables + c->table_at[3];
     sh.consts = c->d_camera_consts;
     sh.varyings = c->d_varyings;
     sh.varying_count = c->blended_varying_base;  // the opaque draws' records
@@ -1003,6 +1028,8 @@ int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh
         ShadeParams bs = sh;
         bs.draws = c->d_blended_draws;
         bs.draw_count = c->blended_draw_count;
+        bs.draw_table = c->d_draw_tables + c->table_at[2];
+        bs.varying_table = c->d_draw_tables + c->table_at[4];
         bs.consts = c->d_blended_consts;
         bs.varying_count = c->varying_count;
         bs.tri_refs = c->d_tri_refs + c->opaque_tris;
@@ -1389,6 +1416,7 @@ void rz_destroy(rz_ctx* c) {
     dfree(c->d_shadow_draws);
     dfree(c->d_opaque_draws);
     dfree(c->d_blended_draws);
+    dfree(c->d_draw_tables);
     dfree(c->d_shadow_mvp);
     dfree(c->d_camera_consts);
     dfree(c->d_blended_consts);

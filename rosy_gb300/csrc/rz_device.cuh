@@ -47,6 +47,17 @@ __device__ __forceinline__ uint32_t find_draw(const DrawRec* __restrict__ draws,
     return lo;
 }
 
+// The same from a table of the draw that holds triangle 256 g (entry g), built with
+// the draw list: one load and as many steps as draws start between there and `tri`,
+// mostly none, where the search of 1,024 draws is a chain of ten dependent loads.
+__device__ __forceinline__ uint32_t draw_from(const DrawRec* __restrict__ draws, uint32_t n, const uint32_t* __restrict__ table,
+                                              uint32_t tri) {
+    if (!table) return find_draw(draws, n, tri);
+    uint32_t d = __ldg(&table[tri >> 8]);
+    while (d + 1 < n && __ldg(&draws[d + 1].tri_base) <= tri) ++d;
+    return d;
+}
+
 // Thread `tid` of `stride` threads' share of zeroing n bytes at ptr: 16-byte
 // stores on the 16-byte-aligned body, byte stores on the unaligned head and
 // tail, so any start address and size is safe.

@@ -149,6 +149,7 @@ constexpr int kMaxSmallExtent = 16;   // edge values of a lane-rasterised triang
 struct PassParams {
     const DrawRec* draws;
     uint32_t draw_count;
+    const uint32_t* draw_table;  // the draw of every 256th triangle id (draw_from), or null
     uint32_t tri_total;       // triangles to set up: ids tri_offset .. tri_offset + tri_total - 1
     uint32_t tri_offset;
     uint32_t chunk_stamps;    // stamps per raster work chunk (tuning)
@@ -196,6 +197,8 @@ struct ShadeParams {
     uint32_t block_offset;
     const DrawRec* draws;     // opaque list
     uint32_t draw_count;
+    const uint32_t* draw_table;    // the draw of every 256th triangle id (draw_from)
+    const uint32_t* varying_table; // the draw of every 256th varying record
     const DrawConsts* consts; // per opaque draw
     float4* varyings;         // 8 float4 per (draw, mesh vertex), written by k_vertex
     uint32_t varying_count;

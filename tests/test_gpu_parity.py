@@ -272,6 +272,32 @@ def test_msaa_raster_parts(gpu, oracle, chunk_stamps, small_extent, spread):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lengths", [[0, 1, 0, 0, 255, 256, 257, 0], [1] * 300, [511, 1, 0, 512, 2], [769]])
+def test_draw_tables(gpu, oracle, lengths):
+    """Draws of no, one, and about 256 triangles (the step of the draw tables), opaque and blended, of two
+    meshes whose vertices also straddle the step."""
+    tris = sum(lengths)
+    a = sc.random_triangles(seed=59, triangles=2 * tris, width=160, height=96, shadow_size=128, texture_size=32)
+    v, i = 3 * tris, np.arange(3 * tris, dtype=np.uint32)
+    a.meshes = [(0, v, 0, v), (v, v, v, v)]
+    a.indices = np.concatenate([i, i])
+    blended = np.concatenate([a.materials, a.materials])
+    blended["alpha_mode"][1], blended["base_color_factor"][1, 3] = 2, 0.5
+    a.materials = blended
+    surfs = np.zeros(2 * len(lengths), sc.SURFACE_DTYPE)
+    for m in range(2):
+        at = 0
+        for k, n in enumerate(lengths):
+            s = surfs[m * len(lengths) + k]
+            s["mesh_index"], s["start_index"], s["index_count"] = m, 3 * at, 3 * n
+            s["material_index"], s["blended"] = m, m
+            at += n
+    a.surfaces = surfs
+    a.draw_config["shadow_cascades"] = 2
+    check_parity(a, *run(a, oracle))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("chunk_stamps,small_extent", [(8, 1), (16, 4), (33, 2), (64, 1), (256, 16)])
 @pytest.mark.parametrize("spread,fov", [(0.03, 60.0), (0.3, 60.0), (1.0, 60.0), (1.0, 1.5)])
 def test_raster_chunks(gpu, oracle, chunk_stamps, small_extent, spread, fov):
