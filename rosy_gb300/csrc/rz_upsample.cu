@@ -205,6 +205,17 @@ __device__ __forceinline__ void tmem_zero(uint32_t taddr, int cols) {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// Programmatic dependent launch. The kernels of a pass follow each other with the
+// next one's launch allowed once every CTA of this one has started (its CTAs then take
+// the SMs as this one's leave them, and set up barriers, tensor memory and weights),
+// and each waits here for the one before to be complete and its writes visible before
+// it touches what the pass computes. As every kernel does so, a kernel that gets past
+// this point comes after all the earlier ones. A pass's first kernel is launched
+// normally, after all that the stream holds. (957x539 inference, five kernels: 78 -> 64
+// us; a training step of two 960x540 frames: 555 -> 494.)
+__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __host__ __device__ constexpr uint32_t tmem_cols_for(int cols) {
     return cols <= 32 ? 32u : cols <= 64 ? 64u : cols <= 128 ? 128u : cols <= 256 ? 256u : 512u;
 }
@@ -246,6 +257,7 @@ __device__ __forceinline__ float matched_weight(uint32_t m4) {
 }
 
 __global__ void k_features(rz_gbuffer g, __nv_bfloat16* __restrict__ feat) {
+    pdl_allow_next();
     const int n = (int)(g.width * g.height);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -499,6 +511,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
     const int ntiles = tiles_x * ((a.H + kTileRows - 1) / kTileRows);
     const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
+    pdl_allow_next();
     __shared__ float s_bias[N];
     __shared__ float s_srcw[16][4];  // final layer: the x2 base's source weights for each source mask
     if (warp == 0) tmem_alloc(tmem_slot, L::TMEM_COLS);
@@ -531,16 +544,19 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
             for (int tt = 0; tt < kTileRows * 4 / kConvEpilogueWarps; ++tt)
                 tmem_zero(tmem + ((uint32_t)(quad * 32) << 16) + b * L::ACC_COLS + (kTileRows + 1 - (row0 + tt)) * N, N);
     }
+    if (warp == kConvEpilogueWarps && lane == 0) {  // the weights (of an earlier pass or call): one bulk copy
+        mbar_expect_tx(wbar, L::B_BYTES);
+        bulk_load(sB, a.wimg, L::B_BYTES, wbar);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait_previous();
     bool ok = true;
     float loss = 0.0f;
 
     if (warp == kConvEpilogueWarps && lane == 0) {
-        // producer: the weights once (one bulk copy), then the TMA loads of each tile's halo
-        mbar_expect_tx(wbar, L::B_BYTES);
-        bulk_load(sB, a.wimg, L::B_BYTES, wbar);
+        // producer: the TMA loads of each tile's halo
         int issued = 0;
         for (int j = 0; j < my_tiles && ok; ++j) {
             const int buf = j % NS;
@@ -733,6 +749,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __gr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_allow_next();
+    pdl_wait_previous();
     bool ok = true;
     if (warp == 0 && lane == 0) {
         int issued = 0;
@@ -1067,14 +1085,29 @@ bool encode_planar(CUtensorMap* map, const void* base, int C, int W, int H, int 
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Launches a kernel of a pass after the one before it on the stream (pdl_wait_previous).
+template <class... P, class... A>
+bool launch_next(void (*kernel)(P...), int grid, int threads, uint32_t smem, cudaStream_t s, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+
 template <int CIN, int N, int EPI>
 bool launch_conv(const rz_upsampler* u, const ConvArgs& a, cudaStream_t s) {
     CUtensorMap map;
     if (!encode_planar(&map, a.in, CIN, a.W, a.H)) return false;
     const int tiles = ((a.W + kTileOut - 1) / kTileOut) * ((a.H + kTileRows - 1) / kTileRows);
     const int grid = std::min(tiles, std::max(u->sms, 1));
-    k_conv<CIN, N, EPI><<<grid, kConvThreads, ConvSmem<CIN, N>::BYTES, s>>>(a, map);
-    return true;
+    return launch_next(k_conv<CIN, N, EPI>, grid, kConvThreads, ConvSmem<CIN, N>::BYTES, s, a, map);
 }
 
 template <int CIN, int N>
@@ -1083,8 +1116,7 @@ bool launch_wgrad(const rz_upsampler* u, const WgradArgs& a, const __nv_bfloat16
     if (!encode_planar(&x_map, x, CIN, a.W, a.H) || !encode_planar(&dy_map, dy, N, a.W, a.H, kWgKP)) return false;
     const int tiles = ((a.W + kWgKP - 1) / kWgKP) * ((a.H + kWgRows - 1) / kWgRows);
     const int grid = std::min(tiles, std::max(u->sms, 1));
-    k_wgrad<CIN, N><<<grid, kWgThreads, WgSmem<CIN, N>::BYTES, s>>>(a, x_map, dy_map);
-    return true;
+    return launch_next(k_wgrad<CIN, N>, grid, kWgThreads, WgSmem<CIN, N>::BYTES, s, a, x_map, dy_map);
 }
 
 bool gbuffer_ok(const rz_upsampler* u, const rz_gbuffer* g) {

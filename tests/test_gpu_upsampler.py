@@ -277,29 +277,87 @@ def test_upsampler_gradients_match_oracle(gpu, w, h):
     hi.deinit()
 
 
-@pytest.mark.parametrize("w,h", [(1, 1), (3, 5), (16, 4), (111, 3), (112, 4), (113, 5), (126, 9), (225, 8), (1230, 61)])
-def test_weight_gradient_tiles(gpu, w, h):
-    """Every layer's weight and bias gradients at the edges of the 112 x 4 tiles (and, at 1230 x 61, with more
-    tiles than SMs) against the oracle's float64 sums. The operands are the same bf16 values up to roundings of
-    fp32 against float64 sums that fall on the other side of a bf16 step (2^-8 of a value, a few in a thousand),
-    so 1e-3 of a layer's norm holds for sums of them; fp32 accumulation adds below 1e-5."""
+def _random_gbuffer(w, h, seed):
+    """Random G-buffer and target: host arrays, the target, the device record, the device target, what to keep alive."""
     import torch
 
     from rosy_gb300 import _abi
 
-    rng = np.random.default_rng(100 * w + h)
+    rng = np.random.default_rng(seed)
     gb = {"color": rng.integers(0, 256, (h, w, 4), np.uint8), "albedo": rng.integers(0, 256, (h, w, 4), np.uint8),
           "depth": (0.3 * rng.random((h, w))).astype(np.float32), "normal": (rng.random((h, w, 2)) - 0.5).astype(np.float16),
           "sources": rng.integers(0, 65536, (h, w), np.uint16)}
     target = rng.integers(0, 256, (2 * h, 2 * w, 4), np.uint8)
-    p = _params(5)
-    ref, _ = U.gradients(p, gb, target)
     dev = {k: torch.from_numpy(v.view(np.int16) if k == "sources" else v).cuda() for k, v in gb.items()}
     tgt = torch.from_numpy(target).cuda()
     torch.cuda.synchronize()
     g = _abi.RzGbuffer(color_rgba8=dev["color"].data_ptr(), depth_f32=dev["depth"].data_ptr(),
                        albedo_rgba8=dev["albedo"].data_ptr(), normal_oct_f16x2=dev["normal"].data_ptr(),
                        sources_u16=dev["sources"].data_ptr(), width=w, height=h)
+    return gb, target, g, tgt, dev
+
+
+@pytest.mark.parametrize("w,h", [(40, 24), (640, 360)])
+def test_passes_back_to_back_and_captured(gpu, w, h):
+    """Inference, training and inference again with nothing between them, on a stream of their own and
+    replayed from a CUDA graph: the kernels of a pass overlap at their ends, the passes' results do not."""
+    import torch
+
+    inputs = [_random_gbuffer(w, h, 7 + i) for i in range(3)]
+    p = _params(6)
+    u = up.Upsampler(0, w, h)
+    u.set_params(p)
+    outs = [torch.zeros((2 * h, 2 * w), dtype=torch.int32, device="cuda") for _ in range(3)]
+    alone = []
+    for x, o in zip(inputs, outs):
+        u.infer(x[2], o.data_ptr())
+        torch.cuda.synchronize()
+        alone.append(o.clone())
+    u.accumulate(inputs[1][2], inputs[1][3].data_ptr())
+    grads, loss, _ = u.grads()
+    u.set_params(p)
+    u.adam_step(0.0)  # the gradients and the loss back to zero
+    stream = torch.cuda.Stream()
+
+    def passes(s):
+        for x, o in zip(inputs, outs):
+            u.infer(x[2], o.data_ptr(), s)
+        u.accumulate(inputs[1][2], inputs[1][3].data_ptr(), None, s)
+        u.infer(inputs[0][2], outs[0].data_ptr(), s)
+
+    def check(times):
+        for a, o in zip(alone, outs):
+            assert torch.equal(a, o)
+            o.zero_()
+        torch.cuda.synchronize()
+        g, l, _ = u.grads()
+        assert np.allclose(g, times * grads, rtol=1e-4, atol=1e-4 * np.abs(times * grads).max())  # atomics' order, sums of sums
+        assert abs(l - times * loss) <= 1e-5 * times * loss
+
+    torch.cuda.synchronize()
+    passes(stream.cuda_stream)
+    stream.synchronize()
+    check(1)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        passes(stream.cuda_stream)
+    graph.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    check(3)
+    assert u.status() == 0
+    u.close()
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (3, 5), (16, 4), (111, 3), (112, 4), (113, 5), (126, 9), (225, 8), (1230, 61)])
+def test_weight_gradient_tiles(gpu, w, h):
+    """Every layer's weight and bias gradients at the edges of the 112 x 4 tiles (and, at 1230 x 61, with more
+    tiles than SMs) against the oracle's float64 sums. The operands are the same bf16 values up to roundings of
+    fp32 against float64 sums that fall on the other side of a bf16 step (2^-8 of a value, a few in a thousand),
+    so 1e-3 of a layer's norm holds for sums of them; fp32 accumulation adds below 1e-5."""
+    gb, target, g, tgt, keep = _random_gbuffer(w, h, 100 * w + h)
+    p = _params(5)
+    ref, _ = U.gradients(p, gb, target)
     u = up.Upsampler(0, w, h)
     u.set_params(p)
     u.accumulate(g, tgt.data_ptr())
