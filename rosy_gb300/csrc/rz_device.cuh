@@ -80,4 +80,38 @@ __device__ __forceinline__ void clear_share(const ClearList& L) {
     for (int b = 0; b < L.count; ++b) zero_share(L.ptr[b], L.bytes[b], tid, stride);
 }
 
+// Two floats in a register pair, and the packed operations on them: each half rounds
+// as the scalar operation does, in one instruction instead of two (kernels that are
+// short of issue slots, not of multipliers).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 both(float x) { return pack2(x, x); }
+__device__ __forceinline__ void unpack2(F2 p, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// The products: a * b - 0, whose sums round like a * b. The assembler contracts a packed
+// multiply and the add after it into one multiply-add (whatever -fmad says, and with a
+// literal -0 too), which rounds once; it does not know this value.
+static __constant__ unsigned long long c_minus_zeros = 0x8000000080000000ull;
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return fma2(a, b, F2{c_minus_zeros}); }
+
 }  // namespace rz

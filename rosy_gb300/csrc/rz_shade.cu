@@ -56,39 +56,6 @@ __device__ __forceinline__ V3 mulm3v(const float* N, V3 v) {
     return {N[0] * v.x + N[3] * v.y + N[6] * v.z, N[1] * v.x + N[4] * v.y + N[7] * v.z, N[2] * v.x + N[5] * v.y + N[8] * v.z};
 }
 
-// Two floats in a register pair, and the packed operations on them: each half rounds
-// as the scalar operation does, in one instruction instead of two (the fragment stage
-// is short of issue slots, not of multipliers).
-struct F2 {
-    unsigned long long v;
-};
-__device__ __forceinline__ F2 pack2(float lo, float hi) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ F2 both(float x) { return pack2(x, x); }
-__device__ __forceinline__ void unpack2(F2 p, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v)); }
-__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
-    F2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
-    F2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-// The products: a * b - 0, whose sums round like a * b. The assembler contracts a packed
-// multiply and the add after it into one multiply-add (whatever -fmad says, and with a
-// literal -0 too), which rounds once; it does not know this value.
-__constant__ unsigned long long c_minus_zeros = 0x8000000080000000ull;
-__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return fma2(a, b, F2{c_minus_zeros}); }
 __device__ __forceinline__ F2 mix2(F2 x, F2 y, F2 w) { return x + w * (y - x); }
 
 // ---------------------------------------------------------------------------

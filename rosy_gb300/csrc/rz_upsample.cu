@@ -47,14 +47,18 @@
 #include <string>
 #include <vector>
 
-#include "rz_internal.h"
+#include "rz_device.cuh"
 
 namespace rz {
 namespace up {
 
 constexpr int kThreads = 128;      // self-test kernel
-constexpr int kConvEpilogueWarps = 16;  // convolution: one epilogue warp per (TMEM lane quadrant, tile row),
-constexpr int kConvThreads = 32 * (kConvEpilogueWarps + 2);  // then a TMA warp and an MMA warp
+// convolution: two groups of epilogue warps, which take tiles in turn (a group's loads
+// and stores wait while the other computes), a warp of a group per TMEM lane quadrant
+// and half of the tile's rows; then a TMA warp and an MMA warp
+constexpr int kConvGroupWarps = 8;
+constexpr int kConvEpilogueWarps = 2 * kConvGroupWarps;
+constexpr int kConvThreads = 32 * (kConvEpilogueWarps + 2);
 constexpr int kTileW = 128;  // conv: MMA rows (M = 128), one row segment of output pixels
 constexpr int kTileRows = 4; // conv: output rows per tile (8 measured 4% slower)
 constexpr int kConvStages = 4; // conv: halo buffers in flight (TMA loads ahead of the MMAs)
@@ -235,14 +239,12 @@ __device__ __forceinline__ size_t act_index(int W, int H, int x, int y, int c) {
 
 // ---- features -----------------------------------------------------------------
 
-// One pixel's 16 input channels from the G-buffer (see rz_upsampler_* in the header).
-// byte / 255, correctly rounded: the product with the rounded reciprocal and one
-// residual-correction step (Markstein's method), which gives the correctly rounded
-// quotient for every byte value (checked exhaustively against IEEE division).
+// byte / 255, correctly rounded: the reciprocal as two floats, the small part's product
+// in the addend of the large one's (checked exhaustively against IEEE division).
 __device__ __forceinline__ float unorm8(uint32_t b) {
     const float x = (float)b, r = 1.0f / 255.0f;
-    const float q = x * r;
-    return __fmaf_rn(__fmaf_rn(-q, 255.0f, x), r, q);
+    const float rest = (float)(1.0 / 255.0 - (double)r);
+    return __fmaf_rn(x, r, x * rest);
 }
 
 // Sum of the bilinear x2 weights of a sample point's marked sources: own pixel
@@ -256,6 +258,7 @@ __device__ __forceinline__ float matched_weight(uint32_t m4) {
     return ws;
 }
 
+// One pixel's 16 input channels from the G-buffer (see rz_upsampler_* in the header).
 __global__ void k_features(rz_gbuffer g, __nv_bfloat16* __restrict__ feat) {
     pdl_allow_next();
     const int n = (int)(g.width * g.height);
@@ -310,8 +313,15 @@ struct ConvArgs {
     long long wait_cycles;          // bound of each pipeline wait
 };
 
+// The low-resolution colours around a tile of the final layer as byte / 255, a plane
+// per channel: rows y0 - 1 .. y0 + kTileRows, columns x0 - 1 .. x0 + kHaloW - 2, clamped
+// to the image.
+struct TileRgb {
+    float v[3][kTileRows + 2][kHaloW];
+};
+
 // Shared memory of the persistent convolution: the weights (B operand) once,
-// then kConvStages halo buffers (A operand) that tiles take in turn. Each halo
+// then NS halo buffers (A operand) that tiles take in turn. Each halo
 // buffer is (kTileRows + 2) rows x (CIN / 8) channel planes x kHaloW pixels x 16
 // bytes; a plane is padded by two pixels (read by the dropped MMA rows, never
 // written) and to a multiple of 128 bytes.
@@ -325,21 +335,27 @@ struct ConvSmem {
     static constexpr uint32_t B_BYTES = 9 * CIN * N * 2;
     static constexpr uint32_t A_OFF0 = (B_BYTES + 1023) / 1024 * 1024;
     static constexpr uint32_t A_STRIDE = (A_BYTES + 1023) / 1024 * 1024;  // between halo buffers
-    static constexpr uint32_t BAR_OFF = A_OFF0 + kConvStages * A_STRIDE;
-    static constexpr uint32_t NBAR = 2 * kConvStages + 5;                // full, empty, tfull[2], tempty[2], weights
+    // the final layer (16 outputs) gives one halo buffer's room to four tiles of colours (k_conv)
+    static constexpr int NS = N == 16 ? kConvStages - 1 : kConvStages;
+    static constexpr uint32_t RGB_OFF = A_OFF0 + NS * A_STRIDE;
+    static constexpr uint32_t RGB_BYTES = N == 16 ? 4 * sizeof(TileRgb) : 0;  // two per epilogue group
+    static constexpr uint32_t BAR_OFF = (RGB_OFF + RGB_BYTES + 15) / 16 * 16;
+    static constexpr uint32_t NBAR = 2 * NS + 5;                          // full, empty, tfull[2], tempty[2], weights
     static constexpr uint32_t BYTES = BAR_OFF + NBAR * 8 + 16;           // the barriers, the TMEM address
     static constexpr uint32_t ACC_COLS = (kTileRows + 4) * N;                 // one accumulator buffer
     static constexpr uint32_t TMEM_COLS = tmem_cols_for(2 * ACC_COLS);        // two of them
 };
 static_assert(ConvSmem<32, 32>::BYTES + 2048 <= 227 * 1024, "conv shared memory (with the static arrays)");
 static_assert(2 * (kTileRows + 4) * 32 <= 512, "two accumulator buffers fit the 512 TMEM columns");
-static_assert(kTileRows * 4 % kConvEpilogueWarps == 0, "epilogue warps split the tile rows evenly");
+constexpr int kWarpRows = kTileRows * 4 / kConvGroupWarps;  // tile rows of an epilogue warp
+static_assert(kWarpRows * kConvGroupWarps == kTileRows * 4, "a group's warps split the tile rows evenly");
 static_assert(2 * kHaloW <= 256, "a halo row is one TMA box (at most 256 elements)");
 static_assert(ConvSmem<32, 32>::S_G % 128 == 0 && ConvSmem<16, 32>::S_R % 128 == 0, "TMA destinations 128-byte aligned");
 
 template <int N, int EPI>
 __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float* acc, int x, int y, float& loss,
-                                              const float* bias, int xl, const float (*srcw)[4]) {
+                                              const float* bias, const float4* srcw, const TileRgb* rgb, int row, int col,
+                                              uint32_t srcmask) {
     const bool inside = x < a.W && y < a.H;
     if (EPI == kEpiRelu) {
         if (!inside) return;
@@ -366,38 +382,11 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float* ac
             *reinterpret_cast<uint4*>(a.out + act_index(a.W, a.H, x, y, 8 * q)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
     } else {  // final: pixel shuffle + x2 base (+ loss gradient)
-        const int W = a.W, H = a.H;
-        // The 3x3 neighbourhood of low-resolution colours (edges clamped), as byte / 255.
-        // The warp's lanes hold consecutive columns xl (the tile's dropped MMA rows
-        // included, clamped), so each lane loads and converts its own column of the
-        // three rows and takes its left and right neighbours' from the adjacent lanes;
-        // lanes 0 and 31 load the column past the warp's edge. Every lane takes part
-        // (the shuffles), then lanes outside the image return.
-        const int lane = threadIdx.x & 31;
-        const int xo = min(max(xl, 0), W - 1);
-        const int xe = min(max(lane == 0 ? xl - 1 : xl + 1, 0), W - 1);
-        const bool edge_lane = lane == 0 || lane == 31;
-        float f[3][3][3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            const int yy = min(max(y + r - 1, 0), H - 1);
-            const uint32_t c = __ldg(a.color_lr + (size_t)yy * W + xo);
-            const uint32_t ce = edge_lane ? __ldg(a.color_lr + (size_t)yy * W + xe) : 0u;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float own = unorm8((c >> (8 * k)) & 255u);
-                const float ext = edge_lane ? unorm8((ce >> (8 * k)) & 255u) : 0.0f;
-                const float lv = __shfl_up_sync(0xFFFFFFFFu, own, 1), rv = __shfl_down_sync(0xFFFFFFFFu, own, 1);
-                f[r][0][k] = lane == 0 ? ext : lv;
-                f[r][1][k] = own;
-                f[r][2][k] = lane == 31 ? ext : rv;
-            }
-        }
         if (!inside) return;
+        const int W = a.W, H = a.H;
         float net[kOutChannels];
 #pragma unroll
         for (int c = 0; c < kOutChannels; ++c) net[c] = acc[c] + bias[c];
-        const uint32_t srcmask = a.sources ? (uint32_t)__ldg(a.sources + (size_t)y * W + x) : 0xFFFFu;
         float g[kOutChannels];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -405,32 +394,41 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float* ac
             const size_t op = (size_t)(2 * y + i) * (2 * W) + 2 * x;
             uint2 t = make_uint2(0u, 0u);
             if (a.target) t = __ldg(reinterpret_cast<const uint2*>(a.target + op));
-            uint32_t o[2];
+            // the two points of this half, in the halves of register pairs: the weights of a point's
+            // sources (own, horizontal, vertical, diagonal) for its source mask are bilinear,
+            // renormalised over the sources that show its triangle
+            const float4 wl = srcw[(srcmask >> (8 * i)) & 15u], wr = srcw[(srcmask >> (8 * i + 4)) & 15u];
+            const F2 w0 = pack2(wl.x, wr.x), w1 = pack2(wl.y, wr.y), w2 = pack2(wl.z, wr.z), w3 = pack2(wl.w, wr.w);
+            float q[2][3];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int qs = j == 0 ? 0 : 2;
-                const uint32_t tj = j == 0 ? t.x : t.y;
-                uint32_t ov = 255u << 24;
-                // the weights of this point's sources (own, horizontal, vertical, diagonal) for
-                // its source mask: bilinear renormalised over the sources that show its triangle
-                const uint32_t m4 = (srcmask >> (4 * (2 * i + j))) & 15u;
-                const float w0 = srcw[m4][0], w1 = srcw[m4][1], w2 = srcw[m4][2], w3 = srcw[m4][3];
+            for (int k = 0; k < 3; ++k) {
+                const float(*f)[kHaloW] = &rgb->v[k][row];  // rows row .. row + 2, columns col .. col + 2
+                F2 base = w0 * both(f[1][col + 1]);
+                base = base + w1 * pack2(f[1][col], f[1][col + 2]);
+                base = base + w2 * both(f[rs][col + 1]);
+                base = base + w3 * pack2(f[rs][col], f[rs][col + 2]);
+                float b[2];
+                unpack2(base, b[0], b[1]);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    float base = w0 * f[1][1][k];
-                    base = base + w1 * f[1][qs][k];
-                    base = base + w2 * f[rs][1][k];
-                    base = base + w3 * f[rs][qs][k];
-                    const float v = base + net[(2 * i + j) * 3 + k];
-                    const float qv = fminf(fmaxf(v, 0.0f), 1.0f);
-                    ov |= (uint32_t)floorf(qv * 255.0f + 0.5f) << (8 * k);
+                for (int j = 0; j < 2; ++j) {
+                    const int c = (2 * i + j) * 3 + k;
+                    q[j][k] = __saturatef(b[j] + net[c]);
                     if (a.target) {
-                        const float d = v - unorm8((tj >> (8 * k)) & 255u);
-                        g[(2 * i + j) * 3 + k] = 2.0f * d;
+                        const uint32_t tj = j == 0 ? t.x : t.y;
+                        const float d = (b[j] + net[c]) - unorm8((tj >> (8 * k)) & 255u);
+                        g[c] = 2.0f * d;
                         loss += d * d;
                     }
                 }
-                o[j] = ov;
+            }
+            uint32_t o[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                uint32_t e[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k)  // floor(q * 255 + 0.5): the low byte of the sum with 2^23, rounded down
+                    e[k] = __float_as_uint(__fadd_rd(q[j][k] * 255.0f + 0.5f, 8388608.0f));
+                o[j] = __byte_perm(__byte_perm(e[0], e[1], 0x0040), e[2], 0x0410) | 0xFF000000u;
             }
             if (a.out_rgba8) *reinterpret_cast<uint2*>(a.out_rgba8 + op) = make_uint2(o[0], o[1]);
         }
@@ -471,18 +469,19 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 
 // Persistent, warp-specialised convolution. CTA b takes tiles b, b + grid, ...
-// (128 pixels x kTileRows rows each) through a ring of kConvStages halo buffers
+// (128 pixels x kTileRows rows each) through a ring of NS halo buffers
 // and two TMEM accumulators:
-//   warp 16 (one thread) TMA-loads tile j's halo into halo buffer j % kConvStages
-//                        once the MMAs of tile j - kConvStages have released it
+//   warp 16 (one thread) TMA-loads tile j's halo into halo buffer j % NS
+//                        once the MMAs of tile j - NS have released it
 //                        (barrier `empty`);
 //   warp 17 (one thread) waits for the halo (`full`) and for the epilogue of
 //                        tile j - 2 to have drained accumulator buffer j % 2
 //                        (`tempty`), issues the tile's tcgen05.mma and commits to
 //                        `empty` and `tfull`;
-//   warps 0-15           wait for `tfull`, read the accumulator (warp w reads
-//                        TMEM lane quadrant w % 4 of tile row w / 4), zero it,
-//                        run the epilogue and arrive on `tempty`.
+//   warps 0-15           two groups of eight, group g for the tiles of accumulator
+//                        g: wait for `tfull`, read the accumulator (warp w reads
+//                        TMEM lane quadrant w % 4 of two tile rows), zero it,
+//                        arrive on `tempty` and run the epilogue.
 // One MMA takes one halo row i, one horizontal tap dx and 16 input channels, and
 // N = 3 x Cout weight columns: the three vertical taps at once. Its three column
 // blocks add halo row i's contributions to output rows i, i - 1 and i - 2, so the
@@ -494,12 +493,16 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // read from shared memory thus feeds 96 weight columns instead of 32.
 // Every wait is bounded; a role whose wait runs out sets kErrMmaTimeout and
 // stops, and the others then run out in turn.
+// Bound by the operand reads of the MMAs (ReLU layers, tensor pipe 48 %) and by the
+// chain of a tile's epilogue (final layer: colours, accumulator, sources, stores), of
+// which two overlap: 957x539 inference 64 us with one group of 16 warps, 59 with two,
+// the final layer's share 22 -> 19 us.
 template <int CIN, int N, int EPI>
 __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __grid_constant__ CUtensorMap in_map) {
     using L = ConvSmem<CIN, N>;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* sB = smem;
-    constexpr int NS = kConvStages;
+    constexpr int NS = L::NS;
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);  // [NS]
     uint64_t* empty = full + NS;                                       // [NS]
     uint64_t* tfull = full + 2 * NS;                                   // [2]
@@ -513,7 +516,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
 
     pdl_allow_next();
     __shared__ float s_bias[N];
-    __shared__ float s_srcw[16][4];  // final layer: the x2 base's source weights for each source mask
+    __shared__ float4 s_srcw[16];  // final layer: the x2 base's source weights for each source mask
     if (warp == 0) tmem_alloc(tmem_slot, L::TMEM_COLS);
     if (tid == 0) {
         for (int b = 0; b < NS; ++b) {
@@ -522,7 +525,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], kConvEpilogueWarps);
+            mbar_init(&tempty[b], kConvGroupWarps);
         }
         mbar_init(wbar, 1);
     }
@@ -532,17 +535,16 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
         // no bit set is plain bilinear (as is every bit set: the sum is 1)
         const uint32_t m = (uint32_t)tid >> 2, s = (uint32_t)tid & 3u;
         const float w = s == 0 ? 0.5625f : (s == 3 ? 0.0625f : 0.1875f);
-        s_srcw[m][s] = m == 0u ? w : (((m >> s) & 1u) ? w * (1.0f / matched_weight(m)) : 0.0f);
+        reinterpret_cast<float*>(s_srcw)[4 * m + s] = m == 0u ? w : (((m >> s) & 1u) ? w * (1.0f / matched_weight(m)) : 0.0f);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    if (warp < kConvEpilogueWarps) {  // the read accumulator rows of both buffers start at zero
-        const int quad = warp & 3, row0 = (warp >> 2) * (kTileRows * 4 / kConvEpilogueWarps);
-        for (int b = 0; b < 2; ++b)
-            for (int tt = 0; tt < kTileRows * 4 / kConvEpilogueWarps; ++tt)
-                tmem_zero(tmem + ((uint32_t)(quad * 32) << 16) + b * L::ACC_COLS + (kTileRows + 1 - (row0 + tt)) * N, N);
+    const int group = warp / kConvGroupWarps, quad = warp & 3, row0 = (warp % kConvGroupWarps >> 2) * kWarpRows;
+    if (warp < kConvEpilogueWarps) {  // the read accumulator rows of both buffers (group g drains buffer g) start at zero
+        for (int tt = 0; tt < kWarpRows; ++tt)
+            tmem_zero(tmem + ((uint32_t)(quad * 32) << 16) + group * L::ACC_COLS + (kTileRows + 1 - (row0 + tt)) * N, N);
     }
     if (warp == kConvEpilogueWarps && lane == 0) {  // the weights (of an earlier pass or call): one bulk copy
         mbar_expect_tx(wbar, L::B_BYTES);
@@ -619,36 +621,58 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
         if (committed > 0 && !mbar_wait(&empty[(committed - 1) % NS], (uint32_t)((committed - 1) / NS) & 1u))
             ok = false;
     } else if (warp < kConvEpilogueWarps) {
-        const int quad = warp & 3, row0 = (warp >> 2) * (kTileRows * 4 / kConvEpilogueWarps);
         // the biases live in registers: shared-memory reads would queue behind the MMAs' operand traffic
         float bias[N];
 #pragma unroll
         for (int c = 0; c < N; ++c) bias[c] = s_bias[c];
-        for (int j = 0; j < my_tiles; ++j) {
-            const int buf = j & 1;
-            // one decision per warp: the epilogue's TMEM loads and shuffles are warp-wide
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&tfull[buf], (uint32_t)(j >> 1) & 1u, a.wait_cycles))) {
-                ok = false;
+        const int col = quad * 32 + lane;
+        for (int j = group; j < my_tiles; j += 2) {
+            const int tile = blockIdx.x + j * gridDim.x;
+            const int x0 = (tile % tiles_x) * kTileOut, y0 = (tile / tiles_x) * kTileRows;
+            const int x = col < kTileOut ? x0 + col : a.W;  // the dropped MMA rows count as outside the image
+            TileRgb* const rgb = reinterpret_cast<TileRgb*>(smem + L::RGB_OFF) + 2 * group + ((j >> 1) & 1);
+            uint32_t srcmask[kWarpRows] = {};
+            if constexpr (EPI == kEpiFinal) {
+                // while the MMAs run: the tile's colours, converted once instead of by the nine pixels
+                // around each. Past the barrier of the group's last tile every warp of it is done with the
+                // one before, whose buffer this is. All the group's warps come to every tile's barrier, also
+                // after a wait has run out.
+                for (int p = tid % (32 * kConvGroupWarps); p < (kTileRows + 2) * kHaloW; p += 32 * kConvGroupWarps) {
+                    const int r = p / kHaloW, c = p % kHaloW;
+                    const int yy = min(max(y0 + r - 1, 0), a.H - 1), xx = min(max(x0 + c - 1, 0), a.W - 1);
+                    const uint32_t v = __ldg(a.color_lr + (size_t)yy * a.W + xx);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) rgb->v[k][r][c] = unorm8((v >> (8 * k)) & 255u);
+                }
+#pragma unroll
+                for (int tt = 0; tt < kWarpRows; ++tt) {
+                    const int y = y0 + row0 + tt;
+                    srcmask[tt] = a.sources && x < a.W && y < a.H ? (uint32_t)__ldg(a.sources + (size_t)y * a.W + x) : 0xFFFFu;
+                }
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * kConvGroupWarps) : "memory");
+            }
+            // one decision per warp: the epilogue's TMEM loads are warp-wide
+            ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(&tfull[group], (uint32_t)(j >> 1) & 1u, a.wait_cycles));
+            if (!ok) {
+                if (EPI == kEpiFinal) continue;
                 break;
             }
             tc_fence_after();
-            const int tile = blockIdx.x + j * gridDim.x;
-            const int x0 = (tile % tiles_x) * kTileOut, y0 = (tile / tiles_x) * kTileRows;
-            const int col = quad * 32 + lane;
-            const int x = col < kTileOut ? x0 + col : a.W;  // the dropped MMA rows count as outside the image
 #pragma unroll
-            for (int tt = 0; tt < kTileRows * 4 / kConvEpilogueWarps; ++tt) {
+            for (int tt = 0; tt < kWarpRows; ++tt) {
                 const int t = row0 + tt;
                 float acc[N];
-                const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + buf * L::ACC_COLS + (kTileRows + 1 - t) * N;
+                const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + group * L::ACC_COLS + (kTileRows + 1 - t) * N;
                 if constexpr (N == 32) tmem_ld32(ta, acc);
                 else tmem_ld16(ta, acc);
                 tmem_zero(ta, N);
-                conv_epilogue<N, EPI>(a, acc, x, y0 + t, loss, bias, x0 + col, s_srcw);
+                if (tt == kWarpRows - 1) {  // the accumulator is free for the tile after next
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[group]);
+                }
+                conv_epilogue<N, EPI>(a, acc, x, y0 + t, loss, bias, s_srcw, rgb, t, col, srcmask[tt]);
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[buf]);
         }
     }
     if (!ok) atomicOr(a.err, kErrMmaTimeout);
