@@ -700,8 +700,9 @@ struct WgradArgs {
 // Shared memory of the weight gradient: a ring of stages, each with a tile's X halo
 // ([row][8-channel group][pixel], kWgRows + 2 rows of kHaloW pixels) and its dY rows
 // ([row][8-channel group][pixel], kWgKP pixels). An M block is 16 consecutive
-// (row, group) planes from output row r on: the three vertical taps' channels, then
-// planes of further rows (or of the dY that follows), whose products are not read.
+// (row, group) planes of X from output row r on, an N block the (row, group) planes of
+// RB output rows from r on: X row a against dY row b is the vertical tap a - b, where
+// that is 0, 1 or 2 (the other products are not read; an M block may run on into the dY).
 template <int CIN, int N>
 struct WgSmem {
     static constexpr int G = CIN / 8;
@@ -709,7 +710,10 @@ struct WgSmem {
     static constexpr uint32_t S_G = kHaloW * 16;              // between channel planes of X (M direction)
     static constexpr uint32_t S_ROW = G * S_G;                // between halo rows
     static constexpr uint32_t X_BYTES = (kWgRows + 2) * S_ROW;
-    static constexpr uint32_t X_READ = (kWgRows - 1) * S_ROW + 16 * S_G;  // end of the furthest M block
+    static constexpr int MR = 16 / G;                         // X rows of an M block
+    static constexpr int RB = MR - 2 < kWgRows ? MR - 2 : kWgRows;  // output rows of an MMA: 2 (32 channels) or 4 (16)
+    static constexpr int NB = RB * N;                         // N of an MMA
+    static constexpr uint32_t X_READ = (kWgRows - RB) * S_ROW + 16 * S_G;  // end of the furthest M block
     static constexpr uint32_t S_COG = kWgKP * 16;             // between channel planes of dY (N direction)
     static constexpr uint32_t S_DYROW = GN * S_COG;
     static constexpr uint32_t DY_OFF = X_BYTES;
@@ -720,7 +724,9 @@ struct WgSmem {
     static constexpr uint32_t BAR_OFF = NS * STAGE;
     static constexpr uint32_t NBAR = 2 * NS + 1;              // full, empty, done
     static constexpr uint32_t BYTES = BAR_OFF + NBAR * 8 + 16;
-    static constexpr uint32_t TMEM_COLS = tmem_cols_for(kWgRows * 3 * N);  // an accumulator per tile row and horizontal tap
+    static constexpr uint32_t TMEM_COLS = tmem_cols_for(kWgRows / RB * 3 * NB);  // an accumulator per RB rows and horizontal tap
+    static constexpr uint32_t DW_BYTES = N * 9 * CIN * 4;     // the CTA's sums, in the ring at the end
+    static_assert(kWgRows % RB == 0 && NB % 16 == 0 && NB <= 256 && DW_BYTES <= BAR_OFF, "rows per MMA");
     static_assert(X_READ <= STAGE, "an M block stays inside its stage");
     static_assert(NS >= 2 && BYTES <= 227 * 1024, "the ring fits shared memory");
     static_assert(S_COG % 128 == 0 && S_G % 128 == 0, "TMA destinations 128-byte aligned");
@@ -734,19 +740,20 @@ struct WgSmem {
 // memory by TMA and into the MMAs without a transposition. A horizontal tap is a
 // start address shifted by a pixel, the vertical taps are M rows.
 //   warp 0 (one thread)  TMA-loads tile j's X halo and dY into stage j % NS;
-//   warp 1 (one thread)  issues the tile's MMAs: per output row, 16 pixels and
-//                        horizontal tap one M = 128, N = cout, K = 16 MMA, into the
-//                        accumulator of that row and tap, which sums over all the
-//                        CTA's tiles (a row's own, so that a sum is short: with one
-//                        for the four rows the gradients of 957x539 were 8e-6 off the
+//   warp 1 (one thread)  issues the tile's MMAs: per RB output rows, 16 pixels and
+//                        horizontal tap one M = 128, N = RB cout, K = 16 MMA, into the
+//                        accumulator of those rows and that tap, which sums over all
+//                        the CTA's tiles (each rows' own, so that a sum is short: with
+//                        one for the tile the gradients of 957x539 were 8e-6 off the
 //                        float64 sums of the same bf16 values, 3e-6 as it is);
-//   warps 2-5            add up the tile's dY (the bias gradient), and at the end
-//                        add the accumulators to the gradient.
+//   warps 2-5            add up the tile's dY (the bias gradient), and at the end add
+//                        the taps' parts of the accumulators, then those to the gradient.
 // Borders and the pixels past a ragged edge are zeros from the tensor map.
-// Bound by the operand reads of N = 32 MMAs (4 KB of X per 32 cycles at 128 bytes a
-// cycle), 11 us a layer of 960x540. As a kernel that transposed X and dY through
-// 2-byte loads into registers, the four layers took 529 of a training step's 709
-// us; a step of two 960x540 frames goes from 1,250 to 555 us.
+// Bound by the MMAs' reads of X, 4 KB each: with one output row per MMA they took 68
+// cycles apiece whatever the channels, 29 us a layer of 960x540; with RB rows that
+// share the read a training step of two frames goes from 480 to 426 us. As a kernel that
+// transposed X and dY through 2-byte loads into registers, the four layers took 529 of
+// one frame's 709 us.
 template <int CIN, int N>
 __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __grid_constant__ CUtensorMap x_map,
                                                          const __grid_constant__ CUtensorMap dy_map) {
@@ -803,7 +810,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __gr
         for (int j = issued - NS > 0 ? issued - NS : 0; j < issued; ++j)
             if (!mbar_wait(&full[j % NS], (uint32_t)(j / NS) & 1u)) ok = false;
     } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = idesc_bf16(128, N) | (1u << 15) | (1u << 16);  // A and B MN-major
+        constexpr uint32_t idesc = idesc_bf16(128, L::NB) | (1u << 15) | (1u << 16);  // A and B MN-major
         bool issued = false;
         for (int j = 0; j < my_tiles; ++j) {
             const int buf = j % NS;
@@ -816,13 +823,13 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __gr
             const uint64_t dx0 = umma_desc(smem_u32(smem + buf * L::STAGE), 128, L::S_G);
             const uint64_t dd0 = umma_desc(smem_u32(smem + buf * L::STAGE + L::DY_OFF), 128, L::S_COG);
 #pragma unroll 1
-            for (int r = 0; r < kWgRows; ++r) {
+            for (int r = 0; r < kWgRows; r += L::RB) {
 #pragma unroll
                 for (int s = 0; s < kWgKP / 16; ++s) {
                     const uint64_t dd = dd0 + ((r * L::S_DYROW + s * 256) >> 4);
 #pragma unroll
                     for (int dx = 0; dx < 3; ++dx)
-                        mma_bf16(tmem + (r * 3 + dx) * N, dx0 + ((r * L::S_ROW + s * 256 + dx * 16) >> 4), dd, idesc,
+                        mma_bf16(tmem + (r / L::RB * 3 + dx) * L::NB, dx0 + ((r * L::S_ROW + s * 256 + dx * 16) >> 4), dd, idesc,
                                  (j > 0 || s > 0) ? 1u : 0u);
                 }
             }
@@ -875,28 +882,38 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __gr
     const bool all_ok = __syncthreads_and(ok ? 1 : 0) != 0;
     tc_fence_after();
     if (all_ok && my_tiles > 0 && warp >= 2) {
+        // the ring is free: every copy has landed and every MMA has read its operands
+        float* const dw = reinterpret_cast<float*>(smem);  // [N][9][CIN], as the gradient
+        auto sync_four = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+        for (int i = tid - 64; i < N * 9 * CIN; i += 128) dw[i] = 0.0f;
+        sync_four();
         const int quad = warp & 3;  // the TMEM lanes this warp may read
-        const int m = quad * 32 + lane, dy = m / 8 / L::G, c_in = m / 8 % L::G * 8 + m % 8;
+        const int m = quad * 32 + lane, xr = m / 8 / L::G, c_in = m / 8 % L::G * 8 + m % 8;
+        for (int b = 0; b < L::RB; ++b) {  // in turn: for one dY row, X rows are different taps
+            const int dy = xr - b;
+#pragma unroll 1
+            for (int dx = 0; dx < 3; ++dx) {
+                float acc[N];
 #pragma unroll
-        for (int dx = 0; dx < 3; ++dx) {
-            float acc[N];
+                for (int c = 0; c < N; ++c) acc[c] = 0.0f;
 #pragma unroll
-            for (int c = 0; c < N; ++c) acc[c] = 0.0f;
+                for (int r = 0; r < kWgRows / L::RB; ++r)
 #pragma unroll
-            for (int r = 0; r < kWgRows; ++r)
+                    for (int c = 0; c < N; c += 16) {
+                        float part[16];
+                        tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (r * 3 + dx) * L::NB + b * N + c, part);
 #pragma unroll
-                for (int c = 0; c < N; c += 16) {
-                    float row[16];
-                    tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (r * 3 + dx) * N + c, row);
+                        for (int i = 0; i < 16; ++i) acc[c + i] += part[i];
+                    }
+                if (dy >= 0 && dy < 3) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[c + i] += row[i];
+                    for (int c = 0; c < N; ++c) dw[(c * 9 + 3 * dy + dx) * CIN + c_in] += acc[c];
                 }
-            if (dy < 3) {
-#pragma unroll
-                for (int c = 0; c < N; ++c)
-                    if (acc[c] != 0.0f) atomicAdd(a.dw + ((size_t)c * 9 + 3 * dy + dx) * CIN + c_in, acc[c]);
             }
+            sync_four();
         }
+        for (int i = tid - 64; i < N * 9 * CIN; i += 128)
+            if (dw[i] != 0.0f) atomicAdd(a.dw + i, dw[i]);
     }
     tc_fence_before();
     __syncthreads();
