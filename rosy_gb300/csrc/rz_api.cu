@@ -236,6 +236,7 @@ struct rz_ctx {
     rz_debug_object* d_debug_objects = nullptr;
     DebugPair* d_debug_pairs = nullptr;
     DebugSeg* d_debug_segs = nullptr;
+    uint2* d_debug_boxes = nullptr;  // of the segments
     size_t debug_seg_capacity = 0;
     uint32_t debug_count = 0;     // segments per view in the current layout (0: overlay off)
     cudaEvent_t stage_ev[RZ_STAGE_COUNT + 1] = {};
@@ -708,8 +709,10 @@ int build_layout(rz_ctx* c) {
         const size_t segs = c->debug_pairs.size() * c->views.size();
         if (segs > c->debug_seg_capacity) {
             dfree(c->d_debug_segs);
+            dfree(c->d_debug_boxes);
             c->debug_seg_capacity = 0;
             RZ_CUDA(c, dalloc(&c->d_debug_segs, segs), "overlay segments");
+            RZ_CUDA(c, dalloc(&c->d_debug_boxes, segs), "overlay segment boxes");
             c->debug_seg_capacity = segs;
         }
         RZ_CUDA(c, dalloc(&c->d_debug_objects, c->debug_objects.size()), "overlay objects");
@@ -1139,7 +1142,7 @@ int enqueue_frame(rz_ctx* c) {
     if (c->blended_tris || c->debug_count) {
         if (c->debug_count)
             launch_debug_prep(c->d_debug_pairs, c->debug_count, c->d_debug_objects, c->d_views, (uint32_t)c->views.size(),
-                              c->d_debug_segs, s);
+                              c->d_debug_segs, c->d_debug_boxes, s);
         BlendParams bp{};
         bp.sh = sh;
         bp.sh.draws = c->d_blended_draws;
@@ -1152,6 +1155,7 @@ int enqueue_frame(rz_ctx* c) {
         bp.error_flags = &c->d_report->camera_errors;
         bp.record_capacity = c->blended_pass.record_capacity;
         bp.debug = c->d_debug_segs;
+        bp.debug_boxes = c->d_debug_boxes;
         bp.debug_count = c->debug_count;
         launch_blend(bp, s);
     }
@@ -1410,6 +1414,7 @@ void rz_destroy(rz_ctx* c) {
     dfree(c->d_debug_objects);
     dfree(c->d_debug_pairs);
     dfree(c->d_debug_segs);
+    dfree(c->d_debug_boxes);
     dfree(c->d_gb_albedo);
     dfree(c->d_gb_normal);
     dfree(c->d_gb_sources);

@@ -226,7 +226,7 @@ struct ShadeParams {
 struct DebugPair {
     float a[4], b[4];
     uint32_t object;
-    uint32_t pad[3];
+    uint32_t pad[6];
 };
 
 // One segment of one view after the vertex stage, clipping and the viewport:
@@ -235,11 +235,13 @@ struct DebugPair {
 struct DebugSeg {
     int32_t X0, Y0, X1, Y1;
     float z0, z1;
-    uint32_t p0, p1;
     float rgb[3];
-    uint32_t live;                // 0: clipped away or outside the view
-    uint32_t pad[4];
+    float reach;                  // half the width times the length, not rounded below it (infinite: not known)
+    uint32_t pad[3];
 };
+
+// The box of a segment that is clipped away or outside the view: it meets no tile.
+constexpr uint32_t kDebugNoBox = 0xffffffffu;
 
 // (half the line width of 5 pixels, in 1/256 pixel)^2
 constexpr int64_t kDebugHalfWidth2 = 640 * 640;
@@ -254,6 +256,7 @@ struct BlendParams {
     uint32_t record_capacity;
     uint32_t debug_count;         // overlay segments per view (0: no overlay)
     const DebugSeg* debug;        // view v's segments at debug + v * debug_count, in draw order
+    const uint2* debug_boxes;     // their pixel boxes (x0 | y0 << 16, x1 | y1 << 16; kDebugNoBox: not drawn)
 };
 
 // Up to four buffers to zero in one launch (16-byte stores, byte tail).
@@ -290,7 +293,7 @@ size_t blend_box_count(uint32_t capacity);
 void launch_blend(const BlendParams& p, cudaStream_t stream);
 // k_debug_prep: the overlay's `count` segments for each of the `view_count` views.
 void launch_debug_prep(const DebugPair* pairs, uint32_t count, const rz_debug_object* objects, const ViewRec* views,
-                       uint32_t view_count, DebugSeg* out, cudaStream_t stream);
+                       uint32_t view_count, DebugSeg* out, uint2* boxes, cudaStream_t stream);
 void launch_shade(const ShadeParams& p, cudaStream_t stream);
 void launch_subpixel_sources(const ShadeParams& p, cudaStream_t stream);
 

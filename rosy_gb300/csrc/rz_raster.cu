@@ -1227,7 +1227,7 @@ __device__ CV debug_vertex(const rz_scene_data& sd, const rz_debug_object& d, co
 __global__ void __launch_bounds__(128) k_debug_prep(const DebugPair* __restrict__ pairs, uint32_t count,
                                                     const rz_debug_object* __restrict__ objects,
                                                     const ViewRec* __restrict__ views, uint32_t view_count,
-                                                    DebugSeg* __restrict__ out) {
+                                                    DebugSeg* __restrict__ out, uint2* __restrict__ boxes) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (uint64_t)count * view_count) return;
     const uint32_t v = (uint32_t)(i / count), k = (uint32_t)(i % count);
@@ -1235,6 +1235,7 @@ __global__ void __launch_bounds__(128) k_debug_prep(const DebugPair* __restrict_
     const rz_debug_object& d = objects[pr.object];
     const ViewRec& VR = views[v];
     DebugSeg s{};
+    uint2 box = make_uint2(kDebugNoBox, 0u);
     s.rgb[0] = d.color[0];
     s.rgb[1] = d.color[1];
     s.rgb[2] = d.color[2];
@@ -1266,25 +1267,26 @@ __global__ void __launch_bounds__(128) k_debug_prep(const DebugPair* __restrict_
         s.Y1 = sb.Y;
         s.z0 = sa.z;
         s.z1 = sb.z;
+        const float dx = (float)((int64_t)sb.X - sa.X), dy = (float)((int64_t)sb.Y - sa.Y);
+        // an end whose w nearly vanishes can land far out, where the products of debug_meets may wrap
+        const bool far = fmaxf(fmaxf(fabsf((float)sa.X), fabsf((float)sa.Y)), fmaxf(fabsf((float)sb.X), fabsf((float)sb.Y))) > 1.0e8f;
+        s.reach = far ? INFINITY : (float)kDebugHalfWidth * sqrtf(dx * dx + dy * dy) * 1.00001f;
         const int x0 = max(0, (min(sa.X, sb.X) - kDebugHalfWidth) >> 8);
         const int x1 = min(VR.width - 1, (max(sa.X, sb.X) + kDebugHalfWidth) >> 8);
         const int y0 = max(0, (min(sa.Y, sb.Y) - kDebugHalfWidth) >> 8);
         const int y1 = min(VR.height - 1, (max(sa.Y, sb.Y) + kDebugHalfWidth) >> 8);
-        live = x0 <= x1 && y0 <= y1;
-        if (live) {
-            s.p0 = (uint32_t)x0 | ((uint32_t)y0 << 16);
-            s.p1 = (uint32_t)x1 | ((uint32_t)y1 << 16);
-        }
+        if (x0 <= x1 && y0 <= y1)
+            box = make_uint2((uint32_t)x0 | ((uint32_t)y0 << 16), (uint32_t)x1 | ((uint32_t)y1 << 16));
     }
-    s.live = live ? 1u : 0u;
     out[i] = s;
+    boxes[i] = box;
 }
 
 void launch_debug_prep(const DebugPair* pairs, uint32_t count, const rz_debug_object* objects, const ViewRec* views,
-                       uint32_t view_count, DebugSeg* out, cudaStream_t stream) {
+                       uint32_t view_count, DebugSeg* out, uint2* boxes, cudaStream_t stream) {
     const uint64_t n = (uint64_t)count * view_count;
     if (n == 0) return;
-    k_debug_prep<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(pairs, count, objects, views, view_count, out);
+    k_debug_prep<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(pairs, count, objects, views, view_count, out, boxes);
     note_launch();
 }
 

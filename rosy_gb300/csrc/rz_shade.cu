@@ -1438,14 +1438,26 @@ void launch_subpixel_sources(const ShadeParams& p, cudaStream_t stream) {
 //   groups that meet it. Neighbours in the list are mostly neighbours on the screen
 //   (a mesh's triangles). Where they are not, every group meets every tile, and the
 //   tile tests the records it tested without the boxes, and 1/32 as many boxes.
+// * A tile's records are prepared once, a thread each (blend_prepare: edges relative to
+//   the tile in 32 bits, records that miss it left out), and each warp keeps those that
+//   meet its two rows. A pixel then tests a record with six multiplications and no branch;
+//   reading the record and its 64-bit edges pixel by pixel was a serial chain, 620 cycles
+//   a record, so that the fullest tile (318 records) ran 125 us.
 // * The fragments are shaded together: a pixel collects up to kBlendRound of them,
 //   the tile lists them (the first ones of all pixels, the second ones, ...), the
 //   block shades the list with all lanes busy, and each pixel blends its own in
 //   order. Shaded where they are met, a triangle of a few pixels ran the fragment
 //   stage for a few lanes of a warp.
-// 1279x717, 12,288 blended triangles (a median 4 square pixels) of 49,152: the frame
-// went from 636 to 125 us.
-constexpr int kBlendBatch = 512;   // records (or overlay segments) listed at a time
+// * The overlay's segments are tested by their boxes (8 bytes each, read in a row; the
+//   64-byte segments cost 118 MB a frame) and then against the tile itself, and a tile
+//   that meets nothing of either list finishes after one test.
+// 1279x717, 12,288 blended triangles (a median 4 square pixels) of 49,152 and 24 overlay
+// objects: the frame went from 636 us to 125 us with the boxes and the shading together,
+// to 113 us with the cheaper fragment stage, and to 91 us with the prepared records and
+// the overlay's boxes. What is left is the latency of the fullest tiles and of the
+// five loads that a tile waits for one after the other.
+constexpr int kBlendBatch = 512;   // group boxes (or overlay segments) tested at a time
+constexpr int kBlendList = 256;    // records of a tile prepared at a time
 constexpr int kBlendRound = 4;     // fragments a pixel collects before the tile shades them
 constexpr int kBlendGroup = 32;    // records of a group box
 constexpr int kBlendItems = 256 * kBlendRound;
@@ -1486,6 +1498,19 @@ __device__ __forceinline__ uint32_t compact_batch(uint32_t start, uint32_t n, in
     return total;
 }
 
+// Whether the 5-pixel line `s` can cover a sample of the 16x16 tile at pixel (tx0, ty0):
+// over the tile, `along` and `perp` of debug_covers differ from their values at its centre
+// by at most 8 pixels times |dx| + |dy|. Most tiles in the box of a long slanted line are
+// not met by the line.
+__device__ __forceinline__ bool debug_meets(const DebugSeg& s, int tx0, int ty0) {
+    if (s.reach > 1.0e30f) return true;
+    const long long dx = (long long)s.X1 - s.X0, dy = (long long)s.Y1 - s.Y0;
+    const long long ex = (long long)(tx0 + 8) * 256 - s.X0, ey = (long long)(ty0 + 8) * 256 - s.Y0;
+    const long long slack = 2048 * (llabs(dx) + llabs(dy)), along = ex * dx + ey * dy;
+    if (along + slack < 0 || along - slack >= dx * dx + dy * dy) return false;
+    return (float)(llabs(dx * ey - dy * ex) - slack) <= s.reach;
+}
+
 // Whether the 5-pixel line `s` covers the sample at (PX, PY) (1/256 pixel), and
 // its depth there: the rectangle 0 <= along < |d|^2, -(w/2)|d| < perp <= (w/2)|d|
 // in exact integers; depth fma(along/|d|^2, z1 - z0, z0) clamped to [0, 1].
@@ -1494,9 +1519,10 @@ __device__ __forceinline__ bool debug_covers(const DebugSeg& s, int32_t PX, int3
     const long long len2 = dx * dx + dy * dy;
     if (len2 == 0) return false;
     const long long ex = (long long)PX - s.X0, ey = (long long)PY - s.Y0;
+    const long long perp = dx * ey - dy * ex;
+    if ((float)llabs(perp) > s.reach) return false;  // further than the half width by more than a rounding
     const long long along = ex * dx + ey * dy;
     if (along < 0 || along >= len2) return false;
-    const long long perp = dx * ey - dy * ex;
     const __int128 lhs = (__int128)perp * perp, rhs = (__int128)kDebugHalfWidth2 * len2;
     if (perp >= 0 ? lhs > rhs : lhs >= rhs) return false;
     const float t = (float)along / (float)len2;
@@ -1570,6 +1596,72 @@ __device__ __forceinline__ uint32_t blend_samples(const TriRecord& rec, int px, 
     return pass;
 }
 
+// A record as a tile's pixels read it: edge i at (ux, uy) 1/256 pixels from the tile's
+// corner is e[i] + a[i] * ux + b[i] * uy, the top-left rule folded into e, and a sample is
+// covered where no edge is negative.
+struct BlendTri {
+    int32_t e[3], a[3], b[3];
+    int32_t X0, Y0;
+    uint32_t id;
+    float z0, dzdx, dzdy;
+    uint32_t wide;  // record + 1 where an edge does not fit 32 bits over the tile, else 0
+};
+static_assert(sizeof(BlendTri) == 64, "four 16-byte reads");
+
+// Prepares record r for the tile at pixel (tx0, ty0); false where an edge leaves the whole
+// tile outside. The values are blend_samples' own: an edge that is negative nowhere in the
+// tile becomes zero, and one that changes sign there is small unless the triangle is huge.
+__device__ __forceinline__ bool blend_prepare(const TriRecord& rec, uint32_t r, int tx0, int ty0, BlendTri& t) {
+    const int4* src = reinterpret_cast<const int4*>(&rec);
+    const int4 q0 = __ldg(src), q1 = __ldg(src + 1);
+    const int32_t X[3] = {q0.x, q0.z, q1.x}, Y[3] = {q0.y, q0.w, q1.y};
+    bool meets = true, wide = false;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int a = (i + 1) % 3, b = (i + 2) % 3;
+        const int32_t dx = X[b] - X[a], dy = Y[b] - Y[a];
+        const bool tl = dy < 0 || (dy == 0 && dx > 0);
+        const int64_t e = (int64_t)dx * ((int64_t)ty0 * 256 - Y[a]) - (int64_t)dy * ((int64_t)tx0 * 256 - X[a]) - (tl ? 0 : 1);
+        const int64_t lo = e + 4096 * ((int64_t)min(dx, 0) - (int64_t)max(dy, 0));
+        const int64_t hi = e + 4096 * ((int64_t)max(dx, 0) - (int64_t)min(dy, 0));
+        meets = meets && hi >= 0;
+        const bool cuts = lo < 0;
+        wide = wide || (cuts && (lo < -2147483647LL || hi > 2147483647LL));
+        t.e[i] = cuts ? (int32_t)e : 0;
+        t.a[i] = cuts ? -dy : 0;
+        t.b[i] = cuts ? dx : 0;
+    }
+    t.X0 = X[0];
+    t.Y0 = Y[0];
+    t.id = rec.id;
+    t.z0 = __int_as_float(q1.z);
+    t.dzdx = __int_as_float(q1.w);
+    t.dzdy = rec.dzdy;
+    t.wide = wide ? r + 1u : 0u;
+    return meets;
+}
+
+// blend_samples from a prepared record of the tile at (tx0, ty0), without a branch.
+template <bool kMsaa>
+__device__ __forceinline__ uint32_t blend_pass(const BlendTri& t, int px, int py, int tx0, int ty0, const float* dst_depth) {
+    const int4* q = reinterpret_cast<const int4*>(&t);
+    const int4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3];  // e, a0 | a1 a2, b0 b1 | b2, X0, Y0, id | z0, dzdx, dzdy, wide
+    uint32_t pass = 0;
+#pragma unroll
+    for (int k = 0; k < (kMsaa ? kMsaaSamples : 1); ++k) {
+        const int32_t PX = px * 256 + (kMsaa ? msaa_x(k) : 128), PY = py * 256 + (kMsaa ? msaa_y(k) : 128);
+        const uint32_t ux = (uint32_t)(PX - tx0 * 256), uy = (uint32_t)(PY - ty0 * 256);
+        const uint32_t E0 = (uint32_t)q0.x + (uint32_t)q0.w * ux + (uint32_t)q1.z * uy;
+        const uint32_t E1 = (uint32_t)q0.y + (uint32_t)q1.x * ux + (uint32_t)q1.w * uy;
+        const uint32_t E2 = (uint32_t)q0.z + (uint32_t)q1.y * ux + (uint32_t)q2.x * uy;
+        float z = fmaf(__int_as_float(q3.y), (float)(PX - q2.y), fmaf(__int_as_float(q3.z), (float)(PY - q2.z), __int_as_float(q3.x)));
+        z = z > 0.0f ? z : 0.0f;
+        z = z > 1.0f ? 1.0f : z;
+        if ((int32_t)(E0 | E1 | E2) >= 0 && z >= dst_depth[k]) pass |= 1u << k;
+    }
+    return pass;
+}
+
 // Shades the listed fragments: item i is the triangle item_id[i] (id + 1) at pixel
 // item_px[i] (row * 16 + column) of the tile; its colour goes to item_out[i], and
 // item_id[i] becomes 0 where it is discarded.
@@ -1594,9 +1686,10 @@ template <bool kMsaa>
 __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
     constexpr int kSamples = kMsaa ? kMsaaSamples : 1;
     __shared__ float s_srgb[256];
-    __shared__ uint32_t s_groups[256];
-    __shared__ uint32_t s_list[kBlendBatch];
-    __shared__ uint2 s_box[kBlendBatch];
+    __shared__ uint32_t s_list[kBlendBatch];  // groups (or overlay segments) that meet the tile
+    __shared__ alignas(16) BlendTri s_tri[kBlendList];
+    __shared__ uint8_t s_rows[kBlendList];           // first and last row of a prepared record in the tile
+    __shared__ uint8_t s_mine[256 / 32][kBlendList]; // the prepared records that meet a warp's two rows
     __shared__ uint32_t s_count[kBlendRound][256 / 32];
     __shared__ TileNdc s_ndc;
     __shared__ uint32_t s_id[kBlendItems];
@@ -1605,10 +1698,17 @@ __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
     __shared__ uint32_t s_view;
     const ShadeParams& P = B.sh;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    s_srgb[tid] = P.srgb_table[tid];
-    if (tid == 0) s_view = tile_view(P.views, P.view_count, blockIdx.x + P.block_offset);
-    __syncthreads();
-    const uint32_t view = s_view;
+    // a pass whose look-back gave up has records at unreliable slots: blend none of them
+    const bool records_ok = !B.error_flags || !(*B.error_flags & kErrLookbackTimeout);
+    const uint32_t n = records_ok ? min(B.header->records, B.record_capacity) : 0u;
+    const uint32_t groups = (n + kBlendGroup - 1) / kBlendGroup;
+    const float srgb = P.srgb_table[tid];
+    uint32_t view = 0;
+    if (P.view_count > 1) {
+        if (tid == 0) s_view = tile_view(P.views, P.view_count, blockIdx.x + P.block_offset);
+        __syncthreads();
+        view = s_view;
+    }
     const ViewRec& VR = P.views[view];
     const uint32_t lt = blockIdx.x + P.block_offset - VR.shade_block_base;
     const uint32_t tiles_x = ((uint32_t)VR.width + 15) / 16;
@@ -1617,98 +1717,130 @@ __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
     const bool inside = px < VR.width && py < VR.height;
     const size_t p = inside ? (size_t)py * VR.width + px : 0;
     const size_t plane = (size_t)VR.width * VR.height;
-    if (tid < 16) s_ndc.x[tid] = ndc(tx0 + tid, VR.width);
-    else if (tid < 32) s_ndc.y[tid - 16] = ndc(ty0 + tid - 16, VR.height);
     // per coverage sample: the RGBA16F value and the opaque depth it is tested against
-    float col[kSamples][4];
+    uint2 held[kSamples];
     float dst_depth[kSamples];
 #pragma unroll
     for (int k = 0; k < kSamples; ++k) {
-        dst_depth[k] = 0.f;
+        held[k] = inside ? VR.color16[p + k * plane] : make_uint2(0u, 0u);
+        dst_depth[k] = !inside ? 0.0f : kMsaa ? __uint_as_float((uint32_t)(VR.vis[p + k * plane] >> 32)) : VR.depth[p];
+    }
+    const int lane = tid & 31, warp = tid >> 5;
+    // Most tiles meet nothing of the list or the overlay: they are known by one test of the boxes
+    bool any = groups > kBlendBatch || B.debug_count > kBlendBatch;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) col[k][i] = 0.f;
-        if (inside) {
-            const uint2 c = VR.color16[p + k * plane];
-            const __half2 rg = *reinterpret_cast<const __half2*>(&c.x), ba = *reinterpret_cast<const __half2*>(&c.y);
-            col[k][0] = __low2float(rg);
-            col[k][1] = __high2float(rg);
-            col[k][2] = __low2float(ba);
-            col[k][3] = __high2float(ba);
-            dst_depth[k] = kMsaa ? __uint_as_float((uint32_t)(VR.vis[p + k * plane] >> 32)) : VR.depth[p];
+    for (int k = 0; k < kBlendBatch / 256; ++k) {
+        const uint32_t i = tid + 256 * k;
+        if (i < groups) {
+            const uint4 b = __ldg(&B.boxes[i]);
+            any = any || (b.z <= view && view <= b.w && box_meets(b.x, b.y, tx0, ty0));
+        }
+        if (i < B.debug_count) {
+            const uint2 b = __ldg(&B.debug_boxes[(size_t)view * B.debug_count + i]);
+            any = any || box_meets(b.x, b.y, tx0, ty0);
         }
     }
-    const bool lit = lit_view(*VR.scene);
-    // a pass whose look-back gave up has records at unreliable slots: blend none of them
-    const bool records_ok = !B.error_flags || !(*B.error_flags & kErrLookbackTimeout);
-    const uint32_t n = records_ok ? min(B.header->records, B.record_capacity) : 0u;
-    const uint32_t groups = (n + kBlendGroup - 1) / kBlendGroup;
-    const int lane = tid & 31, warp = tid >> 5;
-    for (uint32_t first = 0; first < groups; first += 256) {
-        const uint32_t ngroups = compact_batch<1>(first, groups, tid, s_groups, s_count[0], [&](uint32_t g) {
+    s_srgb[tid] = srgb;
+    if (tid < 16) s_ndc.x[tid] = ndc(tx0 + tid, VR.width);
+    else if (tid < 32) s_ndc.y[tid - 16] = ndc(ty0 + tid - 16, VR.height);
+    any = __syncthreads_or(any) != 0;
+    const bool lit = any && lit_view(*VR.scene);
+    float col[kSamples][4];
+#pragma unroll
+    for (int k = 0; k < kSamples; ++k) {
+        const __half2 rg = *reinterpret_cast<const __half2*>(&held[k].x), ba = *reinterpret_cast<const __half2*>(&held[k].y);
+        col[k][0] = __low2float(rg);
+        col[k][1] = __high2float(rg);
+        col[k][2] = __low2float(ba);
+        col[k][3] = __high2float(ba);
+    }
+    for (uint32_t first = 0; any && first < groups; first += kBlendBatch) {
+        const uint32_t ngroups = compact_batch<kBlendBatch / 256>(first, groups, tid, s_list, s_count[0], [&](uint32_t g) {
             const uint4 b = __ldg(&B.boxes[g]);
             return b.z <= view && view <= b.w && box_meets(b.x, b.y, tx0, ty0);
         });
-        for (uint32_t gs = 0; gs < ngroups; gs += kBlendBatch / kBlendGroup) {
-            // the groups' records whose box meets the tile, in order: kPer groups per warp, a record per lane
-            constexpr int kPer = kBlendBatch / kBlendGroup / 8;
-            uint32_t hits[kPer], rec_of[kPer], found = 0;
-            uint2 box[kPer];
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                const uint32_t gi = gs + kPer * warp + q;
+        for (uint32_t gs = 0, listed = 0; gs < ngroups;) {
+            // the groups' records that meet the tile, in order, until the list is full: a group per warp, a record per lane
+            for (; gs < ngroups; gs += 256 / kBlendGroup) {
+                BlendTri t;
+                uint32_t rows = 0;
                 bool hit = false;
-                rec_of[q] = 0u;
-                box[q] = make_uint2(0u, 0u);
-                if (gi < ngroups) {
-                    rec_of[q] = s_groups[gi] * kBlendGroup + lane;
-                    if (rec_of[q] < n) {
-                        const TriRecord& rec = B.records[rec_of[q]];
-                        box[q] = make_uint2(rec.p0, rec.p1);
-                        hit = (rec.view & kViewMask) == view && box_meets(rec.p0, rec.p1, tx0, ty0);
+                if (gs + warp < ngroups) {
+                    const uint32_t r = s_list[gs + warp] * kBlendGroup + lane;
+                    if (r < n) {
+                        const TriRecord& rec = B.records[r];
+                        const uint32_t p0 = rec.p0, p1 = rec.p1;
+                        hit = (rec.view & kViewMask) == view && box_meets(p0, p1, tx0, ty0);
+                        if (hit) hit = blend_prepare(rec, r, tx0, ty0, t);
+                        rows = (uint32_t)(max((int)(p0 >> 16) - ty0, 0) | (min((int)(p1 >> 16) - ty0, 15) << 4));
                     }
                 }
-                hits[q] = __ballot_sync(0xffffffffu, hit);
-                found += __popc(hits[q]);
-            }
-            if (lane == 0) s_count[0][warp] = found;
-            __syncthreads();
-            uint32_t at = 0, total = 0;
-            for (int w = 0; w < 8; ++w) {
-                if (w < warp) at += s_count[0][w];
-                total += s_count[0][w];
-            }
-#pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-                if ((hits[q] >> lane) & 1u) {
-                    const uint32_t i = at + __popc(hits[q] & ((1u << lane) - 1u));
-                    s_list[i] = rec_of[q];
-                    s_box[i] = box[q];
+                const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+                if (lane == 0) s_count[0][warp] = __popc(hits);
+                __syncthreads();
+                uint32_t at = listed, total = 0;
+                for (int w = 0; w < 8; ++w) {
+                    if (w < warp) at += s_count[0][w];
+                    total += s_count[0][w];
                 }
-                at += __popc(hits[q]);
+                const bool full = listed + total > kBlendList;  // they wait for the next list
+                if (hit && !full) {
+                    at += __popc(hits & ((1u << lane) - 1u));
+                    s_tri[at] = t;
+                    s_rows[at] = (uint8_t)rows;
+                }
+                __syncthreads();
+                if (full) break;
+                listed += total;
             }
-            __syncthreads();
-            uint32_t j = 0;  // the pixel's next record of the list
-            bool more = total != 0;
+            uint32_t mine = 0, far = 0;
+            for (uint32_t base = 0; base < listed; base += 32) {
+                const uint32_t i = base + lane, rows = i < listed ? s_rows[i] : 15u;  // 15: none
+                const bool hit = (int)(rows & 15u) <= 2 * warp + 1 && (int)(rows >> 4) >= 2 * warp;
+                const uint32_t m = __ballot_sync(0xffffffffu, hit);
+                if (hit) s_mine[warp][mine + __popc(m & ((1u << lane) - 1u))] = (uint8_t)i;
+                far |= __ballot_sync(0xffffffffu, hit && s_tri[i].wide != 0u);
+                mine += __popc(m);
+            }
+            __syncwarp();
+            uint32_t next = 0, open = 0;  // the warp's next record; the pixel's fragments of the last ones, not yet taken
+            bool more = listed != 0;
+            listed = 0;
             while (more) {
-                // up to kBlendRound fragments of the pixel, in order
+                // up to kBlendRound fragments of the pixel, in order. The warp tests kLook records at a time,
+                // and stops at the first that leave a pixel of it with more fragments than it can take.
+                constexpr uint32_t kLook = 32 / kSamples;
                 uint32_t frag[kBlendRound], pass_of = 0, nf = 0;
 #pragma unroll
                 for (int r = 0; r < kBlendRound; ++r) frag[r] = 0u;
-                if (inside) {
-                    for (; j < total && nf < kBlendRound; ++j) {
-                        const uint2 b = s_box[j];
-                        const int bx0 = b.x & 0xffff, by0 = b.x >> 16, bx1 = b.y & 0xffff, by1 = b.y >> 16;
-                        if (px < bx0 || px > bx1 || py < by0 || py > by1) continue;
-                        const TriRecord& rec = B.records[s_list[j]];
-                        const uint32_t pass = blend_samples<kMsaa>(rec, px, py, dst_depth);
-                        if (!pass) continue;
-                        const uint32_t id = rec.id;
+                for (;;) {
+                    while (open != 0u && nf < kBlendRound) {
+                        const uint32_t at = (uint32_t)(__ffs((int)open) - 1) / kSamples;
+                        const uint32_t id = s_tri[s_mine[warp][next - kLook + at]].id;
 #pragma unroll
                         for (int r = 0; r < kBlendRound; ++r)
                             if (nf == (uint32_t)r) frag[r] = id;
-                        pass_of |= pass << (4 * nf);
+                        constexpr uint32_t kAll = (1u << kSamples) - 1u;
+                        pass_of |= ((open >> (kSamples * at)) & kAll) << (4 * nf);
+                        open &= ~(kAll << (kSamples * at));
                         ++nf;
                     }
+                    if (next >= mine || __any_sync(0xffffffffu, open != 0u)) break;
+                    const uint32_t look = min(mine - next, kLook);
+                    if (far == 0u) {
+#pragma unroll 4
+                        for (uint32_t q = 0; q < look; ++q)
+                            open |= blend_pass<kMsaa>(s_tri[s_mine[warp][next + q]], px, py, tx0, ty0, dst_depth) << (kSamples * q);
+                    } else {
+#pragma unroll 1
+                        for (uint32_t q = 0; q < look; ++q) {
+                            const BlendTri& t = s_tri[s_mine[warp][next + q]];
+                            open |= (t.wide ? blend_samples<kMsaa>(B.records[t.wide - 1u], px, py, dst_depth)
+                                            : blend_pass<kMsaa>(t, px, py, tx0, ty0, dst_depth)) << (kSamples * q);
+                        }
+                    }
+                    if (!inside) open = 0u;
+                    next += kLook;
                 }
                 uint32_t before[kBlendRound];
 #pragma unroll
@@ -1750,25 +1882,26 @@ __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
                         col[k][3] = half_round(a);
                     }
                 }
-                more = __syncthreads_or(inside && j < total) != 0;
+                more = __syncthreads_or(open != 0u || next < mine) != 0;
             }
         }
     }
     // Debug-line overlay after the blended list (src/Engine/Graphics.cpp:5694-5738): the same
     // blend state and depth test, depth writes off; a covered sample in front of the opaque
     // depth takes the line's colour (SRC_ALPHA with alpha 1 keeps only the source).
-    if (B.debug_count) {
+    if (any && B.debug_count) {
         const DebugSeg* __restrict__ segs = B.debug + (size_t)view * B.debug_count;
+        const uint2* __restrict__ boxes = B.debug_boxes + (size_t)view * B.debug_count;
         for (uint32_t start = 0; start < B.debug_count; start += kBlendBatch) {
-            const uint32_t total = compact_batch<2>(start, B.debug_count, tid, s_list, s_count[0], [&](uint32_t r) {
-                const DebugSeg& sg = segs[r];
-                return sg.live && box_meets(sg.p0, sg.p1, tx0, ty0);
+            const uint32_t total = compact_batch<kBlendBatch / 256>(start, B.debug_count, tid, s_list, s_count[0], [&](uint32_t r) {
+                const uint2 b = __ldg(&boxes[r]);
+                return box_meets(b.x, b.y, tx0, ty0) && debug_meets(segs[r], tx0, ty0);
             });
             if (inside) {
                 for (uint32_t j = 0; j < total; ++j) {
                     const DebugSeg& sg = segs[s_list[j]];
-                    const int bx0 = sg.p0 & 0xffff, by0 = sg.p0 >> 16, bx1 = sg.p1 & 0xffff, by1 = sg.p1 >> 16;
-                    if (px < bx0 || px > bx1 || py < by0 || py > by1) continue;
+                    const uint2 b = __ldg(&boxes[s_list[j]]);
+                    if (px < (int)(b.x & 0xffffu) || px > (int)(b.y & 0xffffu) || py < (int)(b.x >> 16) || py > (int)(b.y >> 16)) continue;
                     uint32_t pass = 0;  // samples covered and in front of the opaque depth
 #pragma unroll
                     for (int k = 0; k < kSamples; ++k) {

@@ -87,6 +87,16 @@ def test_overlay_random_objects(gpu, oracle, samples, blended):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("width,height,extent,samples", [(517, 301, 12.0, 1), (61, 700, 30.0, 4), (2200, 33, 2.5, 1)])
+def test_overlay_slanted_lines(gpu, oracle, width, height, extent, samples):
+    """Lines across many tiles, most of which their boxes meet and they do not; over 512 segments."""
+    s = sc.random_triangles(seed=3, triangles=300, width=width, height=height, shadow_size=64, texture_size=32)
+    s.samples = samples
+    s.debug_objects = sc.random_debug_objects(width, 96, extent=extent)
+    check_overlay(s, oracle, render_scene(s))
+
+
+@pytest.mark.gpu
 def test_overlay_updates_in_place_and_turns_off(gpu, oracle):
     s = sc.random_triangles(seed=9, triangles=500, width=160, height=96, shadow_size=128, texture_size=32)
     g = Graphics()

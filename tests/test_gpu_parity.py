@@ -344,6 +344,23 @@ def test_blended_lists(gpu, oracle, samples, width, height, triangles, spread, m
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("samples", [1, 4])
+@pytest.mark.parametrize("width,height,triangles,spread", [
+    (2300, 19, 80, 60.0),  # edges of more than 2,048 pixels do not fit 32 bits over a tile
+    (40, 40, 700, 0.6),    # tiles with more records than are prepared at a time
+    (300, 31, 513, 0.02)])  # most tiles empty; records of a pixel or less
+def test_blended_edges(gpu, oracle, samples, width, height, triangles, spread):
+    s = sc.random_triangles(seed=53, triangles=triangles, width=width, height=height, shadow_size=64, texture_size=32)
+    v = s.vertices[:, 0:3].reshape(-1, 3, 3)
+    s.vertices[:, 0:3] = (v[:, :1] + (v - v[:, :1]) * np.float32(spread)).reshape(-1, 3)
+    s = sc.with_blended(s, 0.9, alpha=0.3)
+    s.samples = samples
+    ref, out = run(s, oracle)
+    assert np.array_equal(out["ids"], ref["ids"])
+    assert np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32)).max() <= COLOR_TOL
+
+
+@pytest.mark.gpu
 def test_shading_error_against_fp64_oracle(gpu, oracle):
     """The oracle also shades in float64; the GPU's 8-bit sRGB colour stays within
     1.5 levels of that (0.5 of it is the 8-bit rounding itself)."""
