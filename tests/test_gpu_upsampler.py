@@ -142,6 +142,21 @@ def test_subpixel_sources_match_oracle(gpu, oracle, name):
         g.deinit()
 
 
+@pytest.mark.parametrize("width,height,triangles", [(33, 35, 6000), (16, 16, 400), (1, 1, 3), (17, 2, 900)])
+def test_subpixel_sources_of_crowded_tiles(gpu, oracle, width, height, triangles):
+    """Tiles that show more triangles than the table holds, and extents at a tile's edges."""
+    s = sc.random_triangles(seed=triangles, triangles=triangles, width=width, height=height, shadow_size=64, texture_size=16)
+    v = s.vertices[:, 0:3].reshape(-1, 3, 3)
+    s.vertices[:, 0:3] = (v[:, :1] + (v - v[:, :1]) * np.float32(0.3)).reshape(-1, 3)
+    g = _render(s)
+    try:
+        ref_ids = oracle.raster(s)["ids"]
+        assert np.array_equal(g.download()["ids"], ref_ids)
+        assert np.array_equal(g.download_gbuffer()["sources"], oracle.subpixel_sources(s, ref_ids))
+    finally:
+        g.deinit()
+
+
 def test_subpixel_sources_in_batched_views_and_not_with_msaa(gpu, oracle):
     """Per view of a batch (triangle ids are global; each view's plane resolves
     them through the whole draw list) the sources equal the oracle's for that view
