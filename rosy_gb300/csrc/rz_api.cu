@@ -181,6 +181,8 @@ struct rz_ctx {
     float* d_depth = nullptr;
     uint32_t* d_shadow = nullptr;
     uint2* d_color16 = nullptr;
+    uint32_t* d_front = nullptr;  // block depths of the camera raster (PassParams::front)
+    size_t front_capacity = 0;
     bool gbuffer = false;             // shading also writes albedo + normal (rz_set_gbuffer)
     uint32_t samples = 1;             // camera-pass samples per pixel (1 or 4)
     uint32_t* d_gb_albedo = nullptr;
@@ -684,6 +686,13 @@ int build_layout(rz_ctx* c) {
         RZ_CUDA(c, dalloc(&c->d_shadow, shadow), "shadow maps");
         c->shadow_capacity = shadow;
     }
+    const size_t front = (size_t)blocks * kTileBlocks;
+    if (front > c->front_capacity) {
+        dfree(c->d_front);
+        c->front_capacity = 0;
+        RZ_CUDA(c, dalloc(&c->d_front, front), "block depths");
+        c->front_capacity = front;
+    }
     // the overlay draws into the per-sample RGBA16F draw images, as the blended list does
     const bool overlay = !c->debug_pairs.empty();
     if ((!blended.empty() || overlay) && pix > c->color16_capacity) {
@@ -859,6 +868,7 @@ PassParams pass_params(rz_ctx* c, int kind) {
         p.mvp = reinterpret_cast<const float*>(c->d_camera_consts);
         p.mvp_stride = sizeof(DrawConsts) / sizeof(float);
         p.write_id = 1;
+        p.front = c->d_front;
         p.header = &c->d_report->camera;
         pb = &c->camera_pass;
     } else {
@@ -1012,7 +1022,9 @@ int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh
         PassParams cp = pass_params(c, 1);
         cp.clear_ptr[0] = c->d_vis;
         cp.clear_bytes[0] = c->pix_total * 8 * c->samples;
-        cp.clear_count = 1;
+        cp.clear_ptr[1] = c->d_front;
+        cp.clear_bytes[1] = (size_t)c->shade_blocks * kTileBlocks * 4;
+        cp.clear_count = 2;
         launch_setup(cp, s);
         cp.clear_count = 0;
         if (stamps) stamp(c, 5);
@@ -1067,7 +1079,9 @@ int enqueue_sequential(rz_ctx* c, cudaStream_t s, const ShadeParams& sh) {
             ClearList c2{};
             c2.ptr[0] = c->camera_pass.tile_status;
             c2.bytes[0] = (size_t)setup_ctas(rg.opaque_tris) * 8;
-            c2.count = 1;
+            c2.ptr[1] = c->d_front + (size_t)rg.block_base * kTileBlocks;
+            c2.bytes[1] = (size_t)rg.blocks * kTileBlocks * 4;
+            c2.count = 2;
             launch_clear(c2, c->sm_count, s);
         }
         if (rg.shadow_tris) {
@@ -1411,6 +1425,7 @@ void rz_destroy(rz_ctx* c) {
     dfree(c->d_depth);
     dfree(c->d_shadow);
     dfree(c->d_color16);
+    dfree(c->d_front);
     dfree(c->d_debug_objects);
     dfree(c->d_debug_pairs);
     dfree(c->d_debug_segs);

@@ -47,6 +47,7 @@ struct ViewRec {
     uint32_t* gb_normal;          // width*height world normal, octahedral 2 x f16, or null
     uint16_t* gb_sources;         // width*height sub-pixel source masks (single-sampled G-buffer), or null
 };
+static_assert(sizeof(ViewRec) == 128, "one cache line: 136 bytes cost every frame about 1 %");
 
 // gpu_material, src/Engine/Graphics.cpp:345-360, packed as in 4071-4150.
 struct GpuMaterial {
@@ -113,6 +114,7 @@ __host__ __device__ constexpr int32_t msaa_y(int k) { return k == 0 ? 32 : k == 
 
 constexpr int kStampW = 8;
 constexpr int kStampH = 4;
+constexpr uint32_t kTileBlocks = (16 / kStampW) * (16 / kStampH);  // stamps on the grid in a shading tile
 constexpr int kChunkStamps = 32;      // default stamps per raster work chunk
 constexpr int kSetupThreads = 256;    // triangles per setup CTA
 constexpr float kGuardBand = 64.0f;
@@ -185,6 +187,9 @@ struct PassParams {
     void* clear_ptr[2];
     size_t clear_bytes[2];
     uint32_t clear_count;
+    // camera pass: per 8x4 block of the visibility, eight to a 16x16 shading tile, a depth
+    // that every pixel of the block reaches (bits; see raster_front)
+    uint32_t* front;
     // camera passes only (else null): per triangle with valid indices, its draw's
     // material and its three varying record indices, for the shading
     uint4* tri_refs;

@@ -201,9 +201,21 @@ __device__ __forceinline__ int64_t area2(const SV& a, const SV& b, const SV& c) 
     return (int64_t)(b.X - a.X) * (int64_t)(c.Y - a.Y) - (int64_t)(c.X - a.X) * (int64_t)(b.Y - a.Y);
 }
 
-__device__ __forceinline__ uint32_t record_stamps(const TriRecord& r) {
+// Whether a camera record's stamps lie on the grid of the target's 8x4 blocks, so that
+// each has a block's depth to be tested against (see raster_front): where the row and the
+// column that this may add are few of many. (24x12 or 16x8 pixels gain nothing on deep
+// overdraw and cost a mesh scene up to 0.4 % more; 64x32 lose 3 % of a soup's frame.
+// Shadow passes have no grid: what they gained was within the noise, and scene-scale
+// frames lost 2 %.)
+constexpr int kGridW = 32, kGridH = 16;
+__device__ __forceinline__ bool on_grid(int px0, int py0, int px1, int py1) { return px1 - px0 >= kGridW - 1 && py1 - py0 >= kGridH - 1; }
+
+// A record's stamps: how many in a row (nsx) and in all.
+__device__ __forceinline__ uint32_t record_stamps(const TriRecord& r, bool camera, uint32_t& nsx) {
     const int px0 = r.p0 & 0xffff, py0 = r.p0 >> 16, px1 = r.p1 & 0xffff, py1 = r.p1 >> 16;
-    return (uint32_t)((px1 - px0) / kStampW + 1) * (uint32_t)((py1 - py0) / kStampH + 1);
+    const int m = camera && on_grid(px0, py0, px1, py1) ? -1 : 0;
+    nsx = (uint32_t)((px1 - px0 + (px0 & m & (kStampW - 1))) / kStampW + 1);
+    return nsx * (uint32_t)((py1 - py0 + (py0 & m & (kStampH - 1))) / kStampH + 1);
 }
 
 // The raster facts of a large record (packed by the setup, decoded by the raster):
@@ -217,7 +229,7 @@ constexpr uint32_t kFactNear = 8u, kFactCut = 16u, kFactSmall = 32u;
 // every edge value over the box plus a stamp of overhang is below 2 * ((90 + 8) * 256)^2 < 2^31
 constexpr int kSmallEdges = 90;
 
-__device__ __forceinline__ uint32_t large_facts(const TriRecord& r, int32_t bb_hi, uint32_t& nsx) {
+__device__ __forceinline__ uint32_t large_facts(const TriRecord& r, int32_t bb_hi) {
     const int32_t X[3] = {r.X0, r.X1, r.X2}, Y[3] = {r.Y0, r.Y1, r.Y2};
     const int px0 = (int)(r.p0 & 0xffff), py0 = (int)(r.p0 >> 16), px1 = (int)(r.p1 & 0xffff), py1 = (int)(r.p1 >> 16);
     uint32_t flags = 0;
@@ -229,14 +241,13 @@ __device__ __forceinline__ uint32_t large_facts(const TriRecord& r, int32_t bb_h
         if (!(dy < 0 || (dy == 0 && dx > 0))) flags |= 1u << i;
         near_origin = near_origin && abs(dx) < (1 << 26) && abs(dy) < (1 << 26);
     }
-    const int32_t lo_x = px0 * 256 - X[0], hi_x = px1 * 256 + 256 - X[0] + kStampW * 256;
-    const int32_t lo_y = py0 * 256 - Y[0], hi_y = py1 * 256 + 256 - Y[0] + kStampH * 256;
+    const int32_t lo_x = px0 * 256 - X[0] - kStampW * 256, hi_x = px1 * 256 + 256 - X[0] + kStampW * 256;
+    const int32_t lo_y = py0 * 256 - Y[0] - kStampH * 256, hi_y = py1 * 256 + 256 - Y[0] + kStampH * 256;
     const int32_t lim = 1 << 23;
     near_origin = near_origin && lo_x > -lim && hi_x < lim && lo_y > -lim && hi_y < lim;
     const int32_t max_x = max(X[0], max(X[1], X[2])), max_y = max(Y[0], max(Y[1], Y[2]));
     const bool cut = ((max_x - bb_hi) >> 8) > px1 || ((max_y - bb_hi) >> 8) > py1;
     const bool small = max_x - min(X[0], min(X[1], X[2])) <= kSmallEdges * 256 && max_y - min(Y[0], min(Y[1], Y[2])) <= kSmallEdges * 256;
-    nsx = (uint32_t)((px1 - px0) / kStampW + 1);
     return flags | (small ? kFactSmall : 0u) | (near_origin ? kFactNear : 0u) | (cut ? kFactCut : 0u);
 }
 
@@ -446,7 +457,8 @@ struct CountEmit {
             return;
         }
         ++recs;
-        stamps += record_stamps(r);
+        uint32_t nsx;
+        stamps += record_stamps(r, refs != nullptr, nsx);
     }
 };
 
@@ -471,13 +483,13 @@ struct WriteEmit {
             return;
         }
         uint32_t nsx;
-        r.view |= large_facts(r, P->bb_hi, nsx) << kRecFlagShift;
+        const uint64_t end = stamp + record_stamps(r, P->tri_refs != nullptr, nsx);
+        r.view |= large_facts(r, P->bb_hi) << kRecFlagShift;
         r.stamp_offset = stamp | ((uint64_t)nsx << kStampOffsetBits);
         store_record(P->records + rec, r);
         // chunks whose first stamp lies inside this record start here
         const uint64_t cs = P->chunk_stamps;
         uint64_t k = (stamp + cs - 1) / cs;
-        const uint64_t end = stamp + record_stamps(r);
         for (; k * cs < end; ++k) {
             if (k >= P->chunk_capacity) {
                 atomicOr(P->error_flags, kErrStampOverflow);
@@ -846,13 +858,15 @@ struct LargeRecord {
     int32_t dx[3], dy[3];
     uint32_t tl_bias[3];  // 0 on top-left edges, 1 otherwise
     bool near_origin, cut, small;  // see large_facts
+    bool grid;            // see on_grid
     float z0, dzdx, dzdy, bias;
-    int px0, py0, px1, py1;
+    int px0, py0, px1, py1;  // first pixel of the first stamp, last pixel of the box
     uint32_t id, nsx, view;
     uint64_t begin, end;
 };
 
 // Decodes a large record from its four 16-byte words.
+template <bool kCamera>
 __device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const int4 q2, const int4 q3, LargeRecord& L) {
     L.X[0] = q0.x;
     L.Y[0] = q0.y;
@@ -869,6 +883,11 @@ __device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const
     L.px1 = q2.w & 0xffff;
     L.py1 = (uint32_t)q2.w >> 16;
     L.id = (uint32_t)q3.x;
+    L.grid = kCamera && on_grid(L.px0, L.py0, L.px1, L.py1);
+    if (L.grid) {
+        L.px0 &= -kStampW;
+        L.py0 &= -kStampH;
+    }
     const uint32_t flags = (uint32_t)q3.y >> kRecFlagShift;
     L.view = (uint32_t)q3.y & kRecViewMask;
     L.begin = (uint64_t)(uint32_t)q3.z | ((uint64_t)((uint32_t)q3.w & 0xffu) << 32);
@@ -886,9 +905,10 @@ __device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const
     L.small = (flags & kFactSmall) != 0;
 }
 
+template <bool kCamera>
 __device__ __forceinline__ void load_large(const TriRecord* rec, LargeRecord& L) {
     const int4* src = reinterpret_cast<const int4*>(rec);
-    decode_large(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3), L);
+    decode_large<kCamera>(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3), L);
 }
 
 // Record staging of the chunk walk: a warp copies the records a chunk starts
@@ -957,6 +977,44 @@ __device__ __forceinline__ bool stamp_edges(const LargeRecord& L, int32_t PX, in
         }
     }
     return rejected != (1u << kSamples) - 1u;
+}
+
+// Where the depth of the 8x4 block at (sx0, sy0) of a record's target is kept.
+__device__ __forceinline__ uint32_t* front_of(const PassParams& P, uint32_t view, int sx0, int sy0) {
+    const ViewRec& V = P.views[view & kViewMask];
+    const uint32_t tile = V.shade_block_base + (uint32_t)(sy0 / 16) * (uint32_t)((V.width + 15) / 16) + (uint32_t)(sx0 / 16);
+    return P.front + (size_t)tile * kTileBlocks + (uint32_t)((sy0 / kStampH) % 4) * 2u + (uint32_t)((sx0 / kStampW) % 2);
+}
+
+// Whether a stamp that lies on the grid has a pixel to draw, given the depth `front` that
+// every pixel of its block reaches; and where it covers the block whole, its own least depth
+// raises that depth. What a stamp draws is always written, so the block reaches the depth
+// at the end whichever stamp is drawn first, and a stamp whose greatest depth stays below it
+// draws nothing that is seen. A lane does this for the stamp it prepares, so a hidden stamp
+// costs a thirty-second of one that is drawn. Frames of 4,096 random triangles over one
+// another: 640x360 44 -> 31.6 us, 960x540 with its network 147 -> 127 us; scenes of
+// small triangles are within 0.3 %. The greatest and least depth are the plane's at the corners:
+// its two sums round monotonically.
+template <int kSamples>
+__device__ __forceinline__ bool raster_front(const LargeRecord& L, int32_t PX, int32_t PY, const int32_t (&q)[kSamples][3],
+                                             uint32_t front, uint32_t* cell) {
+    const float x0 = (float)(PX - L.X[0]), y0 = (float)(PY - L.Y[0]);
+    const float x1 = x0 + (float)((kStampW - 1) * 256 + (kSamples > 1 ? 256 : 0)), y1 = y0 + (float)((kStampH - 1) * 256 + (kSamples > 1 ? 256 : 0));
+    if (!(fabsf(L.dzdx) + fabsf(L.dzdy) < INFINITY)) return true;
+    const bool rx = L.dzdx > 0.0f, ry = L.dzdy > 0.0f;
+    const float far_z = biased_depth(fmaf(L.dzdx, rx ? x0 : x1, fmaf(L.dzdy, ry ? y0 : y1, L.z0)), 0.0f);
+    const float near_z = biased_depth(fmaf(L.dzdx, rx ? x1 : x0, fmaf(L.dzdy, ry ? y1 : y0, L.z0)), 0.0f);
+    if (__float_as_uint(near_z) < front) return false;
+    if (__float_as_uint(far_z) <= front) return true;
+    bool whole = true;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int32_t least = min(L.dx[i], 0) * (kStampH - 1) + min(-L.dy[i], 0) * (kStampW - 1);
+#pragma unroll
+        for (int k = 0; k < kSamples; ++k) whole = whole && q[k][i] + least >= 0;
+    }
+    if (whole) atomicMax(cell, __float_as_uint(far_z));
+    return true;
 }
 
 // Leaves the stamp at (sx0, sy0) with edges q as entry i of w.
@@ -1104,11 +1162,13 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
             int sx0 = 0, sy0 = 0;
             int32_t PX = 0, PY = 0;  // the sample of the stamp's first pixel (its corner with 4x samples)
             int32_t q[kSamples][3];
+            uint32_t* cell = nullptr;  // its block's depth
+            uint32_t front = 0;
             LargeRecord L;
             if (s + lane < s_end && r < n_rec) {
                 const uint32_t j = r - r_cur;
-                if (j < (uint32_t)kStageRecords) decode_large(st[j][0], st[j][1], st[j][2], st[j][3], L);
-                else load_large(P.records + r, L);
+                if (j < (uint32_t)kStageRecords) decode_large<kWriteId>(st[j][0], st[j][1], st[j][2], st[j][3], L);
+                else load_large<kWriteId>(P.records + r, L);
                 if (s + lane >= L.begin && s + lane < L.end) {
                     // stamp i of the record, below 2^24: the quotient by stamps per row, off by one at most
                     const int i = (int)(s + lane - L.begin), nsx = (int)L.nsx;
@@ -1127,12 +1187,17 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
                     if (s + lane + 1 == L.end) ++r_after_this;
                     far = !L.near_origin;
                     live = !far;
+                    if (kWriteId && live && L.grid) {
+                        cell = front_of(P, L.view, sx0, sy0);
+                        front = __ldcg(cell);
+                    }
                 } else {  // cannot happen with a consistent chunk map
                     atomicOr(P.error_flags, kErrStampOverflow);
                 }
             }
             if (__all_sync(kAllLanes, !live || L.small)) live = live && stamp_edges<kSamples, int32_t>(L, PX, PY, q);
             else live = live && stamp_edges<kSamples, int64_t>(L, PX, PY, q);
+            if (kWriteId && cell && live) live = raster_front<kSamples>(L, PX, PY, q, front, cell);
             // the stamps that are left, in order: entry `at`; the first one of its record is a head
             const uint32_t left = __ballot_sync(kAllLanes, live), below = left & ((1u << lane) - 1u);
             const int at = __popc(below);
@@ -1150,7 +1215,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
             else raster_stamps<kWriteId, kSamples, false>(P, work, __popc(left), heads, 0u, lane, lx, ly);
             for (uint32_t m = __ballot_sync(kAllLanes, far); m; m &= m - 1) {
                 const int j = __ffs(m) - 1;
-                load_large(P.records + __shfl_sync(kAllLanes, r, j), L);
+                load_large<kWriteId>(P.records + __shfl_sync(kAllLanes, r, j), L);
                 const int px = __shfl_sync(kAllLanes, sx0, j) + lx, py = __shfl_sync(kAllLanes, sy0, j) + ly;
                 const Target T = view_target<kWriteId>(P, L.view);
                 const size_t plane = kMsaa ? plane_words(P, L.view) : 0;

@@ -346,6 +346,25 @@ def test_blended_lists(gpu, oracle, samples, width, height, triangles, spread, m
 @pytest.mark.gpu
 @pytest.mark.parametrize("samples", [1, 4])
 @pytest.mark.parametrize("width,height,triangles,spread", [
+    (200, 120, 600, 6.0),  # deep overdraw by triangles that cover blocks whole
+    (33, 17, 300, 3.0),    # records of the smallest extent on the block grid, and below it
+    (71, 45, 400, 40.0)])  # boxes cut on every side, blocks cut by the viewport
+def test_hidden_stamps(gpu, oracle, samples, width, height, triangles, spread):
+    """Stamps behind a block's depth are not drawn; of equal depths the later triangle stays."""
+    s = sc.random_triangles(seed=61, triangles=triangles, width=width, height=height, shadow_size=64, texture_size=16)
+    v = s.vertices[:, 0:3].reshape(-1, 3, 3)
+    v = v[:, :1] + (v - v[:, :1]) * np.float32(spread)
+    v[triangles // 2:] = v[:triangles - triangles // 2]  # the same triangles again
+    s.vertices[:, 0:3] = v.reshape(-1, 3)
+    s.samples = samples
+    ref, out = run(s, oracle)
+    assert np.array_equal(out["ids"], ref["ids"])
+    assert np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32)).max() <= COLOR_TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("samples", [1, 4])
+@pytest.mark.parametrize("width,height,triangles,spread", [
     (2300, 19, 80, 60.0),  # edges of more than 2,048 pixels do not fit 32 bits over a tile
     (40, 40, 700, 0.6),    # tiles with more records than are prepared at a time
     (300, 31, 513, 0.02)])  # most tiles empty; records of a pixel or less
