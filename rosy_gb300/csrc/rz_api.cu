@@ -925,6 +925,15 @@ void stamp(rz_ctx* c, int i) {
     if (c->timing) cudaEventRecord(c->stage_ev[i], c->stream);
 }
 
+// Whether a pass's setup and raster start as the launch before them ends (launch_next).
+// Where the depth targets take a while to zero, the setup's CTAs that come early stand in
+// the other branch's way: a 1080p frame with a 4096^2 shadow map (84 MB) went from 151.2 to
+// 152.9 us, 32 views (over 100 MB) from 149.0 to 149.9. Below that the latency counts:
+// 1280x720 with a 2048^2 map (24 MB), read back to the host, 144.3 -> 136.7 us, 640x360
+// (6 MB) 31.7 -> 31.1, and a 96x64 frame alone 62.8 -> 55.4. (With the raster let in before the setup's last CTAs end,
+// its persistent CTAs hold the SMs: the 640x360 frame took 35.9 us.)
+bool chained(const rz_ctx* c) { return c->shadow_total * 4 + c->pix_total * 8 * c->samples <= (32u << 20); }
+
 // Shadow passes of all views (src/Engine/Graphics.cpp:5195-5292): clear to 0,
 // per-draw matrices, setup, raster.
 // The shadow maps are zeroed by the setup launch when there is one (the raster
@@ -948,13 +957,14 @@ void enqueue_shadow(rz_ctx* c, cudaStream_t s, bool stamps) {
     else launch_clear(cl, c->sm_count, s);
     if (stamps) stamp(c, 1);
     if (c->shadow_tris) {
+        const bool chain = !stamps && chained(c);
         PassParams sp = pass_params(c, 0);
         sp.clear_ptr[0] = c->d_shadow;
         sp.clear_bytes[0] = c->shadow_total * 4;
         sp.clear_count = 1;
-        launch_setup(sp, s);
+        launch_setup(sp, s, chain);
         if (stamps) stamp(c, 2);
-        launch_raster(sp, c->sm_count, s);
+        launch_raster(sp, c->sm_count, s, 1, chain);
     } else if (stamps) {
         stamp(c, 2);
     }
@@ -966,7 +976,7 @@ void enqueue_shadow(rz_ctx* c, cudaStream_t s, bool stamps) {
 // by side on branches of their own, each with its part of the resident CTAs.
 int launch_camera_raster(rz_ctx* c, PassParams cp, cudaStream_t s, bool branches) {
     if (c->samples <= 1) {
-        launch_raster(cp, c->sm_count, s);
+        launch_raster(cp, c->sm_count, s, 1, branches && chained(c));
         return RZ_OK;
     }
     if (branches) RZ_CUDA(c, cudaEventRecord(c->msaa_fork, s), "camera raster fork");
@@ -1025,7 +1035,7 @@ int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh
         cp.clear_ptr[1] = c->d_front;
         cp.clear_bytes[1] = (size_t)c->shade_blocks * kTileBlocks * 4;
         cp.clear_count = 2;
-        launch_setup(cp, s);
+        launch_setup(cp, s, !stamps && chained(c));
         cp.clear_count = 0;
         if (stamps) stamp(c, 5);
         const int rc = launch_camera_raster(c, cp, s, !stamps);

@@ -284,9 +284,11 @@ void launch_prep(const DrawRec* draws, uint32_t n, const rz_object* objects, con
                  float* out_mvp, cudaStream_t stream, const ClearList* clear = nullptr, int sm_count = 0);
 void launch_prep_camera(const DrawRec* draws, uint32_t n, const rz_object* objects, const ViewRec* views,
                         DrawConsts* out, cudaStream_t stream, const ClearList* clear = nullptr, int sm_count = 0);
-void launch_setup(const PassParams& p, cudaStream_t stream);
+// `next`: follows the launch before it on the stream as launch_next does; that one is the pass's
+// k_prep or k_prep_camera (launch_setup) or its k_setup (launch_raster)
+void launch_setup(const PassParams& p, cudaStream_t stream, bool next = false);
 // `share`: the launch is one of that many that run side by side (its grid is that part of the resident CTAs)
-void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int share = 1);
+void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int share = 1, bool next = false);
 void launch_vertex(const ShadeParams& p, cudaStream_t stream);
 // k_vertex over the varying records [first, varying_count) of the draws in p
 // (whose varying_base values start at `first`).

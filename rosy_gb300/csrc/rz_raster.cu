@@ -40,6 +40,7 @@ namespace rz {
 // the two need one launch.
 __global__ void k_prep(const DrawRec* __restrict__ draws, uint32_t n, const rz_object* __restrict__ objects,
                        const ViewRec* __restrict__ views, float* __restrict__ out, ClearList L) {
+    pdl_allow_next();
     const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
     clear_share(L);
     if (d >= n) return;
@@ -528,16 +529,18 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
     __shared__ uint64_t s_base_recs, s_base_stamps;
     __shared__ uint32_t s_small_warp[kSetupThreads / 32];
     __shared__ uint32_t s_small_base;
+    // the pass's depth target is zeroed by the same launch: its stores overlap the
+    // setup arithmetic, and the raster (the next launch) sees it cleared. The frames
+    // that used it are done when the launch before this one starts.
+    for (uint32_t b = 0; b < P.clear_count; ++b)
+        zero_share(P.clear_ptr[b], P.clear_bytes[b], (size_t)blockIdx.x * blockDim.x + threadIdx.x,
+                   (size_t)gridDim.x * blockDim.x);
+    pdl_wait_previous();
     // The ordered list's look-back needs tiles numbered in the order the CTAs
     // start (a CTA only waits on tiles that have started); the unordered passes
     // wait on nobody and use the block index, sparing one same-address atomic
     // per CTA.
     if (P.ordered && threadIdx.x == 0) s_tile = atomicAdd(&P.header->ticket, 1u);
-    // the pass's depth target is zeroed by the same launch: its stores overlap the
-    // setup arithmetic, and the raster (the next launch) sees it cleared
-    for (uint32_t b = 0; b < P.clear_count; ++b)
-        zero_share(P.clear_ptr[b], P.clear_bytes[b], (size_t)blockIdx.x * blockDim.x + threadIdx.x,
-                   (size_t)gridDim.x * blockDim.x);
     const uint32_t tri_ctas = (P.tri_total + kSetupThreads - 1) / kSetupThreads;
     // CTAs launched only to share the zeroing hold no triangles: done
     if (!P.ordered && blockIdx.x >= tri_ctas) return;
@@ -703,7 +706,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
 
 int setup_ctas(uint32_t tri_total) { return (int)((tri_total + kSetupThreads - 1) / kSetupThreads); }
 
-void launch_setup(const PassParams& p, cudaStream_t stream) {
+void launch_setup(const PassParams& p, cudaStream_t stream, bool next) {
     int ctas = setup_ctas(p.tri_total);
     if (ctas == 0) return;
     if (!p.ordered && p.clear_count) {
@@ -715,7 +718,8 @@ void launch_setup(const PassParams& p, cudaStream_t stream) {
         const size_t want = std::min<size_t>(most / 32768, 4096);
         if ((size_t)ctas < want) ctas = (int)want;
     }
-    k_setup<<<ctas, kSetupThreads, 0, stream>>>(p);
+    if (next) launch_next(k_setup, ctas, kSetupThreads, 0, stream, p);
+    else k_setup<<<ctas, kSetupThreads, 0, stream>>>(p);
     note_launch();
 }
 
@@ -1121,6 +1125,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
     // a multisampled pass's launches number their warps together
     const uint32_t warps = ((gridDim.x * blockDim.x) >> 5) * (kMsaa ? kMsaaSamples : 1u);
     const uint32_t warp_id = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kMsaa ? kMsaaSamples : 1u) + (kMsaa ? P.part : 0u);
+    pdl_wait_previous();
     const uint64_t n_small = min(P.header->small_records, P.small_capacity);
     for (uint64_t base = (uint64_t)warp_id * 32u; base < n_small; base += (uint64_t)warps * 32u)
         if (base + lane < n_small) raster_small<kWriteId, kMsaa>(P, P.small_records + base + lane);
@@ -1235,7 +1240,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int share) {
+void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int share, bool next) {
     // persistent grid: as many CTAs as can be resident at once, with the launches beside this one
     static int occ[3] = {0, 0, 0};
     const int t = !p.write_id ? 0 : p.msaa ? 2 : 1;
@@ -1245,7 +1250,9 @@ void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int s
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kRasterThreads, 0);
         occ[t] = n > 0 ? n : 1;
     }
-    kernel<<<(sm_count * occ[t] + share - 1) / share, kRasterThreads, 0, stream>>>(p);
+    const int ctas = (sm_count * occ[t] + share - 1) / share;
+    if (next) launch_next(kernel, ctas, kRasterThreads, 0, stream, p);
+    else kernel<<<ctas, kRasterThreads, 0, stream>>>(p);
     note_launch();
 }
 

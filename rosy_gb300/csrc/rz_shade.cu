@@ -66,6 +66,7 @@ __device__ __forceinline__ F2 mix2(F2 x, F2 y, F2 w) { return x + w * (y - x); }
 // so that the two need one launch.
 __global__ void k_prep_camera(const DrawRec* __restrict__ draws, uint32_t n, const rz_object* __restrict__ objects,
                               const ViewRec* __restrict__ views, DrawConsts* __restrict__ out, ClearList L) {
+    pdl_allow_next();
     const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
     clear_share(L);
     if (d >= n) return;

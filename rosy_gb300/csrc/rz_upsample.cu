@@ -209,17 +209,6 @@ __device__ __forceinline__ void tmem_zero(uint32_t taddr, int cols) {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// Programmatic dependent launch. The kernels of a pass follow each other with the
-// next one's launch allowed once every CTA of this one has started (its CTAs then take
-// the SMs as this one's leave them, and set up barriers, tensor memory and weights),
-// and each waits here for the one before to be complete and its writes visible before
-// it touches what the pass computes. As every kernel does so, a kernel that gets past
-// this point comes after all the earlier ones. A pass's first kernel is launched
-// normally, after all that the stream holds. (957x539 inference, five kernels: 78 -> 64
-// us; a training step of two 960x540 frames: 555 -> 494.)
-__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __host__ __device__ constexpr uint32_t tmem_cols_for(int cols) {
     return cols <= 32 ? 32u : cols <= 64 ? 64u : cols <= 128 ? 128u : cols <= 256 ? 256u : 512u;
 }
@@ -1126,29 +1115,13 @@ bool encode_planar(CUtensorMap* map, const void* base, int C, int W, int H, int 
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launches a kernel of a pass after the one before it on the stream (pdl_wait_previous).
-template <class... P, class... A>
-bool launch_next(void (*kernel)(P...), int grid, int threads, uint32_t smem, cudaStream_t s, const A&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
-}
-
 template <int CIN, int N, int EPI>
 bool launch_conv(const rz_upsampler* u, const ConvArgs& a, cudaStream_t s) {
     CUtensorMap map;
     if (!encode_planar(&map, a.in, CIN, a.W, a.H)) return false;
     const int tiles = ((a.W + kTileOut - 1) / kTileOut) * ((a.H + kTileRows - 1) / kTileRows);
     const int grid = std::min(tiles, std::max(u->sms, 1));
-    return launch_next(k_conv<CIN, N, EPI>, grid, kConvThreads, ConvSmem<CIN, N>::BYTES, s, a, map);
+    return rz::launch_next(k_conv<CIN, N, EPI>, grid, kConvThreads, ConvSmem<CIN, N>::BYTES, s, a, map);
 }
 
 template <int CIN, int N>
@@ -1157,7 +1130,7 @@ bool launch_wgrad(const rz_upsampler* u, const WgradArgs& a, const __nv_bfloat16
     if (!encode_planar(&x_map, x, CIN, a.W, a.H) || !encode_planar(&dy_map, dy, N, a.W, a.H, kWgKP)) return false;
     const int tiles = ((a.W + kWgKP - 1) / kWgKP) * ((a.H + kWgRows - 1) / kWgRows);
     const int grid = std::min(tiles, std::max(u->sms, 1));
-    return launch_next(k_wgrad<CIN, N>, grid, kWgThreads, WgSmem<CIN, N>::BYTES, s, a, x_map, dy_map);
+    return rz::launch_next(k_wgrad<CIN, N>, grid, kWgThreads, WgSmem<CIN, N>::BYTES, s, a, x_map, dy_map);
 }
 
 bool gbuffer_ok(const rz_upsampler* u, const rz_gbuffer* g) {

@@ -393,6 +393,37 @@ def test_shading_error_against_fp64_oracle(gpu, oracle):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shadow,samples", [(64, 1), (2880, 1), (2896, 1), (2880, 4)])
+def test_frames_in_a_row_around_32_mb_of_targets(gpu, oracle, shadow, samples):
+    """Setup and raster start as the launch before them ends where the depth targets take at most
+    32 MB: frames in a row, each other's leftovers in the targets, on both sides of that."""
+    from rosy_gb300.graphics import Graphics
+
+    s = sc.scene_scale(seed=5, meshes=6, triangles_per_mesh=256, materials=3, texture_size=32, width=97, height=65,
+                       shadow_size=shadow, frames=4)
+    s.samples = samples
+    g = Graphics()
+    g.init(s.width, s.height, s.shadow_size, samples=samples)
+    try:
+        g.set_asset(s)
+        g.set_graphic_objects(s.objects, s.surfaces)
+        g.set_draw_config(s.draw_config)
+        for cam in (0, 1, 2, 3, 1):
+            g.update(s.cameras[cam])
+            g.render()
+            if cam == 0 and g.sync_code() == 14:
+                g.render()
+        g.sync()
+        s.scene = s.cameras[1]
+        ref, out = oracle.render(s), g.download()
+        assert np.array_equal(out["ids"], ref["ids"])
+        assert np.array_equal(out["shadow"].view(np.uint32), ref["shadow"].view(np.uint32))
+        assert np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32)).max() <= COLOR_TOL
+    finally:
+        g.deinit()
+
+
+@pytest.mark.gpu
 def test_read_back_with_frames_in_flight(gpu, oracle):
     """Frames read back through rz_read_frame while the next ones render (two
     host buffers, rz_read_sync before refilling one): every buffer holds its own
