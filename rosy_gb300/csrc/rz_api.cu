@@ -1018,6 +1018,30 @@ int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh
     }
     // the per-draw constants and the clear in one launch
     launch_prep_camera(c->d_opaque_draws, c->opaque_draw_count, c->d_objects, c->d_views, c->d_camera_consts, s, &cl, c->sm_count);
+    // the blended list's setup and vertex stage, and the overlay's segments: only k_blend needs
+    // them, so outside stage timing they follow the vertex stage on its branch instead of
+    // standing between the camera raster and the shading (1279x717, 12,288 blended triangles:
+    // 106.1 -> 104.5 us; latency-bound launches that overlap the rasters)
+    auto blended = [&](cudaStream_t b) {
+        if (c->blended_tris) {
+            launch_prep_camera(c->d_blended_draws, c->blended_draw_count, c->d_objects, c->d_views, c->d_blended_consts, b);
+            launch_setup(pass_params(c, 2), b);
+            launch_blend_boxes(c->blended_pass.records, &c->d_report->blended, c->blended_pass.record_capacity,
+                               c->blended_pass.boxes, b);
+            ShadeParams bs = sh;
+            bs.draws = c->d_blended_draws;
+            bs.draw_count = c->blended_draw_count;
+            bs.draw_table = c->d_draw_tables + c->table_at[2];
+            bs.varying_table = c->d_draw_tables + c->table_at[4];
+            bs.consts = c->d_blended_consts;
+            bs.varying_count = c->varying_count;
+            bs.tri_refs = c->d_tri_refs + c->opaque_tris;
+            launch_vertex_range(bs, c->blended_varying_base, b);
+        }
+        if (c->debug_count)
+            launch_debug_prep(c->d_debug_pairs, c->debug_count, c->d_debug_objects, c->d_views, (uint32_t)c->views.size(),
+                              c->d_debug_segs, c->d_debug_boxes, b);
+    };
     // the vertex stage needs only the per-draw constants: outside stage timing it
     // runs on a branch of its own beside the camera pass's setup and raster
     const bool vtx_branch = !stamps;
@@ -1025,6 +1049,7 @@ int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh
         cudaEventRecord(c->vtx_fork, s);
         cudaStreamWaitEvent(c->vtx, c->vtx_fork, 0);
         launch_vertex(sh, c->vtx);
+        blended(c->vtx);
         cudaEventRecord(c->vtx_join, c->vtx);
     }
     if (stamps) stamp(c, 4);
@@ -1045,21 +1070,7 @@ int enqueue_camera(rz_ctx* c, cudaStream_t s, bool stamps, const ShadeParams& sh
     }
     if (vtx_branch) cudaStreamWaitEvent(s, c->vtx_join, 0);
     else launch_vertex(sh, s);
-    if (c->blended_tris) {
-        launch_prep_camera(c->d_blended_draws, c->blended_draw_count, c->d_objects, c->d_views, c->d_blended_consts, s);
-        launch_setup(pass_params(c, 2), s);
-        launch_blend_boxes(c->blended_pass.records, &c->d_report->blended, c->blended_pass.record_capacity,
-                           c->blended_pass.boxes, s);
-        ShadeParams bs = sh;
-        bs.draws = c->d_blended_draws;
-        bs.draw_count = c->blended_draw_count;
-        bs.draw_table = c->d_draw_tables + c->table_at[2];
-        bs.varying_table = c->d_draw_tables + c->table_at[4];
-        bs.consts = c->d_blended_consts;
-        bs.varying_count = c->varying_count;
-        bs.tri_refs = c->d_tri_refs + c->opaque_tris;
-        launch_vertex_range(bs, c->blended_varying_base, s);
-    }
+    if (!vtx_branch) blended(s);
     return RZ_OK;
 }
 
@@ -1164,9 +1175,6 @@ int enqueue_frame(rz_ctx* c) {
     if (c->batched || c->blended_tris || c->timing || c->debug_count) launch_shade(sh, s);
     if (sources && !sources_side) launch_subpixel_sources(sh, s);
     if (c->blended_tris || c->debug_count) {
-        if (c->debug_count)
-            launch_debug_prep(c->d_debug_pairs, c->debug_count, c->d_debug_objects, c->d_views, (uint32_t)c->views.size(),
-                              c->d_debug_segs, c->d_debug_boxes, s);
         BlendParams bp{};
         bp.sh = sh;
         bp.sh.draws = c->d_blended_draws;
