@@ -799,15 +799,10 @@ int build_layout(rz_ctx* c) {
         RZ_CUDA(c, cudaMemcpy(c->d_opaque_draws, opaque.data(), opaque.size() * sizeof(DrawRec), cudaMemcpyHostToDevice), "upload draws");
     if (!blended.empty())
         RZ_CUDA(c, cudaMemcpy(c->d_blended_draws, blended.data(), blended.size() * sizeof(DrawRec), cudaMemcpyHostToDevice), "upload draws");
-    // entry g: the last draw whose first triangle (or varying record) is at most 256 g
     std::vector<uint32_t> tables;
     auto add_table = [&](int which, const std::vector<DrawRec>& list, uint64_t end, uint32_t DrawRec::*base) {
         c->table_at[which] = tables.size();
-        uint32_t d = 0;
-        for (uint64_t at = 0; at < std::max<uint64_t>(end, 1); at += 256) {
-            while (d + 1 < list.size() && list[d + 1].*base <= at) ++d;
-            tables.push_back(d);
-        }
+        add_draw_table(tables, (uint32_t)list.size(), end, [&](uint32_t d) { return list[d].*base; });
     };
     add_table(0, shadow_list, shadow_tris, &DrawRec::tri_base);
     add_table(1, opaque, opaque_tris, &DrawRec::tri_base);

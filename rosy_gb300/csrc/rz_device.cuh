@@ -36,26 +36,12 @@ __device__ __forceinline__ float4 transform_point(const float* __restrict__ M, f
     return o;
 }
 
-// Index of the draw whose triangle range holds `tri` (draws sorted by tri_base).
-__device__ __forceinline__ uint32_t find_draw(const DrawRec* __restrict__ draws, uint32_t n, uint32_t tri) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(&draws[mid].tri_base) <= tri) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// The same from a table of the draw that holds triangle 256 g (entry g), built with
-// the draw list: one load and as many steps as draws start between there and `tri`,
-// mostly none, where the search of 1,024 draws is a chain of ten dependent loads.
+// The draw that holds triangle `tri`, from the list's table; null: of the list's n draws.
 __device__ __forceinline__ uint32_t draw_from(const DrawRec* __restrict__ draws, uint32_t n, const uint32_t* __restrict__ table,
                                               uint32_t tri) {
-    if (!table) return find_draw(draws, n, tri);
-    uint32_t d = __ldg(&table[tri >> 8]);
-    while (d + 1 < n && __ldg(&draws[d + 1].tri_base) <= tri) ++d;
-    return d;
+    const auto base = [&](uint32_t d) { return __ldg(&draws[d].tri_base); };
+    if (!table) return draw_between(0u, n - 1u, tri, base);
+    return draw_in_table(tri, [&](uint32_t g) { return __ldg(&table[g]); }, base);
 }
 
 // Thread `tid` of `stride` threads' share of zeroing n bytes at ptr: 16-byte

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "../../include/rosy_gb300.h"
+#include "rz_draws.h"
 
 namespace rz {
 

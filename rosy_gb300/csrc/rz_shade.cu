@@ -755,8 +755,8 @@ __global__ void __launch_bounds__(256) k_vertex(ShadeParams P, uint32_t first) {
     const uint32_t lane = threadIdx.x & 31u;
     float4 (*const rec)[kVaryingF4] = s_rec[threadIdx.x >> 5];
     if (i < P.varying_count) {
-        uint32_t d = __ldg(&P.varying_table[i >> 8]);
-        while (d + 1 < P.draw_count && __ldg(&P.draws[d + 1].varying_base) <= i) ++d;
+        const uint32_t d = draw_in_table(i, [&](uint32_t g) { return __ldg(&P.varying_table[g]); },
+                                         [&](uint32_t k) { return __ldg(&P.draws[k].varying_base); });
         const DrawRec dr = P.draws[d];
         const DrawConsts& dc = P.consts[d];
         const rz_object& gd = P.objects[dr.object];
