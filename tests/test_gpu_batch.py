@@ -1,6 +1,8 @@
 """Batched views: several scenes and views of uneven size rendered by one
 rz_render (one launch per stage over all views); every view must match the
 oracle rendering that view alone, bit-exactly for visibility/depth/shadow."""
+import time
+
 import numpy as np
 import pytest
 
@@ -118,3 +120,43 @@ def test_batch_with_msaa_cascades_and_blending(gpu, oracle):
         assert np.array_equal(out["shadow"].view(np.uint32), ref["shadow"].view(np.uint32))
         d = np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32))
         assert d.max() <= 1, d.max()
+
+
+@pytest.mark.gpu
+def test_multisampled_views_one_at_a_time(gpu):
+    """Per-view launches with 4 samples: the batch's ids and colours; and the parts of a view's raster run side by
+    side, so that the frame stays below 2.3 times the single-sampled one (with one raster per sample over all its
+    records it was 2.25 times; with the parts one after the other 3.2)."""
+    s = sc.scene_scale(seed=1, meshes=8, triangles_per_mesh=1024, materials=2, texture_size=64, width=256, height=256,
+                       shadow_size=256, frames=1)
+    views = [sc.view_of(s, 200 + 7 * i, 200 - 3 * i, 256) for i in range(16)]
+    ms, outs = {}, {}
+    for samples in (1, 4):
+        g = Graphics()
+        g.init(64, 64, 256, samples=samples)
+        try:
+            g.add_scene(s)
+            g.set_views([(0, v.width, v.height, v.shadow_size, v.draw_config) for v in views])
+            for i, v in enumerate(views):
+                g.update_view(i, v.scene)
+            for batched in (True, False):
+                g.set_tuning(batched=batched)
+                for _ in range(2):
+                    g.render()
+                    while g.sync_code() == 14:
+                        g.render()
+                outs[samples, batched] = [g.download_view(i) for i in range(len(views))]
+            times = []
+            for _ in range(5):
+                t0 = time.perf_counter()
+                for _ in range(20):
+                    g.render()
+                g.sync()
+                times.append(time.perf_counter() - t0)
+            ms[samples] = min(times) * 50
+        finally:
+            g.deinit()
+    for samples in (1, 4):
+        for a, b in zip(outs[samples, True], outs[samples, False]):
+            assert np.array_equal(a["ids"], b["ids"]) and np.array_equal(a["color"], b["color"])
+    assert ms[4] < 2.3 * ms[1], ms
