@@ -734,6 +734,16 @@ __device__ __forceinline__ uint32_t encode_unorm8(float c) {
 }
 __device__ __forceinline__ float half_round(float x) { return __half2float(__float2half_rn(x)); }
 
+// A value of the RGBA16F draw image.
+__device__ __forceinline__ uint2 pack_rgba16(float r, float g, float b, float a) {
+    const __half2 rg = __floats2half2_rn(r, g), ba = __floats2half2_rn(b, a);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&rg), *reinterpret_cast<const uint32_t*>(&ba));
+}
+__device__ __forceinline__ float4 unpack_rgba16(uint2 v) {
+    const float2 rg = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), ba = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+    return make_float4(rg.x, rg.y, ba.x, ba.y);
+}
+
 // Varying record of one (draw, vertex): the vertex-stage outputs the fragment
 // stage reads plus the clip position, 32 floats:
 //   0-2 normal, 3-5 viewDir, 6-8 lightDir, 9-11 tangent, 12 sigma, 13 color.a,
@@ -1464,6 +1474,11 @@ void launch_subpixel_sources(const ShadeParams& p, cudaStream_t stream) {
 // to 113 us with the cheaper fragment stage, and to 91 us with the prepared records and
 // the overlay's boxes. What is left is the latency of the fullest tiles and of the
 // five loads that a tile waits for one after the other.
+// Three CTAs per SM of 80 registers, and a pixel's values packed as they are stored: with
+// five of 48 the fragment stage spilled, and deep overdraw was slower than fragments shaded
+// where they are met (100 triangles across 640x360: 376 us a frame, 471 without the BRDF;
+// 294 and 287 shaded so; 276 and 288 with three). The frame above takes 87 us with three or
+// five, 85 with four, which lose on deep overdraw (290 and 341).
 constexpr int kBlendBatch = 512;   // group boxes (or overlay segments) tested at a time
 constexpr int kBlendList = 256;    // records of a tile prepared at a time
 constexpr int kBlendRound = 4;     // fragments a pixel collects before the tile shades them
@@ -1691,7 +1706,7 @@ __device__ __forceinline__ void shade_fragments(const ShadeParams& P, const View
 }
 
 template <bool kMsaa>
-__global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
+__global__ void __launch_bounds__(256, 3) k_blend(const __grid_constant__ BlendParams B) {
     constexpr int kSamples = kMsaa ? kMsaaSamples : 1;
     __shared__ float s_srgb[256];
     __shared__ uint32_t s_list[kBlendBatch];  // groups (or overlay segments) that meet the tile
@@ -1753,15 +1768,6 @@ __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
     else if (tid < 32) s_ndc.y[tid - 16] = ndc(ty0 + tid - 16, VR.height);
     any = __syncthreads_or(any) != 0;
     const bool lit = any && lit_view(*VR.scene);
-    float col[kSamples][4];
-#pragma unroll
-    for (int k = 0; k < kSamples; ++k) {
-        const __half2 rg = *reinterpret_cast<const __half2*>(&held[k].x), ba = *reinterpret_cast<const __half2*>(&held[k].y);
-        col[k][0] = __low2float(rg);
-        col[k][1] = __high2float(rg);
-        col[k][2] = __low2float(ba);
-        col[k][3] = __high2float(ba);
-    }
     for (uint32_t first = 0; any && first < groups; first += kBlendBatch) {
         const uint32_t ngroups = compact_batch<kBlendBatch / 256>(first, groups, tid, s_list, s_count[0], [&](uint32_t g) {
             const uint4 b = __ldg(&B.boxes[g]);
@@ -1881,13 +1887,12 @@ __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
                     const uint32_t i = (uint32_t)(slots >> (16 * r)) & 0xffffu;
                     if (s_id[i] == 0u) continue;  // discarded
                     const float4 o = s_out[i];
-                    const float s4[3] = {o.x, o.y, o.z}, a = o.w;
+                    const float a = o.w;
 #pragma unroll
                     for (int k = 0; k < kSamples; ++k) {
                         if (!((pass_of >> (4 * r + k)) & 1u)) continue;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) col[k][c] = half_round(s4[c] * a + col[k][c] * (1.0f - a));
-                        col[k][3] = half_round(a);
+                        const float4 d = unpack_rgba16(held[k]);
+                        held[k] = pack_rgba16(o.x * a + d.x * (1.0f - a), o.y * a + d.y * (1.0f - a), o.z * a + d.z * (1.0f - a), a);
                     }
                 }
                 more = __syncthreads_or(open != 0u || next < mine) != 0;
@@ -1922,9 +1927,7 @@ __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
 #pragma unroll
                     for (int k = 0; k < kSamples; ++k) {
                         if (!(pass & (1u << k))) continue;
-#pragma unroll
-                        for (int i = 0; i < 3; ++i) col[k][i] = half_round(sg.rgb[i]);
-                        col[k][3] = 1.0f;
+                        held[k] = pack_rgba16(sg.rgb[0], sg.rgb[1], sg.rgb[2], 1.0f);
                     }
                 }
             }
@@ -1932,13 +1935,13 @@ __global__ void __launch_bounds__(256, 5) k_blend(BlendParams B) {
         }
     }
     if (!inside) return;
-    float o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if constexpr (kMsaa) o[i] = resolve4(col[0][i], col[1][i], col[2][i], col[3][i]);
-        else o[i] = col[0][i];
+    float4 o = unpack_rgba16(held[0]);
+    if constexpr (kMsaa) {
+        const float4 o1 = unpack_rgba16(held[1]), o2 = unpack_rgba16(held[2]), o3 = unpack_rgba16(held[3]);
+        o = make_float4(resolve4(o.x, o1.x, o2.x, o3.x), resolve4(o.y, o1.y, o2.y, o3.y), resolve4(o.z, o1.z, o2.z, o3.z),
+                        resolve4(o.w, o1.w, o2.w, o3.w));
     }
-    VR.color[p] = encode_srgb8(o[0]) | (encode_srgb8(o[1]) << 8) | (encode_srgb8(o[2]) << 16) | (encode_unorm8(o[3]) << 24);
+    VR.color[p] = encode_srgb8(o.x) | (encode_srgb8(o.y) << 8) | (encode_srgb8(o.z) << 16) | (encode_unorm8(o.w) << 24);
 }
 
 void launch_blend_boxes(const TriRecord* records, const PassHeader* header, uint32_t capacity, uint4* boxes,

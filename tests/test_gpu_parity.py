@@ -407,7 +407,7 @@ def frame_ms(s):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("triangles,spread,most", [(400, 0.6, 1.17)])
+@pytest.mark.parametrize("triangles,spread,most", [(400, 0.6, 1.17), (100, 2.0, 1.1)])
 def test_simple_lighting_is_not_slower(gpu, triangles, spread, most):
     """The fragment stage's copy for views without the BRDF does less arithmetic than the one with it, so deep
     overdraw by large blended triangles takes no longer but for what its register spills cost."""
