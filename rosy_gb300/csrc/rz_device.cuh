@@ -106,7 +106,8 @@ __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return fma2(a, b, F2{c_min
 // depend on it. It waits in pdl_wait_previous for the one before to be complete and its
 // writes visible, before it touches what that one computes. Where every kernel of a chain
 // waits so, one that gets past this point comes after all the earlier ones. The first
-// kernel of a chain is launched normally, after all that the stream holds. (957x539
+// kernel of a chain is launched normally, after all that the stream holds. A kernel that
+// allocates tensor memory lets the next one in after that, and the wait comes later still. (957x539
 // upsampler inference, five kernels: 78 -> 64 us; a training step of two 960x540 frames:
 // 555 -> 494. Frames: see chained in rz_api.cu.)
 __device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
