@@ -202,19 +202,22 @@ __device__ __forceinline__ int64_t area2(const SV& a, const SV& b, const SV& c) 
     return (int64_t)(b.X - a.X) * (int64_t)(c.Y - a.Y) - (int64_t)(c.X - a.X) * (int64_t)(b.Y - a.Y);
 }
 
-// Whether a camera record's stamps lie on the grid of the target's 8x4 blocks, so that
-// each has a block's depth to be tested against (see raster_front): where the row and the
-// column that this may add are few of many. (24x12 or 16x8 pixels gain nothing on deep
+// Whether a record's stamps lie on the grid of the target's 8x4 blocks, so that each has a
+// block's depth to be tested against (see raster_front): in passes with block depths
+// (PassParams::front, asked by the setup that counts the stamps and by the raster that takes
+// them), where the row and the column that this may add are few of many. (24x12 or 16x8 pixels gain nothing on deep
 // overdraw and cost a mesh scene up to 0.4 % more; 64x32 lose 3 % of a soup's frame.
 // Shadow passes have no grid: what they gained was within the noise, and scene-scale
 // frames lost 2 %.)
 constexpr int kGridW = 32, kGridH = 16;
-__device__ __forceinline__ bool on_grid(int px0, int py0, int px1, int py1) { return px1 - px0 >= kGridW - 1 && py1 - py0 >= kGridH - 1; }
+__device__ __forceinline__ bool on_grid(const PassParams& P, int px0, int py0, int px1, int py1) {
+    return P.front != nullptr && px1 - px0 >= kGridW - 1 && py1 - py0 >= kGridH - 1;
+}
 
 // A record's stamps: how many in a row (nsx) and in all.
-__device__ __forceinline__ uint32_t record_stamps(const TriRecord& r, bool camera, uint32_t& nsx) {
+__device__ __forceinline__ uint32_t record_stamps(const PassParams& P, const TriRecord& r, uint32_t& nsx) {
     const int px0 = r.p0 & 0xffff, py0 = r.p0 >> 16, px1 = r.p1 & 0xffff, py1 = r.p1 >> 16;
-    const int m = camera && on_grid(px0, py0, px1, py1) ? -1 : 0;
+    const int m = on_grid(P, px0, py0, px1, py1) ? -1 : 0;
     nsx = (uint32_t)((px1 - px0 + (px0 & m & (kStampW - 1))) / kStampW + 1);
     return nsx * (uint32_t)((py1 - py0 + (py0 & m & (kStampH - 1))) / kStampH + 1);
 }
@@ -434,6 +437,7 @@ __device__ __forceinline__ void store_record(TriRecord* dst, const TriRecord& r)
 
 // Phase A: count the records (small and large) a triangle produces.
 struct CountEmit {
+    const PassParams* P;
     uint32_t recs = 0;     // large
     uint64_t stamps = 0;   // of the large ones
     uint32_t small = 0;
@@ -459,7 +463,7 @@ struct CountEmit {
         }
         ++recs;
         uint32_t nsx;
-        stamps += record_stamps(r, refs != nullptr, nsx);
+        stamps += record_stamps(*P, r, nsx);
     }
 };
 
@@ -484,7 +488,7 @@ struct WriteEmit {
             return;
         }
         uint32_t nsx;
-        const uint64_t end = stamp + record_stamps(r, P->tri_refs != nullptr, nsx);
+        const uint64_t end = stamp + record_stamps(*P, r, nsx);
         r.view |= large_facts(r, P->bb_hi) << kRecFlagShift;
         r.stamp_offset = stamp | ((uint64_t)nsx << kStampOffsetBits);
         store_record(P->records + rec, r);
@@ -549,7 +553,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
     const uint32_t local = tile * kSetupThreads + threadIdx.x;
     const uint32_t tri = P.tri_offset + local;
 
-    CountEmit cnt;
+    CountEmit cnt{&P};
     cnt.refs = P.tri_refs;
     cnt.tri = tri;
     if (local < P.tri_total) setup_triangle(P, tri, cnt);
@@ -870,8 +874,8 @@ struct LargeRecord {
 };
 
 // Decodes a large record from its four 16-byte words.
-template <bool kCamera>
-__device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const int4 q2, const int4 q3, LargeRecord& L) {
+template <bool kCamera>  // only the camera raster has block depths
+__device__ __forceinline__ void decode_large(const PassParams& P, const int4 q0, const int4 q1, const int4 q2, const int4 q3, LargeRecord& L) {
     L.X[0] = q0.x;
     L.Y[0] = q0.y;
     L.X[1] = q0.z;
@@ -887,7 +891,7 @@ __device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const
     L.px1 = q2.w & 0xffff;
     L.py1 = (uint32_t)q2.w >> 16;
     L.id = (uint32_t)q3.x;
-    L.grid = kCamera && on_grid(L.px0, L.py0, L.px1, L.py1);
+    L.grid = kCamera && on_grid(P, L.px0, L.py0, L.px1, L.py1);
     if (L.grid) {
         L.px0 &= -kStampW;
         L.py0 &= -kStampH;
@@ -910,9 +914,9 @@ __device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const
 }
 
 template <bool kCamera>
-__device__ __forceinline__ void load_large(const TriRecord* rec, LargeRecord& L) {
+__device__ __forceinline__ void load_large(const PassParams& P, const TriRecord* rec, LargeRecord& L) {
     const int4* src = reinterpret_cast<const int4*>(rec);
-    decode_large<kCamera>(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3), L);
+    decode_large<kCamera>(P, __ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3), L);
 }
 
 // Record staging of the chunk walk: a warp copies the records a chunk starts
@@ -1172,8 +1176,8 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
             LargeRecord L;
             if (s + lane < s_end && r < n_rec) {
                 const uint32_t j = r - r_cur;
-                if (j < (uint32_t)kStageRecords) decode_large<kWriteId>(st[j][0], st[j][1], st[j][2], st[j][3], L);
-                else load_large<kWriteId>(P.records + r, L);
+                if (j < (uint32_t)kStageRecords) decode_large<kWriteId>(P, st[j][0], st[j][1], st[j][2], st[j][3], L);
+                else load_large<kWriteId>(P, P.records + r, L);
                 if (s + lane >= L.begin && s + lane < L.end) {
                     // stamp i of the record, below 2^24: the quotient by stamps per row, off by one at most
                     const int i = (int)(s + lane - L.begin), nsx = (int)L.nsx;
@@ -1220,7 +1224,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
             else raster_stamps<kWriteId, kSamples, false>(P, work, __popc(left), heads, 0u, lane, lx, ly);
             for (uint32_t m = __ballot_sync(kAllLanes, far); m; m &= m - 1) {
                 const int j = __ffs(m) - 1;
-                load_large<kWriteId>(P.records + __shfl_sync(kAllLanes, r, j), L);
+                load_large<kWriteId>(P, P.records + __shfl_sync(kAllLanes, r, j), L);
                 const int px = __shfl_sync(kAllLanes, sx0, j) + lx, py = __shfl_sync(kAllLanes, sy0, j) + ly;
                 const Target T = view_target<kWriteId>(P, L.view);
                 const size_t plane = kMsaa ? plane_words(P, L.view) : 0;

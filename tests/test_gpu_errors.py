@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from kat_scenes import flat_scene
 from rosy_gb300 import scene as sc
 from rosy_gb300._lib import RzError
 from rosy_gb300.graphics import Graphics
@@ -109,5 +110,27 @@ def test_launch_count_is_exact(gpu, samples):
             g.render()
             g.sync()
             assert g.stats().kernel_launches == expected
+    finally:
+        g.deinit()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("blended", [1])
+def test_work_queue_of_the_stamps_a_frame_needs(gpu, blended):
+    """A triangle whose box of 32x16 pixels starts at no block's corner: 16 stamps of 8x4 pixels, a queue of two
+    chunks of eight."""
+    s = flat_scene([[(7.25, 3.25, 0.5), (7.25, 18.75, 0.5), (38.75, 18.75, 0.5)]], W=64, H=32)
+    s.surfaces["blended"] = blended
+    g = Graphics()
+    g.init(s.width, s.height, s.shadow_size)
+    try:
+        g.set_asset(s)
+        g.set_graphic_objects(s.objects, s.surfaces)
+        g.set_draw_config(s.draw_config)
+        g.set_tuning(chunk_stamps=8, small_extent=8, queue_chunks=2)
+        g.update(s.scene)
+        g.render()
+        assert g.sync_code() == 0
+        assert (g.download()["color"][4:18, 8:38] != g.download()["color"][0, 63]).any()
     finally:
         g.deinit()
