@@ -282,12 +282,16 @@ void free_pass(PassBuffers& p) {
 }
 
 // Sizes the raster scratch of a pass: one record per triangle plus room for
-// clipped fans, and a chunk map for `stamps_hint` stamps.
-int size_pass(rz_ctx* c, PassBuffers& p, uint32_t tris, uint64_t stamps_hint) {
+// clipped fans, and a chunk map for `stamps_hint` stamps. `grid`: the stamps of large
+// records lie on the block grid, which gives a box of 32x16 pixels or more up to a row
+// and a column more of them, 25 for 16 at most: the queue holds that many more, so that
+// it is as deep in stamps counted from the boxes' corners as the other passes' queues.
+int size_pass(rz_ctx* c, PassBuffers& p, uint32_t tris, uint64_t stamps_hint, bool grid = false) {
     const uint32_t rec_cap = tris + tris / 4 + 4096;
     const uint32_t tiles = (uint32_t)setup_ctas(tris) + 1;
     uint64_t chunks = (stamps_hint + c->chunk_stamps - 1) / c->chunk_stamps + 1024;
     if (c->queue_chunks) chunks = c->queue_chunks;
+    if (grid) chunks += (9 * chunks + 15) / 16;
     if (chunks > 0xFFFFFFFFull) chunks = 0xFFFFFFFFull;
     if (rec_cap > p.record_capacity) {
         dfree(p.records);
@@ -823,7 +827,7 @@ int build_layout(rz_ctx* c) {
     c->shadow_total = shadow;
     c->shade_blocks = blocks;
     int rc = size_pass(c, c->shadow_pass, c->shadow_tris, stamp_hint(c->shadow_tris, shadow));
-    if (rc == RZ_OK) rc = size_pass(c, c->camera_pass, c->opaque_tris, stamp_hint(c->opaque_tris, pix));
+    if (rc == RZ_OK) rc = size_pass(c, c->camera_pass, c->opaque_tris, stamp_hint(c->opaque_tris, pix), true);
     if (rc == RZ_OK && c->blended_tris) rc = size_pass(c, c->blended_pass, c->blended_tris, stamp_hint(c->blended_tris, pix));
     if (rc == RZ_OK && c->blended_tris) rc = size_boxes(c, c->blended_pass);
     if (rc != RZ_OK) return rc;

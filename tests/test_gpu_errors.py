@@ -115,7 +115,7 @@ def test_launch_count_is_exact(gpu, samples):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("blended", [1])
+@pytest.mark.parametrize("blended", [1, 0])
 def test_work_queue_of_the_stamps_a_frame_needs(gpu, blended):
     """A triangle whose box of 32x16 pixels starts at no block's corner: 16 stamps of 8x4 pixels, a queue of two
     chunks of eight."""
