@@ -188,9 +188,9 @@ struct PassParams {
     void* clear_ptr[2];
     size_t clear_bytes[2];
     uint32_t clear_count;
-    // opaque camera pass (else null, and no record's stamps lie on the block grid): per 8x4
-    // block of the visibility, eight to a 16x16 shading tile, a depth that every pixel of the
-    // block reaches (bits; see raster_front)
+    // opaque camera pass (the unordered one with tri_refs), else null: per 8x4 block of the
+    // visibility, eight to a 16x16 shading tile, a depth that every pixel of the block reaches
+    // (bits; see raster_front)
     uint32_t* front;
     // camera passes only (else null): per triangle with valid indices, its draw's
     // material and its three varying record indices, for the shading

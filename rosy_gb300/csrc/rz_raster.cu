@@ -203,21 +203,21 @@ __device__ __forceinline__ int64_t area2(const SV& a, const SV& b, const SV& c) 
 }
 
 // Whether a record's stamps lie on the grid of the target's 8x4 blocks, so that each has a
-// block's depth to be tested against (see raster_front): in passes with block depths
-// (PassParams::front, asked by the setup that counts the stamps and by the raster that takes
-// them), where the row and the column that this may add are few of many. (24x12 or 16x8 pixels gain nothing on deep
-// overdraw and cost a mesh scene up to 0.4 % more; 64x32 lose 3 % of a soup's frame.
-// Shadow passes have no grid: what they gained was within the noise, and scene-scale
-// frames lost 2 %.)
+// block's depth to be tested against (see raster_front): in the opaque camera pass, the one
+// unordered pass with triangle references and the one that k_raster takes with ids
+// (launch_raster sees to it), where the row and the column that this may add are few of many. (24x12
+// or 16x8 pixels gain nothing on deep overdraw and cost a mesh scene up to 0.4 % more; 64x32
+// lose 3 % of a soup's frame. Shadow passes have no grid: what they gained was within the noise,
+// and scene-scale frames lost 2 %.)
 constexpr int kGridW = 32, kGridH = 16;
-__device__ __forceinline__ bool on_grid(const PassParams& P, int px0, int py0, int px1, int py1) {
-    return P.front != nullptr && px1 - px0 >= kGridW - 1 && py1 - py0 >= kGridH - 1;
+__device__ __forceinline__ bool on_grid(bool camera, int px0, int py0, int px1, int py1) {
+    return camera && px1 - px0 >= kGridW - 1 && py1 - py0 >= kGridH - 1;
 }
 
 // A record's stamps: how many in a row (nsx) and in all.
-__device__ __forceinline__ uint32_t record_stamps(const PassParams& P, const TriRecord& r, uint32_t& nsx) {
+__device__ __forceinline__ uint32_t record_stamps(const TriRecord& r, bool camera, uint32_t& nsx) {
     const int px0 = r.p0 & 0xffff, py0 = r.p0 >> 16, px1 = r.p1 & 0xffff, py1 = r.p1 >> 16;
-    const int m = on_grid(P, px0, py0, px1, py1) ? -1 : 0;
+    const int m = on_grid(camera, px0, py0, px1, py1) ? -1 : 0;
     nsx = (uint32_t)((px1 - px0 + (px0 & m & (kStampW - 1))) / kStampW + 1);
     return nsx * (uint32_t)((py1 - py0 + (py0 & m & (kStampH - 1))) / kStampH + 1);
 }
@@ -315,7 +315,7 @@ __device__ __forceinline__ int make_record(const SV& v0, const SV& v1, const SV&
 }
 
 // Runs the fixed-function front end for one triangle and hands each record to `emit`.
-template <class Emit>
+template <bool kOrdered, class Emit>
 __device__ __forceinline__ void setup_triangle(const PassParams& P, uint32_t tri, Emit& emit) {
     const uint32_t d = draw_from(P.draws, P.draw_count, P.draw_table, tri);
     const DrawRec dr = P.draws[d];
@@ -338,7 +338,7 @@ __device__ __forceinline__ void setup_triangle(const PassParams& P, uint32_t tri
     const bool msaa = P.write_id && VR.samples > 1;
     V.bb_lo = msaa ? 224 : 128;
     V.bb_hi = msaa ? 32 : 128;
-    V.cull_front = P.ordered ? 0 : VR.cull_front;
+    V.cull_front = kOrdered ? 0 : VR.cull_front;
     V.ccw_front = VR.ccw_front;
     V.bias_enabled = P.write_id ? 0 : VR.bias_enabled;
     V.bias_constant = VR.bias_constant;
@@ -398,7 +398,7 @@ __device__ __forceinline__ void setup_triangle(const PassParams& P, uint32_t tri
             c.z = v[2].z / v[2].w;
         }
         TriRecord r;
-        const int kind = S > 0 ? make_record(a, b, c, S, V, P.ordered != 0, P.small_extent, id, r) : make_record(a, c, b, -S, V, P.ordered != 0, P.small_extent, id, r);
+        const int kind = S > 0 ? make_record(a, b, c, S, V, kOrdered, P.small_extent, id, r) : make_record(a, c, b, -S, V, kOrdered, P.small_extent, id, r);
         if (kind) emit(r, kind == 2);
         return;
     }
@@ -422,8 +422,8 @@ __device__ __forceinline__ void setup_triangle(const PassParams& P, uint32_t tri
         const int64_t si = area2(sv[0], sv[i], sv[i + 1]);
         if (si == 0 || ((si > 0) != (S > 0))) continue;
         TriRecord r;
-        const int kind = si > 0 ? make_record(sv[0], sv[i], sv[i + 1], si, V, P.ordered != 0, P.small_extent, id, r)
-                                : make_record(sv[0], sv[i + 1], sv[i], -si, V, P.ordered != 0, P.small_extent, id, r);
+        const int kind = si > 0 ? make_record(sv[0], sv[i], sv[i + 1], si, V, kOrdered, P.small_extent, id, r)
+                                : make_record(sv[0], sv[i + 1], sv[i], -si, V, kOrdered, P.small_extent, id, r);
         if (kind) emit(r, kind == 2);
     }
 }
@@ -436,8 +436,8 @@ __device__ __forceinline__ void store_record(TriRecord* dst, const TriRecord& r)
 }
 
 // Phase A: count the records (small and large) a triangle produces.
+template <bool kOrdered>
 struct CountEmit {
-    const PassParams* P;
     uint32_t recs = 0;     // large
     uint64_t stamps = 0;   // of the large ones
     uint32_t small = 0;
@@ -463,13 +463,14 @@ struct CountEmit {
         }
         ++recs;
         uint32_t nsx;
-        stamps += record_stamps(*P, r, nsx);
+        stamps += record_stamps(r, !kOrdered && refs != nullptr, nsx);
     }
 };
 
 // Phase B: large records at their compacted index with their stamp offsets,
 // small records at their slot in the small list (whose order does not matter:
 // the depth test is an atomic max).
+template <bool kOrdered>
 struct WriteEmit {
     const PassParams* P;
     uint32_t rec;
@@ -488,7 +489,7 @@ struct WriteEmit {
             return;
         }
         uint32_t nsx;
-        const uint64_t end = stamp + record_stamps(*P, r, nsx);
+        const uint64_t end = stamp + record_stamps(r, !kOrdered && P->tri_refs != nullptr, nsx);
         r.view |= large_facts(r, P->bb_hi) << kRecFlagShift;
         r.stamp_offset = stamp | ((uint64_t)nsx << kStampOffsetBits);
         store_record(P->records + rec, r);
@@ -527,6 +528,7 @@ __device__ __forceinline__ uint64_t to_status(uint64_t recs, uint64_t stamps) {
 // and 188 us with a binary search of the draws, nine divisions by w and 64-bit scans;
 // with the draw table, w known to be 1 under the orthographic light, depths divided
 // after culling and ballots for the counts it is 624 instructions and 148 us.
+template <bool kOrdered>
 __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
     __shared__ uint32_t s_tile;
     __shared__ uint64_t s_warp[kSetupThreads / 32];
@@ -544,19 +546,19 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
     // start (a CTA only waits on tiles that have started); the unordered passes
     // wait on nobody and use the block index, sparing one same-address atomic
     // per CTA.
-    if (P.ordered && threadIdx.x == 0) s_tile = atomicAdd(&P.header->ticket, 1u);
+    if (kOrdered && threadIdx.x == 0) s_tile = atomicAdd(&P.header->ticket, 1u);
     const uint32_t tri_ctas = (P.tri_total + kSetupThreads - 1) / kSetupThreads;
     // CTAs launched only to share the zeroing hold no triangles: done
-    if (!P.ordered && blockIdx.x >= tri_ctas) return;
+    if (!kOrdered && blockIdx.x >= tri_ctas) return;
     __syncthreads();
-    const uint32_t tile = P.ordered ? s_tile : blockIdx.x;
+    const uint32_t tile = kOrdered ? s_tile : blockIdx.x;
     const uint32_t local = tile * kSetupThreads + threadIdx.x;
     const uint32_t tri = P.tri_offset + local;
 
-    CountEmit cnt{&P};
+    CountEmit<kOrdered> cnt;
     cnt.refs = P.tri_refs;
     cnt.tri = tri;
-    if (local < P.tri_total) setup_triangle(P, tri, cnt);
+    if (local < P.tri_total) setup_triangle<kOrdered>(P, tri, cnt);
 
     // CTA-wide inclusive scan of (records, stamps) packed in one 64-bit word, and of the
     // small records. Nearly every triangle gives none or one, so that within a warp the
@@ -614,7 +616,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
     // max, so records may land in any order; one 64-bit atomicAdd per CTA
     // allocates its record slots and its stamp range. The ordered blended list
     // keeps submission order with a decoupled look-back instead.
-    if (!P.ordered) {
+    if (!kOrdered) {
         if (threadIdx.x == 0) {
             const uint64_t old =
                 total ? atomicAdd(reinterpret_cast<unsigned long long*>(&P.header->alloc), (unsigned long long)total) : 0ull;
@@ -639,7 +641,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
     }
     // Decoupled look-back (warp 0): publish this tile's aggregate, then sum the
     // predecessors' values 32 at a time until an inclusive prefix is found.
-    if (P.ordered && warp == 0) {
+    if (kOrdered && warp == 0) {
         const uint64_t agg_recs = total >> kStampBits, agg_stamps = total & kStampMask;
         volatile unsigned long long* status = reinterpret_cast<volatile unsigned long long*>(P.tile_status);
         uint64_t pre_recs = 0, pre_stamps = 0;
@@ -702,10 +704,10 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(PassParams P) {
     }
     __syncthreads();
     if (cnt.recs + cnt.small == 0) return;
-    WriteEmit w{&P, (uint32_t)(s_base_recs + (excl >> kStampBits)), s_base_stamps + (excl & kStampMask),
+    WriteEmit<kOrdered> w{&P, (uint32_t)(s_base_recs + (excl >> kStampBits)), s_base_stamps + (excl & kStampMask),
                 s_small_base + small_excl};
     if (cnt.recs + cnt.small == 1) w(cnt.first, cnt.first_small);
-    else setup_triangle(P, tri, w);
+    else setup_triangle<kOrdered>(P, tri, w);
 }
 
 int setup_ctas(uint32_t tri_total) { return (int)((tri_total + kSetupThreads - 1) / kSetupThreads); }
@@ -722,8 +724,9 @@ void launch_setup(const PassParams& p, cudaStream_t stream, bool next) {
         const size_t want = std::min<size_t>(most / 32768, 4096);
         if ((size_t)ctas < want) ctas = (int)want;
     }
-    if (next) launch_next(k_setup, ctas, kSetupThreads, 0, stream, p);
-    else k_setup<<<ctas, kSetupThreads, 0, stream>>>(p);
+    void (*const kernel)(PassParams) = p.ordered ? k_setup<true> : k_setup<false>;
+    if (next) launch_next(kernel, ctas, kSetupThreads, 0, stream, p);
+    else kernel<<<ctas, kSetupThreads, 0, stream>>>(p);
     note_launch();
 }
 
@@ -874,8 +877,8 @@ struct LargeRecord {
 };
 
 // Decodes a large record from its four 16-byte words.
-template <bool kCamera>  // only the camera raster has block depths
-__device__ __forceinline__ void decode_large(const PassParams& P, const int4 q0, const int4 q1, const int4 q2, const int4 q3, LargeRecord& L) {
+template <bool kCamera>
+__device__ __forceinline__ void decode_large(const int4 q0, const int4 q1, const int4 q2, const int4 q3, LargeRecord& L) {
     L.X[0] = q0.x;
     L.Y[0] = q0.y;
     L.X[1] = q0.z;
@@ -891,7 +894,7 @@ __device__ __forceinline__ void decode_large(const PassParams& P, const int4 q0,
     L.px1 = q2.w & 0xffff;
     L.py1 = (uint32_t)q2.w >> 16;
     L.id = (uint32_t)q3.x;
-    L.grid = kCamera && on_grid(P, L.px0, L.py0, L.px1, L.py1);
+    L.grid = on_grid(kCamera, L.px0, L.py0, L.px1, L.py1);
     if (L.grid) {
         L.px0 &= -kStampW;
         L.py0 &= -kStampH;
@@ -914,9 +917,9 @@ __device__ __forceinline__ void decode_large(const PassParams& P, const int4 q0,
 }
 
 template <bool kCamera>
-__device__ __forceinline__ void load_large(const PassParams& P, const TriRecord* rec, LargeRecord& L) {
+__device__ __forceinline__ void load_large(const TriRecord* rec, LargeRecord& L) {
     const int4* src = reinterpret_cast<const int4*>(rec);
-    decode_large<kCamera>(P, __ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3), L);
+    decode_large<kCamera>(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3), L);
 }
 
 // Record staging of the chunk walk: a warp copies the records a chunk starts
@@ -1176,8 +1179,8 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
             LargeRecord L;
             if (s + lane < s_end && r < n_rec) {
                 const uint32_t j = r - r_cur;
-                if (j < (uint32_t)kStageRecords) decode_large<kWriteId>(P, st[j][0], st[j][1], st[j][2], st[j][3], L);
-                else load_large<kWriteId>(P, P.records + r, L);
+                if (j < (uint32_t)kStageRecords) decode_large<kWriteId>(st[j][0], st[j][1], st[j][2], st[j][3], L);
+                else load_large<kWriteId>(P.records + r, L);
                 if (s + lane >= L.begin && s + lane < L.end) {
                     // stamp i of the record, below 2^24: the quotient by stamps per row, off by one at most
                     const int i = (int)(s + lane - L.begin), nsx = (int)L.nsx;
@@ -1224,7 +1227,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
             else raster_stamps<kWriteId, kSamples, false>(P, work, __popc(left), heads, 0u, lane, lx, ly);
             for (uint32_t m = __ballot_sync(kAllLanes, far); m; m &= m - 1) {
                 const int j = __ffs(m) - 1;
-                load_large<kWriteId>(P, P.records + __shfl_sync(kAllLanes, r, j), L);
+                load_large<kWriteId>(P.records + __shfl_sync(kAllLanes, r, j), L);
                 const int px = __shfl_sync(kAllLanes, sx0, j) + lx, py = __shfl_sync(kAllLanes, sy0, j) + ly;
                 const Target T = view_target<kWriteId>(P, L.view);
                 const size_t plane = kMsaa ? plane_words(P, L.view) : 0;
@@ -1245,6 +1248,8 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
 }
 
 void launch_raster(const PassParams& p, int sm_count, cudaStream_t stream, int share, bool next) {
+    // with ids it is the opaque camera pass, whose large stamps were counted on the block grid (on_grid)
+    if (p.write_id && (p.ordered || !p.tri_refs || !p.front)) return;
     // persistent grid: as many CTAs as can be resident at once, with the launches beside this one
     static int occ[3] = {0, 0, 0};
     const int t = !p.write_id ? 0 : p.msaa ? 2 : 1;
