@@ -1179,6 +1179,7 @@ int enqueue_frame(rz_ctx* c) {
     if (sources && !sources_side) launch_subpixel_sources(sh, s);
     if (c->blended_tris || c->debug_count) {
         BlendParams bp{};
+        bp.list = c->blended_tris != 0;
         bp.sh = sh;
         bp.sh.draws = c->d_blended_draws;
         bp.sh.draw_count = c->blended_draw_count;

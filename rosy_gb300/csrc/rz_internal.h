@@ -255,6 +255,7 @@ constexpr int64_t kDebugHalfWidth2 = 640 * 640;
 constexpr int32_t kDebugHalfWidth = 640;
 
 struct BlendParams {
+    bool list;                    // there are blended draws
     ShadeParams sh;               // blended draws, their constants and varyings
     const TriRecord* records;     // setup records of the blended triangles, in submission order
     const uint4* boxes;           // the boxes of their groups (launch_blend_boxes)

@@ -1474,11 +1474,15 @@ void launch_subpixel_sources(const ShadeParams& p, cudaStream_t stream) {
 // to 113 us with the cheaper fragment stage, and to 91 us with the prepared records and
 // the overlay's boxes. What is left is the latency of the fullest tiles and of the
 // five loads that a tile waits for one after the other.
-// Three CTAs per SM of 80 registers, and a pixel's values packed as they are stored: with
-// five of 48 the fragment stage spilled, and deep overdraw was slower than fragments shaded
-// where they are met (100 triangles across 640x360: 376 us a frame, 471 without the BRDF;
-// 294 and 287 shaded so; 276 and 288 with three). The frame above takes 87 us with three or
-// five, 85 with four, which lose on deep overdraw (290 and 341).
+// A pixel's values are held packed as they are stored, and a CTA has 64 registers a thread,
+// four to an SM (80 and three with 4 samples). With five of 48 the fragment stage spilled, and
+// deep overdraw was slower than fragments shaded where they are met: 100 triangles across
+// 640x360 376 us a frame, 471 without the BRDF, 496 with 4 samples, against 294, 287 and 355;
+// now 289, 339 and 321. Three per SM would take 274 and 286 for the first two, but the tiles
+// that meet little want more of them: 3840x2160 with 640 blended triangles 271 us, 249 with
+// four, 260 with five. (The frame above: 87, 85 and 87.)
+// Without a blended list only the overlay is compiled in, 40 registers and six CTAs: 900
+// overlay objects at 1080p 737 -> 595 us.
 constexpr int kBlendBatch = 512;   // group boxes (or overlay segments) tested at a time
 constexpr int kBlendList = 256;    // records of a tile prepared at a time
 constexpr int kBlendRound = 4;     // fragments a pixel collects before the tile shades them
@@ -1705,8 +1709,8 @@ __device__ __forceinline__ void shade_fragments(const ShadeParams& P, const View
     }
 }
 
-template <bool kMsaa>
-__global__ void __launch_bounds__(256, 3) k_blend(const __grid_constant__ BlendParams B) {
+template <bool kMsaa, bool kList>  // kList: there is a blended list (else only the overlay)
+__global__ void __launch_bounds__(256, !kList ? 6 : kMsaa ? 3 : 4) k_blend(const __grid_constant__ BlendParams B) {
     constexpr int kSamples = kMsaa ? kMsaaSamples : 1;
     __shared__ float s_srgb[256];
     __shared__ uint32_t s_list[kBlendBatch];  // groups (or overlay segments) that meet the tile
@@ -1723,7 +1727,7 @@ __global__ void __launch_bounds__(256, 3) k_blend(const __grid_constant__ BlendP
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     // a pass whose look-back gave up has records at unreliable slots: blend none of them
     const bool records_ok = !B.error_flags || !(*B.error_flags & kErrLookbackTimeout);
-    const uint32_t n = records_ok ? min(B.header->records, B.record_capacity) : 0u;
+    const uint32_t n = kList && records_ok ? min(B.header->records, B.record_capacity) : 0u;
     const uint32_t groups = (n + kBlendGroup - 1) / kBlendGroup;
     const float srgb = P.srgb_table[tid];
     uint32_t view = 0;
@@ -1767,8 +1771,8 @@ __global__ void __launch_bounds__(256, 3) k_blend(const __grid_constant__ BlendP
     if (tid < 16) s_ndc.x[tid] = ndc(tx0 + tid, VR.width);
     else if (tid < 32) s_ndc.y[tid - 16] = ndc(ty0 + tid - 16, VR.height);
     any = __syncthreads_or(any) != 0;
-    const bool lit = any && lit_view(*VR.scene);
-    for (uint32_t first = 0; any && first < groups; first += kBlendBatch) {
+    const bool lit = kList && any && lit_view(*VR.scene);
+    for (uint32_t first = 0; kList && any && first < groups; first += kBlendBatch) {
         const uint32_t ngroups = compact_batch<kBlendBatch / 256>(first, groups, tid, s_list, s_count[0], [&](uint32_t g) {
             const uint4 b = __ldg(&B.boxes[g]);
             return b.z <= view && view <= b.w && box_meets(b.x, b.y, tx0, ty0);
@@ -1956,8 +1960,9 @@ size_t blend_box_count(uint32_t capacity) { return (capacity + (size_t)kBlendGro
 
 void launch_blend(const BlendParams& p, cudaStream_t stream) {
     if (p.sh.shade_blocks == 0) return;
-    if (p.sh.samples > 1) k_blend<true><<<p.sh.shade_blocks, dim3(16, 16), 0, stream>>>(p);
-    else k_blend<false><<<p.sh.shade_blocks, dim3(16, 16), 0, stream>>>(p);
+    void (*const kernel)(BlendParams) = p.list ? (p.sh.samples > 1 ? k_blend<true, true> : k_blend<false, true>)
+                                               : (p.sh.samples > 1 ? k_blend<true, false> : k_blend<false, false>);
+    kernel<<<p.sh.shade_blocks, dim3(16, 16), 0, stream>>>(p);
     note_launch();
 }
 

@@ -3,8 +3,6 @@
 Bar: visibility (triangle id per pixel), depth and the shadow map are
 bit-exact; the RGBA8 sRGB colour is within 1/255 per channel.
 """
-import time
-
 import numpy as np
 import pytest
 
@@ -379,46 +377,6 @@ def test_blended_edges(gpu, oracle, samples, width, height, triangles, spread):
     ref, out = run(s, oracle)
     assert np.array_equal(out["ids"], ref["ids"])
     assert np.abs(out["color"].astype(np.int32) - ref["color"].astype(np.int32)).max() <= COLOR_TOL
-
-
-def frame_ms(s):
-    """Time of a frame, the least of six runs of 40."""
-    g = Graphics()
-    g.init(s.width, s.height, s.shadow_size, samples=s.samples)
-    try:
-        g.set_asset(s)
-        g.set_graphic_objects(s.objects, s.surfaces)
-        g.set_draw_config(s.draw_config)
-        g.update(s.scene)
-        for _ in range(3):
-            g.render()
-            while g.sync_code() == 14:
-                g.render()
-        times = []
-        for _ in range(6):
-            t0 = time.perf_counter()
-            for _ in range(40):
-                g.render()
-            g.sync()
-            times.append(time.perf_counter() - t0)
-        return min(times) * 25
-    finally:
-        g.deinit()
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("triangles,spread,most", [(400, 0.6, 1.17), (100, 2.0, 1.1)])
-def test_simple_lighting_is_not_slower(gpu, triangles, spread, most):
-    """The fragment stage's copy for views without the BRDF does less arithmetic than the one with it, so deep
-    overdraw by large blended triangles takes no longer but for what its register spills cost."""
-    s = sc.random_triangles(seed=3, triangles=triangles, width=640, height=360, shadow_size=512, texture_size=64)
-    v = s.vertices[:, 0:3].reshape(-1, 3, 3)
-    s.vertices[:, 0:3] = (v[:, :1] + (v - v[:, :1]) * np.float32(spread)).reshape(-1, 3)
-    s = sc.with_blended(s, 0.99, alpha=0.3)
-    lit = frame_ms(s)
-    s.scene["brdf_lighting_enabled"] = 0
-    simple = frame_ms(s)
-    assert simple <= most * lit, (simple, lit)
 
 
 @pytest.mark.gpu
