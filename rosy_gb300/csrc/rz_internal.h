@@ -100,7 +100,8 @@ constexpr uint32_t kCascadeMask = 3u;     // cascade = (view >> kViewBits) & kCa
 // Large records also carry raster facts the setup computed once, so that the
 // raster decodes them instead of recomputing them: view bits 26-28 the top-left
 // bias of edges 0-2 (1: not a top-left edge), 29 near origin, 30 box cut by the
-// viewport; stamp_offset bits 40-63 the stamps per row of the record's box.
+// viewport, 31 edge functions fit 32 bits (large_facts); stamp_offset bits 40-63 the
+// stamps per row of the record's box.
 constexpr uint32_t kRecFlagShift = 26;
 constexpr uint32_t kRecViewMask = (1u << kRecFlagShift) - 1u;  // view index and cascade
 constexpr int kStampOffsetBits = 40;
@@ -233,19 +234,21 @@ struct ShadeParams {
 struct DebugPair {
     float a[4], b[4];
     uint32_t object;
-    uint32_t pad[6];
+    uint32_t pad[3];
 };
+static_assert(sizeof(DebugPair) == 48, "three 16-byte words");
 
-// One segment of one view after the vertex stage, clipping and the viewport:
-// window ends in 1/256 pixel, their depths, the inclusive pixel box
-// (x | y << 16) that can hold covered samples, the object's colour; 64 bytes.
+// One segment of one view after the vertex stage, clipping and the viewport: its
+// ends in 1/256 pixel with their depths, its colour, and the most that |perp| of
+// debug_covers can be on it. Its pixel box is in an array of its own (k_debug_prep).
 struct DebugSeg {
     int32_t X0, Y0, X1, Y1;
     float z0, z1;
     float rgb[3];
     float reach;                  // half the width times the length, not rounded below it (infinite: not known)
-    uint32_t pad[3];
+    uint32_t pad[6];
 };
+static_assert(sizeof(DebugSeg) == 64, "half a cache line, so that none straddles two");
 
 // The box of a segment that is clipped away or outside the view: it meets no tile.
 constexpr uint32_t kDebugNoBox = 0xffffffffu;
