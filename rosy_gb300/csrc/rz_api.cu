@@ -845,8 +845,6 @@ PassParams pass_params(rz_ctx* c, int kind) {
     p.chunk_stamps = c->chunk_stamps;
     p.small_extent = c->small_extent;
     p.lookback_spins = c->lookback_spins;
-    p.sample_x = 128;  // pixel centre
-    p.sample_y = 128;
     p.msaa = (kind != 0 && c->samples > 1) ? 1 : 0;
     p.bb_hi = p.msaa ? 32 : 128;
     PassBuffers* pb;

@@ -114,6 +114,8 @@ constexpr int kMsaaSamples = 4;
 __host__ __device__ constexpr int32_t msaa_x(int k) { return k == 0 ? 96 : k == 1 ? 224 : k == 2 ? 32 : 160; }
 __host__ __device__ constexpr int32_t msaa_y(int k) { return k == 0 ? 32 : k == 1 ? 96 : k == 2 ? 160 : 224; }
 
+constexpr int32_t kCentre = 128;      // the sample of a single-sampled pass, the pixel centre, in 1/256 pixel
+
 constexpr int kStampW = 8;
 constexpr int kStampH = 4;
 constexpr uint32_t kTileBlocks = (16 / kStampW) * (16 / kStampH);  // stamps on the grid in a shading tile
@@ -176,8 +178,6 @@ struct PassParams {
     PassHeader* header;
     uint32_t* error_flags;
     uint32_t lookback_spins;  // bound of each look-back wait (ordered passes)
-    // coverage sample, in 1/256 pixel: the pixel centre (128, 128)
-    int32_t sample_x, sample_y;
     int32_t bb_hi;  // smallest sample offset the setup boxed for (32 with 4x samples, else 128)
     // 4x multisampled camera pass: every record at the four standard positions, each
     // into its plane; the records are dealt to kMsaaSamples launches, of which this is `part`

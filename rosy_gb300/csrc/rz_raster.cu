@@ -848,9 +848,9 @@ __device__ __forceinline__ void raster_small(const PassParams& P, const TriRecor
         }
     } else {
         for (int py = py0; py <= py1; ++py) {
-            const int32_t ry = py * 256 + P.sample_y - Y[0];
+            const int32_t ry = py * 256 + kCentre - Y[0];
             for (int px = px0; px <= px1; ++px) {
-                const int32_t rx = px * 256 + P.sample_x - X[0];
+                const int32_t rx = px * 256 + kCentre - X[0];
                 const int32_t e0 = c[0] + dx[0] * ry - dy[0] * rx;
                 const int32_t e1 = c[1] + dx[1] * ry - dy[1] * rx;
                 const int32_t e2 = c[2] + dx[2] * ry - dy[2] * rx;
@@ -1194,8 +1194,8 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
                     }
                     sx0 = L.px0 + sx * kStampW;
                     sy0 = L.py0 + sy * kStampH;
-                    PX = sx0 * 256 + (kMsaa ? 0 : P.sample_x);
-                    PY = sy0 * 256 + (kMsaa ? 0 : P.sample_y);
+                    PX = sx0 * 256 + (kMsaa ? 0 : kCentre);
+                    PY = sy0 * 256 + (kMsaa ? 0 : kCentre);
                     if (s + lane + 1 == L.end) ++r_after_this;
                     far = !L.near_origin;
                     live = !far;
@@ -1234,7 +1234,7 @@ __global__ void __launch_bounds__(kRasterThreads, 3) k_raster(PassParams P) {
 #pragma unroll 1
                 for (int i = 0; i < kSamples; ++i) {
                     const Target Ti{reinterpret_cast<TargetWord<kWriteId>*>(T.ptr) + i * plane, T.pitch};
-                    raster_far_pixel<kWriteId>(Ti, L, px, py, kMsaa ? msaa_x(i) : P.sample_x, kMsaa ? msaa_y(i) : P.sample_y);
+                    raster_far_pixel<kWriteId>(Ti, L, px, py, kMsaa ? msaa_x(i) : kCentre, kMsaa ? msaa_y(i) : kCentre);
                 }
             }
             r_first = __shfl_sync(kAllLanes, r_after_this, 31);
