@@ -505,7 +505,12 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
 
     __shared__ float s_bias[N];
     __shared__ float4 s_srcw[16];  // final layer: the x2 base's source weights for each source mask
-    if (warp == 0) tmem_alloc(tmem_slot, L::TMEM_COLS);
+    if (warp == 0) {
+        tmem_alloc(tmem_slot, L::TMEM_COLS);
+        // not before this CTA has its tensor memory: a CTA of the next kernel that came first would
+        // hold its own while it waits for this kernel, which would wait in the allocation
+        pdl_allow_next();
+    }
     if (tid == 0) {
         for (int b = 0; b < NS; ++b) {
             mbar_init(&full[b], 1);
@@ -528,9 +533,6 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(ConvArgs a, const __gr
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // not before this CTA has its tensor memory: a CTA of the next kernel that came first would
-    // hold its own while it waits for this kernel, which would wait in the allocation
-    pdl_allow_next();
     const uint32_t tmem = *tmem_slot;
     const int group = warp / kConvGroupWarps, quad = warp & 3, row0 = (warp % kConvGroupWarps >> 2) * kWarpRows;
     if (warp < kConvEpilogueWarps) {  // the read accumulator rows of both buffers (group g drains buffer g) start at zero
@@ -759,7 +761,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __gr
     const int tiles_x = (a.W + kWgKP - 1) / kWgKP;
     const int ntiles = tiles_x * ((a.H + kWgRows - 1) / kWgRows);
     const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    if (warp == 0) tmem_alloc(tmem_slot, L::TMEM_COLS);
+    if (warp == 0) {
+        tmem_alloc(tmem_slot, L::TMEM_COLS);
+        pdl_allow_next();  // with its tensor memory, as in k_conv
+    }
     if (tid == 0) {
         for (int b = 0; b < NS; ++b) {
             mbar_init(&full[b], 1);
@@ -770,7 +775,6 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(WgradArgs a, const __gr
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_allow_next();  // with its tensor memory, as in k_conv
     const uint32_t tmem = *tmem_slot;
     pdl_wait_previous();
     bool ok = true;
