@@ -231,9 +231,10 @@ typedef struct rz_config {
     uint32_t samples;          /* rasterisation samples per pixel: 1 */
     int32_t device;            /* CUDA device ordinal */
     uint32_t queue_chunks;     /* raster work-queue depth per pass, in chunks of 32
-                                  8x4-pixel stamps; 0 = sized from the scene. A frame
-                                  that needs more reports RZ_OVERFLOW and the queue
-                                  grows for the next frame. */
+                                  8x4-pixel stamps counted from each triangle's box;
+                                  0 = sized from the scene. A frame that needs more
+                                  reports RZ_OVERFLOW and the queue grows for the
+                                  next frame. */
     uint32_t reserved[2];
 } rz_config;
 
@@ -318,7 +319,11 @@ int rz_render(struct rz_ctx* ctx);
 
 /* Waits for the stream, at most timeout_ms milliseconds (0 = no limit).
  * Returns RZ_TIMEOUT if the frame is still running, RZ_OVERFLOW or
- * RZ_GRAPHICS_FRAME_FAILURE if the device flagged an error in a frame. */
+ * RZ_GRAPHICS_FRAME_FAILURE if the device flagged an error in a frame.
+ * The calling thread polls: without a pause for the first millisecond of the
+ * wait (a frame takes a fraction of it), then every 50 us. Until then it keeps a
+ * core busy; a program with more waiting threads than cores calls later, or with
+ * several contexts waits for them from one thread. */
 int rz_sync(struct rz_ctx* ctx, uint32_t timeout_ms);
 
 /* Device pointers of the buffers of the frame rendered last (valid until the
@@ -341,8 +346,8 @@ int rz_read_frame(struct rz_ctx* ctx, void* color_host, size_t color_bytes,
 /* Waits until at most `pending` (0 or 1) of the read-backs queued by
  * rz_read_frame are still travelling: 1 waits for all but the newest, so a
  * caller with two host buffers may refill the older one. RZ_TIMEOUT after
- * timeout_ms (0: no limit). Library addition (the reference presents to a
- * swapchain instead). */
+ * timeout_ms (0: no limit). Polls as rz_sync does. Library addition (the
+ * reference presents to a swapchain instead). */
 int rz_read_sync(struct rz_ctx* ctx, uint32_t pending, uint32_t timeout_ms);
 
 /* Counters of the last completed frame (call after rz_sync). */
